@@ -113,6 +113,14 @@ static RhsParams rhs_params(const af_operator* o, int stage) {
     r.ca[2] = r.ct[2] = r.cg[2] = o->b3;
     r.cgI = 0.0;
   }
+  for (int j = 0; j < 3; ++j) {
+    const double a = r.ca[j] * r.dt, t = r.ct[j] * r.dt, g = r.cg[j] * r.dt;
+    r.r_[j] = a; r.p_[j] = t * r.invMa2; r.f_[j] = g * r.invFr2; r.e_[j] = g * r.Ma2Fr2;
+    r.k_[j] = 0.5 * a * r.Ma2; r.h_[j] = t * r.gg;
+    r.r2_[j] = 0.5 * a; r.p2_[j] = 0.5 * t * r.invMa2; r.k2_[j] = 0.25 * a * r.Ma2; r.h2_[j] = 0.5 * t * r.gg;
+    r.j_[j] = 0.5 * t * r.g1;
+  }
+  r.fI = r.cgI * r.dt * r.invFr2; r.eI = r.cgI * r.dt * r.Ma2Fr2; r.hMa2 = 0.5 * r.Ma2;
   return r;
 }
 

@@ -1,25 +1,40 @@
 // af_cellop.cuh -- generic cell-centric, sum-factorised DG operator kernel for sm_100a.
 //
-// One CTA owns CB consecutive cells (deal.II active-cell order = DoF order) and NQ
-// threads per cell ("members").  Every operator of the reference's EULEROperator is a
-// sum over "groups" of input fields of (cell integral) + (face integral) terms, so a
-// Phys policy describes, per group, the input arrays, the pointwise integrand and the
-// numerical flux; this kernel does the data movement and the tensor-product algebra:
+// One CTA owns CB consecutive cells (deal.II active-cell order = DoF order) and NQ threads per
+// cell.  Every operator of the reference's EULEROperator is a sum over "groups" of input fields
+// of (cell integral) + (face integral) terms, so a Phys policy describes, per group, the input
+// arrays, the pointwise integrand and the numerical flux; this kernel does the data movement and
+// the tensor-product algebra:
 //
-//   per group:  global -> smem (coalesced, 16-byte loads, odd-padded per cell)
-//               X pass : rows (i, P-i) combined even/odd, contracted along x  -> smem
-//               Z pass : member = quadrature column qx; points (qz, NQ-1-qz) in pairs,
-//                        integrand, then test-function contraction along z accumulated
-//                        in registers (even/odd split, constant-memory coefficients)
-//               faces  : member = face quadrature point; own trace and the neighbour's
-//                        trace (GLL nodes on the face), numerical flux, weighted and
-//                        accumulated per (face, output, point) in smem
-//   then:       XT pass: contraction along x of the accumulated rows, plus the face
-//                        terms on the face nodes -> smem -> coalesced global stores.
+//   per batch of groups (PhysInfo):
+//     traces : 1D contractions of the neighbours' face nodes, read directly from global memory
+//              while the own cells' nodes arrive by bulk copies
+//     lines  : 1D contractions of the own nodes along x, rows (i, P-i) combined even/odd, and of
+//              the own x-faces' nodes; one line per thread, consecutive threads on consecutive
+//              cells
+//     faces  : thread = face point; numerical flux from the traces of both sides
+//     z pass : thread = quadrature column qx; points (qz, NQ-1-qz) in pairs, integrand, then the
+//              test-function contraction along z accumulated in registers (even/odd split,
+//              constant-memory coefficients)
+//   then:      contraction along x of the accumulated rows, plus the face terms on the x-faces'
+//              nodes -> shared memory -> bulk stores.
 //
-// Faces are evaluated from both sides (cell-centric): no atomics, deterministic, and the
-// flux seen by the two cells of a face is the exact negation of each other because the
-// normals come from the same two vertices.  Boundary faces call Phys::boundary.
+// Faces are evaluated from both sides (cell-centric): no atomics, deterministic, and both cells of
+// a face form its normal from the same two vertices.  Boundary faces call Phys::boundary.
+//
+// What bounds it and why this split (FP64, degree 4, 512x256 cells, fused stage-1 right-hand sides):
+// FP64 issue (68 M warp instructions, a 110 us floor at the pipe's rate, against 44 us of HBM
+// traffic) and the shared-memory data path (41 M wavefronts).  402 us before this layout, 206 us with
+// it.  What gave that:
+// - 14 cells x 9 points fill 4 warps and three such CTAs an SM (168 registers, 74 KB); 16 cells left
+//   half a warp idle and two CTAs an SM;
+// - the face traces are 1D contractions done once per face line (even/odd, one thread) instead of at
+//   each of the 9 face points, the x-neighbours' read from the own lines of the same CTA, and the
+//   own z-face traces are sums of rows that the z pass needs anyway;
+// - rows are laid out [row][cell][point], lines at an odd stride: no bank conflicts in the z pass;
+// - fluxes are linear in the normal, so edge vectors replace unit normals (no square roots), and the
+//   quadrature weights sit in the tables and in one factor per accumulator;
+// - the three groups of stage 3 run in batches (below): 10.8 -> 3.8 ms at 2048x512.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -36,7 +51,7 @@ struct MeshDev {
   const double2* vtx;  // (nz+1)*(nx+1) vertices, row-major in (j, i)
   int nx, nz, periodic_x, gravity;
   double radial_a;
-  int cell0;  // cell kernels: the first cell of the launch (a multiple of its cells per CTA);
+  int cell0;  // cell kernels: the first cell of the launch;
               // the launch covers [cell0, ncell).  0 for whole-mesh launches
   // Status word of the caller (host-visible; null: not reported).  A kernel that gives up a
   // bounded wait writes kStatusStageTimeout there and leaves without writing its outputs.
@@ -60,19 +75,21 @@ struct PointGeo {
 // d/dxi of the gradient fields; deta holds their d/deta).  Policies without nfg_of have none.
 template <class Phys, class = void>
 struct NfgOf {
+  static constexpr bool any = false;
   static constexpr int get(int) { return 0; }
 };
 template <class Phys>
 struct NfgOf<Phys, std::void_t<decltype(Phys::nfg_of(0))>> {
+  static constexpr bool any = true;
   static constexpr int get(int g) { return Phys::nfg_of(g); }
 };
 
 // Policies may map their integrand to the reference cell themselves (Phys::MAPPED): their
-// point_mapped<G>(prm, v, pg, A, dw, fv, fx, fe) adds, per output o, fv[o] = value * |J| w and
+// point_mapped<G>(prm, v, pg, A, dw, fv, fx, fe) adds, per output o, fv[o] = value * |J| and
 // (fx[o], fe[o]) = (A0 g0 - A1 g1, A3 g1 - A2 g0) for the output's flux g, with
-// A = (J11, J01, J10, J00) w = adj(J) w.  A policy that knows the structure of its fluxes can
-// share products of the Jacobian between outputs (contravariant velocities); the others return
-// physical values and fluxes and the kernel maps them.
+// A = (J11, J01, J10, J00) = adj(J) and dw = |J| (the kernel applies the quadrature weights).  A
+// policy that knows the structure of its fluxes can share products of the Jacobian between outputs
+// (contravariant velocities); the others return physical values and fluxes and the kernel maps them.
 template <class Phys, class = void>
 struct MappedOf {
   static constexpr bool value = false;
@@ -80,20 +97,6 @@ struct MappedOf {
 template <class Phys>
 struct MappedOf<Phys, std::void_t<decltype(Phys::MAPPED)>> {
   static constexpr bool value = Phys::MAPPED;
-};
-
-// Policies opt in to z-face folding (Layout::FOLD_Z) with Phys::FOLD = true.  Measured at
-// 512x256, p = 4: the fused rhs 439 -> 399 us with it, its stage-1 backward 1.53 -> 1.43 ms;
-// C (the enthalpy operator) 125 -> 153 us and the FP64 IMEX step 265 -> 275 ms, where the
-// z-faces evaluated after the z pass serialise behind it; the FP32 smoother kernels are
-// indifferent (mixed step 77.1 vs 77.4 ms).
-template <class Phys, class = void>
-struct FoldOf {
-  static constexpr bool value = false;
-};
-template <class Phys>
-struct FoldOf<Phys, std::void_t<decltype(Phys::FOLD)>> {
-  static constexpr bool value = Phys::FOLD;
 };
 
 // Whether a policy's point functions read the physical position: Phys::NEED_X, and for
@@ -164,6 +167,19 @@ __device__ __forceinline__ const Tab<P>& tab() {
 template <int P, class R>
 __device__ __forceinline__ const CobT<P, R>& cobr();
 
+// Outputs that the integrands of batch B feed with values and with fluxes: those of the policy, or
+// fewer where it says so (val_in(B, o), grad_in(B, o)).
+template <class Phys, class = void>
+struct TermsOf {
+  static constexpr bool val(int, int o) { return Phys::has_val(o); }
+  static constexpr bool grad(int, int o) { return Phys::has_grad(o); }
+};
+template <class Phys>
+struct TermsOf<Phys, std::void_t<decltype(Phys::val_in(0, 0))>> {
+  static constexpr bool val(int b, int o) { return Phys::has_val(o) && Phys::val_in(b, o); }
+  static constexpr bool grad(int b, int o) { return Phys::has_grad(o) && Phys::grad_in(b, o); }
+};
+
 // Fused multiply-add in the working precision (no silent promotion of float operands).
 __device__ __forceinline__ double fmaR(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fmaR(float a, float b, float c) { return __fmaf_rn(a, b, c); }
@@ -184,12 +200,6 @@ __device__ __forceinline__ void cp_async_el(float* smem_dst, const float* gsrc) 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 constexpr int odd(int n) { return n | 1; }
-
-// Own-cell staging by bulk copies (1) or per-element cp.async (0); see Layout::BULK.
-#ifndef AF_BULK_STAGING
-#define AF_BULK_STAGING 1
-#endif
-constexpr bool kBulkStaging = AF_BULK_STAGING != 0;
 
 // Programmatic dependent launch between consecutive cell-operator launches in a stream: every
 // CTA allows the next launch at its entry (griddepcontrol.launch_dependents), so the next
@@ -243,26 +253,11 @@ __device__ __forceinline__ void report_status(int* status, int code) {
   }
 }
 
-// Unroll factor of the z-pass loop over quadrature-point pairs (see the kernel).
-#ifndef AF_Z_UNROLL
-#define AF_Z_UNROLL 1
-#endif
-constexpr int kZUnroll = AF_Z_UNROLL;
-
-// Cells per CTA and the CTAs-per-SM hint of __launch_bounds__, per degree.  Measured on
-// B200 for the fused stage-1 right-hand side at 512x256 cells, degree 4 (CB, MINB):
-// (16,1) 781 us, (16,2) 502 us, (32,1) 529 us, (8,3) 592 us, (8,4) 588 us (z loop not
-// unrolled; fully unrolled: 764 / 521 / 567 / 554 / 550 us).  Degree 5: (8,3) 822 us,
-// (8,2) 842, (12,2) 863, (16,2) 995 (one CTA per SM: 128 KB of shared memory).  Degree 6:
-// (8,2) 1070 us, (4,4) 1153, (6,3) 1406.  Degree 3: (16,3) 244 us, (16,2) 266, (24,2) 273,
-// (32,1) 299.
-template <int P>
+// Cells per CTA, per degree (see the kernel).
+template <int P, class R = double>
 constexpr int cells_per_block() {
-  return P <= 1 ? 64 : (P == 2 ? 32 : (P <= 4 ? 16 : 8));
-}
-template <int P>
-constexpr int min_blocks_per_sm() {
-  return P == 3 || P == 5 ? 3 : 2;
+  if (sizeof(R) == 4) return P <= 1 ? 64 : (P == 2 ? 32 : (P <= 4 ? 16 : 8));
+  return P <= 1 ? 42 : (P == 2 ? 24 : (P == 3 ? 18 : (P == 4 ? 14 : (P == 5 ? 11 : 8))));
 }
 
 template <int MAXARR, int MAXOUT, class R = double>
@@ -276,73 +271,131 @@ struct ArgPtrs {
 // ----------------------------------------------------------------------------------
 template <class Phys, int G>
 struct GroupInfo {
-  static constexpr int NARR = Phys::template Grp<G>::NARR;
-  static constexpr int arr_base() {
-    int b = 0;
-    for (int g = 0; g < G; ++g) b += Phys::narr_of(g);
-    return b;
-  }
+  using Gr = typename Phys::template Grp<G>;
+  static constexpr int NARR = Gr::NARR;
+  static constexpr bool FACE = Phys::FACES && Gr::FACE;
   static constexpr int NF = [] {
     int n = 0;
-    for (int a = 0; a < NARR; ++a) n += Phys::template Grp<G>::ncomp(a);
+    for (int a = 0; a < NARR; ++a) n += Gr::ncomp(a);
     return n;
   }();
   static constexpr int NF_GRAD = NfgOf<Phys>::get(G);  // the last NF_GRAD cell fields
   static constexpr int NF_CELL = [] {  // fields used by cell integrals (face-only ones last)
     int n = 0;
     for (int a = 0; a < NARR; ++a)
-      if (!Phys::template Grp<G>::face_only(a)) n += Phys::template Grp<G>::ncomp(a);
+      if (!Gr::face_only(a)) n += Gr::ncomp(a);
     return n;
   }();
+  static constexpr int arr_of(int f) {  // array of field f
+    int a = 0;
+    for (int n = Gr::ncomp(0); f >= n; n += Gr::ncomp(a)) ++a;
+    return a;
+  }
+  static constexpr int first_field(int a) {
+    int n = 0;
+    for (int k = 0; k < a; ++k) n += Gr::ncomp(k);
+    return n;
+  }
+};
+
+// Policies whose faces read only some fields of a group declare face_field(G, f); the others
+// read all of them.
+template <class Phys, class = void>
+struct FaceFieldOf {
+  static constexpr bool get(int, int) { return true; }
+};
+template <class Phys>
+struct FaceFieldOf<Phys, std::void_t<decltype(Phys::face_field(0, 0))>> {
+  static constexpr bool get(int g, int f) { return Phys::face_field(g, f); }
 };
 
 template <class Phys, int... G>
-constexpr int count_face_groups(std::integer_sequence<int, G...>) {
-  return ((Phys::FACES && Phys::template Grp<G>::FACE ? 1 : 0) + ... + 0);
-}
-template <class Phys, int... G>
-constexpr int last_face_group(std::integer_sequence<int, G...>) {
-  int r = -1;
-  ((r = (Phys::FACES && Phys::template Grp<G>::FACE) ? G : r), ...);
-  return r;
+constexpr int arr_total(int upto, std::integer_sequence<int, G...>) {
+  return ((G < upto ? GroupInfo<Phys, G>::NARR : 0) + ... + 0);
 }
 
+// The groups of a policy run in batches: one batch stages its groups' fields, contracts them
+// along x and evaluates them together at the points, so that their integrands share one mapping
+// and one test contraction.  A policy with one face group is one batch; with several (the stages
+// with two and three explicit groups) each is its own batch and so is the implicit group after
+// them: the batches' fields follow one another through the same shared memory, which keeps two or
+// three CTAs on an SM (all of them at once left one CTA of 16 cells per SM at degree 4: the
+// stage-3 right-hand sides at 2048x512 10.8 ms, in batches 5.4 ms).
 template <class Phys>
 struct PhysInfo {
-  static constexpr int NFACEG = count_face_groups<Phys>(std::make_integer_sequence<int, Phys::NG>{});
-  static constexpr int FACE_G = last_face_group<Phys>(std::make_integer_sequence<int, Phys::NG>{});
-  static constexpr int NFMAX = [] {
-    int m = 0;
-    for (int g = 0; g < Phys::NG; ++g) m = m > Phys::nf_of(g) ? m : Phys::nf_of(g);
-    return m;
-  }();
-  static constexpr int NARR_TOTAL = [] {
+  using Seq = std::make_integer_sequence<int, Phys::NG>;
+  static constexpr int NARR_TOTAL = arr_total<Phys>(Phys::NG, Seq{});
+  static constexpr int arr_base(int G) { return arr_total<Phys>(G, Seq{}); }
+  template <int... G>
+  static constexpr int batch_of_impl(int g, std::integer_sequence<int, G...>) {
+    const bool face[] = {GroupInfo<Phys, G>::FACE...};
+    int b = 0, nface = 0;
+    for (int k = 0; k < Phys::NG; ++k) nface += face[k] ? 1 : 0;
+    bool has = false;
+    for (int k = 0; k <= g; ++k) {
+      if (has && (face[k] || nface > 1)) {
+        ++b;
+        has = false;
+      }
+      has = has || face[k];
+    }
+    return b;
+  }
+  static constexpr int batch_of(int g) { return batch_of_impl(g, Seq{}); }
+  static constexpr int NB = batch_of(Phys::NG - 1) + 1;
+  template <int... G>
+  static constexpr int face_group_impl(int b, std::integer_sequence<int, G...>) {
+    int r = -1;
+    ((r = (GroupInfo<Phys, G>::FACE && batch_of(G) == b) ? G : r), ...);
+    return r;
+  }
+  // the face group of batch b (-1: none)
+  static constexpr int face_group(int b) { return face_group_impl(b, Seq{}); }
+  // x-contracted slots before group G in its batch: per group its cell fields (contracted with
+  // S), then its gradient fields again (contracted with D, for d/dxi)
+  template <int... G>
+  static constexpr int slots_impl(int g, int b, std::integer_sequence<int, G...>) {
+    return ((G < g && batch_of(G) == b ? GroupInfo<Phys, G>::NF_CELL + GroupInfo<Phys, G>::NF_GRAD : 0) + ... + 0);
+  }
+  static constexpr int slot_offset(int g) { return slots_impl(g, batch_of(g), Seq{}); }
+  static constexpr int slots(int b) { return slots_impl(Phys::NG, b, Seq{}); }
+  template <int... G>
+  static constexpr int grads_impl(int g, int b, std::integer_sequence<int, G...>) {
+    return ((G < g && batch_of(G) == b ? GroupInfo<Phys, G>::NF_GRAD : 0) + ... + 0);
+  }
+  static constexpr int grad_offset(int g) { return grads_impl(g, batch_of(g), Seq{}); }
+  static constexpr int grads(int b) { return grads_impl(Phys::NG, b, Seq{}); }
+};
+
+// The fields that the faces of group G read: count, and the k-th one; those that are face-only
+// (no x-contracted rows) come last.
+template <class Phys, int G>
+struct FaceInfo {
+  using Gi = GroupInfo<Phys, G < 0 ? 0 : G>;
+  static constexpr int NF = [] {
     int n = 0;
-    for (int g = 0; g < Phys::NG; ++g) n += Phys::narr_of(g);
+    if (G >= 0)
+      for (int f = 0; f < Gi::NF; ++f) n += FaceFieldOf<Phys>::get(G, f) ? 1 : 0;
     return n;
   }();
-  // cell fields (all groups) evaluated together in the merged z pass
-  // x-contracted slots: per group its cell fields (S rows), then its gradient fields again
-  // (D rows, for d/dxi)
-  static constexpr int NFC_TOTAL = [] {
+  static constexpr int NC = [] {  // of them with x-contracted rows
     int n = 0;
-    for (int g = 0; g < Phys::NG; ++g) n += Phys::nfc_of(g) + NfgOf<Phys>::get(g);
+    if (G >= 0)
+      for (int f = 0; f < Gi::NF_CELL; ++f) n += FaceFieldOf<Phys>::get(G, f) ? 1 : 0;
     return n;
   }();
-  static constexpr int eo_offset(int G) {
+  static constexpr int before(int f) {  // face fields before field f
     int n = 0;
-    for (int g = 0; g < G; ++g) n += Phys::nfc_of(g) + NfgOf<Phys>::get(g);
+    if (G >= 0)
+      for (int i = 0; i < f; ++i) n += FaceFieldOf<Phys>::get(G, i) ? 1 : 0;
     return n;
   }
-  static constexpr int NFG_TOTAL = [] {
-    int n = 0;
-    for (int g = 0; g < Phys::NG; ++g) n += NfgOf<Phys>::get(g);
-    return n;
-  }();
-  static constexpr int grad_offset(int G) {
-    int n = 0;
-    for (int g = 0; g < G; ++g) n += NfgOf<Phys>::get(g);
-    return n;
+  static constexpr int field(int k) {
+    int f = 0;
+    for (;; ++f) {
+      if (!FaceFieldOf<Phys>::get(G, f)) continue;
+      if (k-- == 0) return f;
+    }
   }
 };
 
@@ -357,94 +410,145 @@ struct NQOf<P, Phys, std::void_t<decltype(Phys::REDUCED_Q)>> {
   static constexpr int value = Phys::REDUCED_Q ? P + 1 : 2 * P + 1;
 };
 
-template <int P, class Phys, int CB_ = cells_per_block<P>()>
+constexpr int imax(int a, int b) { return a > b ? a : b; }
+
+template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>()>
 struct Layout {
   using R = RealOf<Phys>;
+  using I = PhysInfo<Phys>;
   using T = TabT<P, R, NQOf<P, Phys>::value>;
   static constexpr int P1 = T::P1, NQ = T::NQ, ND = P1 * P1;
   static constexpr int CB = CB_;
   static constexpr int NT = CB * NQ;
   static constexpr int NDP = odd(ND);
-  static constexpr int P1P = odd(P1);
-  static constexpr int EOS = odd(P1 * NQ);
-  static constexpr int NF = PhysInfo<Phys>::NFMAX;
-  static constexpr int NFC = PhysInfo<Phys>::NFC_TOTAL;
   static constexpr int NOUT = Phys::NOUT;
-  // region A: x-contracted rows of every cell field, later the z-accumulators
-  static constexpr int R_EO = NFC * CB * EOS;
-  static constexpr int R_ACC = NOUT * 2 * CB * EOS;
-  static constexpr int ALIGN = 16 / (int)sizeof(R);  // region B starts on a 16-byte boundary
-  static constexpr int RA = ((R_EO > R_ACC ? R_EO : R_ACC) + ALIGN - 1) / ALIGN * ALIGN;
-  // Own-cell staging by bulk asynchronous copies (TMA, one per array and CTA): the
-  // shared-memory image of an array equals its global chunk, laid out [cell][comp][node], and
-  // chunk sizes are multiples of 16 bytes (CB even).  Without padding an even ND puts the same
-  // node of consecutive cells on few banks: at degree 3 (ND 16, every cell on the same bank)
-  // bulk staging measured 414 us against 245 us with the padded per-element copies, at degree 5
-  // (ND 36 doubles, a 4-way conflict) 748 us against 836 us, and 707 us with the padded slots
-  // below; so even ND stages in bulk only at degree 5 in FP64.
-  static constexpr bool BULK =
-      kBulkStaging && (CB % 2 == 0) && ((ND % 2 == 1) || (P == 5 && sizeof(R) == 8));
-  // Padded bulk layout (even ND, i.e. degree 5 in FP64): each cell's chunk of an array arrives
-  // by its own bulk copy into a slot 16 bytes longer than the chunk (38 doubles for a scalar
-  // field, 74 for a velocity), so that the same node of the CTA's 8 cells lies on 8 different
-  // bank pairs instead of 4 (36 doubles = 8 banks apart).  The copies are spread over warp 0.
+  static constexpr int NB = I::NB;
+  // Rows: one value per (cell, point) of the CTA at stride NQP per cell.  A thread owns the
+  // point m of cell cl at offset cl NQP + m, so a warp reads a row without bank conflicts, and a
+  // line task writes or reads the NQ values of one cell at an odd stride between consecutive
+  // cells, again without conflicts.
+  static constexpr int NQP = odd(NQ);
+  static constexpr int RS = CB * NQP;
+  static constexpr int ALIGN = 16 / (int)sizeof(R);
+  // The rows of one x-contracted slot, and the x-face traces of one field (up to two outer
+  // neighbours per side), padded to 8 (mod 16) FP64 elements: the line tasks of a velocity
+  // alternate between its components, whose results then fall on the two halves of the banks.
+  static constexpr int half_banks(int n) { return n + (24 - n % 16) % 16; }
+  static constexpr int SLS = half_banks(P1 * RS);
+  static constexpr int TXS = half_banks((CB + 2) * NQP);
+  static constexpr int up(int n) { return (n + ALIGN - 1) / ALIGN * ALIGN; }
+  // Own-cell staging: the nodes of every (cell, component) of a batch's arrays form one list of
+  // lines of ND nodes at stride LS, array after array, [cell][component] inside an array (the
+  // global order).  With an odd number of nodes per cell the list is the arrays' image and arrives
+  // by one bulk copy (TMA) per array; with an even number in FP64 by one bulk copy per line, 16
+  // bytes apart against bank conflicts (degree 5: unpadded 748 us, padded 707 us for the fused
+  // right-hand sides at 512x256); else by per-element copies.  Consecutive threads take
+  // consecutive lines, an odd number of elements apart.
+  static constexpr bool BULK = (ND % 2 == 1 && (CB * ND * (int)sizeof(R)) % 16 == 0) || (ND % 2 == 0 && sizeof(R) == 8 && P >= 3);
   static constexpr int PADB = (BULK && ND % 2 == 0) ? ALIGN : 0;
-  static constexpr int slot(int nc) { return nc * ND + PADB; }  // one cell of an array
-  static constexpr int ISSUE_LANES = PADB ? 32 : 1;             // threads that issue the copies
-  // region B: one group's nodal values and neighbour face nodes, later the outputs
-  static constexpr int R_IN = NF * CB * (NDP > ND + PADB ? NDP : ND + PADB);
-  static constexpr int R_NB = Phys::FACES ? 4 * NF * CB * P1P : 0;
-  static constexpr int R_OUT = NOUT * CB * NDP;
-  static constexpr int RB = (R_IN + R_NB) > R_OUT ? (R_IN + R_NB) : R_OUT;
-  // z-face folding: with one face group whose staged nodes and neighbour face nodes are still in
-  // place after the z pass (no later group reuses its buffer), the fluxes of the z-faces are
-  // evaluated at the end of the z pass by the thread of quadrature column q and added to its
-  // accumulators of node rows 0 and P (the face term of node (iz, ix) on face 2 is
-  // delta(iz, 0) sum_q S(q, ix) F(q), the x-transpose pass's contraction of row 0); the
-  // x-transpose pass then has no edge rows with extra work
-  // (two input buffers: FACE_G + 2 >= NG; one buffer: FACE_G is the last group)
-  static constexpr int FACE_G = PhysInfo<Phys>::FACE_G;
-  static constexpr bool FOLD_OK = FoldOf<Phys>::value && Phys::FACES && PhysInfo<Phys>::NFACEG == 1;
-  static constexpr bool FOLD_2BUF = FOLD_OK && FACE_G + 2 >= Phys::NG;
-  static constexpr bool FOLD_1BUF = FOLD_OK && FACE_G == Phys::NG - 1;
-  static constexpr int flux_size(bool fold) { return Phys::FACES ? (fold ? 2 : 4) * NOUT * CB * NQ : 0; }
-
-  // per cell: A,B,C,v0 (8) + 4 faces x (nx,nz,len) (12) + 4 nb; an odd stride, so that a warp
-  // reading one slot of consecutive cells meets no bank conflicts (4- and 8-byte elements)
-  static constexpr int GS = 25;
-  static constexpr int R_GEO = CB * GS;
-  static constexpr int R_S = NQ * P1 + NQ;
-  // bulk staging of several groups: the own-cell chunks of group G+1 are copied into a second
-  // input buffer while group G is computed (group 0's at kernel entry); buffers alternate.
-  // Only where the second buffer leaves the number of resident CTAs per SM unchanged (228 KB
-  // of shared memory per SM, 1 KB reserved per CTA).
-  static constexpr int RBA = (RB + ALIGN - 1) / ALIGN * ALIGN;
-  static constexpr int R_IN_A = (R_IN + ALIGN - 1) / ALIGN * ALIGN;
-  static constexpr int EPI = EpiOf<Phys>::value;
-  static constexpr int NE = EPI >= 2 ? 4 : 1;
-  static constexpr int total_with(int rin2, int rflux) {
-    const int base = RA + RBA + rin2 + rflux + R_GEO + R_S;
-    return EPI ? (base + ALIGN - 1) / ALIGN * ALIGN + NE * CB * ND : base;
+  static constexpr int LS = BULK ? ND + PADB : odd(ND);
+  static constexpr int ISSUE_LANES = PADB ? 32 : 1;  // threads that issue the copies
+  // fields of the groups before G0 in its batch (G0 = NG: of batch b): cell fields, face-only fields
+  template <int... G>
+  static constexpr int cells_before(int g0, int b, std::integer_sequence<int, G...>) {
+    return ((G < g0 && I::batch_of(G) == b ? GroupInfo<Phys, G>::NF_CELL : 0) + ... + 0);
   }
-  static constexpr int ctas_per_sm(int total) { return (228 * 1024) / ((int)sizeof(R) * total + 1024); }
-  static constexpr int T_PF = total_with(R_IN_A, flux_size(FOLD_2BUF)), T_NOPF = total_with(0, flux_size(FOLD_1BUF));
-  static constexpr bool PREFETCH =
-      BULK && Phys::NG > 1 && (int)sizeof(R) * T_PF <= 227 * 1024 && ctas_per_sm(T_PF) >= ctas_per_sm(T_NOPF);
-  static constexpr int R_IN2 = PREFETCH ? R_IN_A : 0;
-  static constexpr bool FOLD_Z = PREFETCH ? FOLD_2BUF : FOLD_1BUF;
-  // the flux accumulators of the x-faces (0, 1) and, unless folded, of the z-faces (2, 3)
-  static constexpr int R_FLUX = flux_size(FOLD_Z);
-  static constexpr int RB2 = RBA + R_IN2;
+  template <int... G>
+  static constexpr int only_before(int g0, int b, std::integer_sequence<int, G...>) {
+    return ((G < g0 && I::batch_of(G) == b ? GroupInfo<Phys, G>::NF - GroupInfo<Phys, G>::NF_CELL : 0) + ... + 0);
+  }
+  // first line of array a of group G in its batch: the cell fields of all groups come first, then
+  // the face-only ones
+  template <int G>
+  static constexpr int line_base(int a) {
+    using Gi = GroupInfo<Phys, G>;
+    using S = typename I::Seq;
+    const int b = I::batch_of(G), f = Gi::first_field(a);
+    if (f < Gi::NF_CELL) return CB * (cells_before(G, b, S{}) + f);
+    return CB * (cells_before(Phys::NG, b, S{}) + only_before(G, b, S{}) + f - Gi::NF_CELL);
+  }
+  template <int G>
+  static constexpr int group_size() {
+    return CB * GroupInfo<Phys, G>::NF * LS;
+  }
+  template <int... G>
+  static constexpr int batch_in(int b, std::integer_sequence<int, G...>) {
+    return ((I::batch_of(G) == b ? group_size<G>() : 0) + ... + 0);
+  }
+  template <int B>
+  struct Batch {
+    static constexpr int FG = I::face_group(B);
+    using F = FaceInfo<Phys, FG>;
+    static constexpr int NS = I::slots(B), NG = I::grads(B);
+    static constexpr int IN = batch_in(B, typename I::Seq{});
+    // face traces: of the own x-faces (and up to two neighbours outside the CTA per side), of the
+    // z-neighbours, and of the own z-faces for face-only fields
+    static constexpr int NX = 2 * F::NF * TXS, NZ = 2 * F::NF * RS, NO = 2 * (F::NF - F::NC) * RS;
+    static constexpr int TR = NX + NZ + NO;
+    // lines of cell fields (they precede those of face-only fields), of gradient fields (the last
+    // of them), of face fields
+    static constexpr int NLC = (NS - NG) * CB, NLG = NG * CB, NLF = F::NF * CB;
+  };
+  template <class F, int... B>
+  static constexpr int over(F f, std::integer_sequence<int, B...>) {
+    int m = 0;
+    ((m = imax(m, f(std::integral_constant<int, B>{}))), ...);
+    return m;
+  }
+  using BSeq = std::make_integer_sequence<int, NB>;
+  static constexpr int R_EO = up(over([](auto b) { return Batch<decltype(b)::value>::NS * SLS; }, BSeq{}));
+  static constexpr int R_IN = up(over([](auto b) { return Batch<decltype(b)::value>::IN; }, BSeq{}));
+  static constexpr int R_TR = up(over([](auto b) { return Batch<decltype(b)::value>::TR; }, BSeq{}));
+  static constexpr int NTF = over([](auto b) { return Batch<decltype(b)::value>::F::NF; }, BSeq{});
+  static constexpr int NTL = over([](auto b) { return Batch<decltype(b)::value>::NLC; }, BSeq{});
+  static constexpr int NTT = imax(1, over([](auto b) { return Batch<decltype(b)::value>::NLF; }, BSeq{}));
+  static_assert(NB == 1 || I::grads(0) == 0, "gradient fields in a policy of several batches");
+  static_assert(imax(R_EO, imax(R_IN, R_TR)) < 65536, "offsets of the line tables");
+  // x-face fluxes, then their z-contracted rows
+  static constexpr int R_FX = Phys::FACES ? up(2 * NOUT * RS) : 0;
+  // accumulators after the z pass: per output the rows tested with phi and with d/dxi phi, then
+  // the contracted x-face fluxes [face][output][row][cell]
+  static constexpr int O_XF = NOUT * (Phys::has_grad(0) ? 2 : 1) * P1 * RS;
+  static constexpr int R_ACC = up(O_XF + (Phys::FACES ? 2 * NOUT * P1 * CB : 0));
+  static constexpr int R_OUT = up(NOUT * CB * NDP);
+  static constexpr int O_IN = R_EO, O_TR = O_IN + R_IN;
+  // the x-face fluxes of a single batch take the place of its staged nodes, which the line tasks
+  // have consumed; those of several batches are summed in a region of their own
+  static constexpr int O_FX1 = imax(R_EO, R_ACC);
+  static constexpr bool FX_IN = NB == 1 && O_FX1 + R_FX <= O_TR;
+  static constexpr int O_FX = FX_IN ? O_FX1 : imax(O_TR + R_TR, R_ACC);
+  static constexpr int O_OUT = R_ACC;
+  static constexpr int BASE = imax(imax(O_TR + R_TR, O_FX + R_FX), O_OUT + R_OUT);
+  // per cell: A, B, C (bilinear map), v0, edges of the faces xi = 1 and eta = 1 (two each)
+  static constexpr int GS = 13;
+  static constexpr int O_GEO = BASE;
   // region E (epilogue policies): the CTA's Gauss-point inverse weights, 16-byte aligned
-  static constexpr int OE = (RA + RB2 + R_FLUX + R_GEO + R_S + ALIGN - 1) / ALIGN * ALIGN;
+  static constexpr int EPI = EpiOf<Phys>::value;
   // (EPI 2 and 3 also prefetch the residual (or z), the previous direction and the iterate of
   // their cells: NE chunks)
-  static constexpr int TOTAL = EPI ? OE + NE * CB * ND : RA + RB2 + R_FLUX + R_GEO + R_S;
-  // the epilogue's scratch (input rows and half-transformed values) lives in region A
-  static_assert(EPI == 0 || RA >= (NOUT + 1) * CB * ND, "region A too small for the epilogue");
+  static constexpr int NE = EPI >= 2 ? 4 : 1;
+  static constexpr int OE = up(O_GEO + CB * GS);
+  static constexpr int TOTAL = EPI ? OE + NE * CB * ND : O_GEO + CB * GS;
+  // the epilogue's scratch (input rows and half-transformed values) lives in the accumulators' place
+  static_assert(EPI == 0 || O_OUT >= (NOUT + 1) * CB * ND, "accumulator region too small for the epilogue");
   static constexpr size_t BYTES = sizeof(R) * TOTAL;
-  static_assert(BYTES <= 227 * 1024, "shared memory of one CTA above the sm_100 limit");
+  // static shared memory: tables, neighbours, barriers (bound)
+  static constexpr int STATIC = 2 * NB * (NTL + 2 * NTT) + 12 * NB * NTF + 16 * CB + 4 * NOUT + 64;
+  static constexpr size_t MAX_BYTES = 225 * 1024;  // 227 KB per CTA, up to 2 KB of it static
+  // CTAs per SM, the hint of __launch_bounds__: as many as the shared memory holds, at most three
+  static constexpr int FIT = (int)(228 * 1024 / (BYTES + 1024 + STATIC));
+  static constexpr int MOST = P >= 5 ? 2 : 3;  // degrees 5 and 6 need more than 168 registers
+  static constexpr int CTAS = FIT < 1 ? 1 : (FIT > MOST ? MOST : FIT);
 };
+
+// The most cells per CTA, from CB down in steps of two, with which two CTAs share an SM (one, when
+// two do not fit even with two cells).
+template <int P, class Phys, int CB>
+constexpr int fit_cells() {
+  constexpr size_t bytes = Layout<P, Phys, CB>::BYTES;
+  if constexpr (2 * (bytes + 2048) <= 228 * 1024 || CB <= 2) return CB;
+  else return fit_cells<P, Phys, CB - 2>();
+}
 
 // even/odd contraction of a P1-vector r along one direction to NQ values
 template <int P, class R, int NQ>
@@ -460,21 +564,20 @@ __device__ __forceinline__ void contract_eo(const R* r, R* y) {
   const R rm = T::MIDN ? r[P / 2] : 0.0;
 #pragma unroll
   for (int k = 0; k < T::QH; ++k) {
-    R e = 0.0, o = 0.0;
+    R e = T::MIDN ? t.Sm[k] * rm : t.Se[k][0] * re[0], o = t.So[k][0] * ro[0];
 #pragma unroll
     for (int i = 0; i < T::H; ++i) {
-      e = fmaR(t.Se[k][i], re[i], e);
-      o = fmaR(t.So[k][i], ro[i], o);
+      if (T::MIDN || i > 0) e = fmaR(t.Se[k][i], re[i], e);
+      if (i > 0) o = fmaR(t.So[k][i], ro[i], o);
     }
-    if (T::MIDN) e = fmaR(t.Sm[k], rm, e);
     y[k] = e + o;
     y[T::NQ - 1 - k] = e - o;
   }
   if constexpr (T::QMID) {  // the middle point sees the even part only
-    R e = 0.0;
+    R e = T::MIDN ? t.Sm[T::QH] * rm : t.Se[T::QH][0] * re[0];
 #pragma unroll
-    for (int i = 0; i < T::H; ++i) e = fmaR(t.Se[T::QH][i], re[i], e);
-    if (T::MIDN) e = fmaR(t.Sm[T::QH], rm, e);
+    for (int i = 0; i < T::H; ++i)
+      if (T::MIDN || i > 0) e = fmaR(t.Se[T::QH][i], re[i], e);
     y[T::QH] = e;
   }
 }
@@ -505,41 +608,75 @@ __device__ __forceinline__ void contract_eo_D(const R* r, R* y) {
   }
 }
 
+// transposed contraction of NQ values f to P1 values y[i] = sum_q S[q][i] f[q]
+template <int P, class R, int NQ>
+__device__ __forceinline__ void contract_eo_T(const R* f, R* y) {
+  using T = TabT<P, R, NQ>;
+  const T& t = tabr<P, R, NQ>();
+  R e[T::H > 0 ? T::H : 1], o[T::H > 0 ? T::H : 1], mid = R(0);
+#pragma unroll
+  for (int i = 0; i < T::H; ++i) {
+    e[i] = T::QMID ? t.Se[T::QE - 1][i] * f[T::QE - 1] : R(0);
+    o[i] = R(0);
+  }
+  if (T::MIDN && T::QMID) mid = t.Sm[T::QE - 1] * f[T::QE - 1];
+#pragma unroll
+  for (int k = 0; k < T::QH; ++k) {
+    const R s = f[k] + f[NQ - 1 - k], d = f[k] - f[NQ - 1 - k];
+#pragma unroll
+    for (int i = 0; i < T::H; ++i) {
+      e[i] = fmaR(t.Se[k][i], s, e[i]);
+      o[i] = fmaR(t.So[k][i], d, o[i]);
+    }
+    if (T::MIDN) mid = fmaR(t.Sm[k], s, mid);
+  }
+#pragma unroll
+  for (int i = 0; i < T::H; ++i) {
+    y[i] = e[i] + o[i];
+    y[P - i] = e[i] - o[i];
+  }
+  if (T::MIDN) y[P / 2] = mid;
+}
+
 // ----------------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------------
-template <int P, class Phys, int CB_ = cells_per_block<P>(), int MINB = min_blocks_per_sm<P>()>
+template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>(), int MINB = Layout<P, Phys, CB_>::CTAS>
 __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
-    k_cellop(const MeshDev mesh, const ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>> ptr,
-             const typename Phys::Params prm, const int ncell) {
+    k_cellop(const __grid_constant__ MeshDev mesh,
+             const __grid_constant__ ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>> ptr,
+             const __grid_constant__ typename Phys::Params prm, const int ncell) {
   using L = Layout<P, Phys, CB_>;
+  using I = PhysInfo<Phys>;
   using R = RealOf<Phys>;
   using T = typename L::T;
-  constexpr int P1 = L::P1, NQ = L::NQ, ND = L::ND, CB = L::CB, NT = L::NT;
+  constexpr int P1 = L::P1, NQ = L::NQ, ND = L::ND, CB = L::CB, NT = L::NT, NQP = L::NQP, RS = L::RS;
   constexpr int H = T::H;
   constexpr bool MIDN = T::MIDN;
   constexpr int QH = T::QH;  // quadrature point pairs (q, NQ-1-q); middle point QH if T::QMID
-  constexpr int NOUT = Phys::NOUT;
-  constexpr int NFC_ALL = L::NFC;
+  constexpr int NOUT = Phys::NOUT, NB = L::NB;
   const T& tb = tabr<P, R, NQ>();
+  static_assert(L::BYTES <= L::MAX_BYTES, "shared memory of one CTA above the sm_100 limit");
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* smem = reinterpret_cast<R*>(smem_raw);
-  R* s_eo = smem;             // region A
-  R* s_acc = smem;            //   (after the z pass)
-  R* s_in0 = smem + L::RA;    // region B
-  R* s_nb = s_in0 + L::R_IN;
-  R* s_out = s_in0;           //   (after the last group)
-  R* s_in2 = smem + L::RA + (L::RB2 - L::R_IN2);  // second input buffer (Layout::PREFETCH)
-  R* s_flux = smem + L::RA + L::RB2;
-  R* s_geo = s_flux + L::R_FLUX;
-  R* s_S = s_geo + L::R_GEO;
-  R* s_w = s_S + NQ * P1;
-
-  // bulk-copy completion (Layout::BULK), one barrier per input buffer
-  __shared__ alignas(8) unsigned long long s_bar[2];
-  const unsigned bar = (unsigned)__cvta_generic_to_shared(&s_bar[0]);
-  const unsigned bar2 = (unsigned)__cvta_generic_to_shared(&s_bar[1]);
+  R* const smem = reinterpret_cast<R*>(smem_raw);
+  R* const s_eo = smem;              // x-contracted rows of the batch
+  R* const s_acc = smem;             //   (after the z pass)
+  R* const s_tr = smem + L::O_TR;    // face traces of the batch
+  R* const s_fx = smem + L::O_FX;    // x-face fluxes
+  R* const s_out = smem + L::O_OUT;  //   (after the z pass)
+  R* const s_geo = smem + L::O_GEO;
+  // neighbours of the CTA's cells: x-faces: the slot of the neighbour's trace (-1: wall), z-faces: 0 or -1
+  __shared__ int s_nb[4 * CB];
+  // line tables: per cell line its place in the x-contracted rows, per face line its place in the
+  // input buffer and in the traces; per face field its global array and the array's components
+  __shared__ unsigned short s_line[NB * L::NTL], s_tsrc[NB * L::NTT], s_tdst[NB * L::NTT];
+  __shared__ int s_tc[Phys::FACES ? NB * L::NTF : 1];
+  __shared__ const R* s_tp[Phys::FACES ? NB * L::NTF : 1];
+  __shared__ int s_to[NOUT];
+  // completion of the input buffer's bulk copies
+  __shared__ alignas(8) unsigned long long s_bar;
+  const unsigned bar = (unsigned)__cvta_generic_to_shared(&s_bar);
   pdl_allow_next();
   if (mesh.test_wait_polls > 0) {
     // test hook: the bounded wait gives up on a phase that nobody completes (s_bar is armed
@@ -553,160 +690,55 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
     }
     if (__syncthreads_or(!ok)) return;
   }
+  const int tid = threadIdx.x;
   const int c0 = mesh.cell0 + blockIdx.x * CB;
   const int ncb = min(CB, ncell - c0);  // valid cells in this block
-  // own cells of a group: the contiguous chunk of each array, by one bulk copy per array (TMA)
-  // when the layout allows (uniform per CTA), otherwise by coalesced per-element copies
-  const bool bulk = L::BULK && ((size_t)ncb * ND * sizeof(R)) % 16 == 0;
-  // issued by warp 0 (lane 0 alone without padding): group G's chunks into input buffer G % 2
-  // (buffer 0 without prefetch)
-  auto issue_group = [&](auto gc) {
-    constexpr int G = decltype(gc)::value;
-    using Gi = GroupInfo<Phys, G>;
-    using Gr = typename Phys::template Grp<G>;
-    R* buf = (L::PREFETCH && (G & 1)) ? s_in2 : s_in0;
-    const unsigned gbar = (L::PREFETCH && (G & 1)) ? bar2 : bar;
-    const int lane = threadIdx.x;
-    if (lane == 0) {
+  // bulk staging when every chunk starts and ends on 16 bytes (uniform per CTA); a chunk starts
+  // off a boundary only with an odd number of nodes per cell and an odd first cell
+  const bool bulk = L::BULK && ((size_t)ncb * ND * sizeof(R)) % 16 == 0 && ((size_t)c0 * ND * sizeof(R)) % 16 == 0;
+  // batch B's arrays into its input buffer, by warp 0 (lane 0 alone without padding)
+  auto issue_batch = [&](auto bc) {
+    constexpr int B = decltype(bc)::value;
+    R* const buf = smem + L::O_IN;
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    if (tid == 0) {
       unsigned bytes = 0;
-      sfor<Gi::NARR>([&](auto ac) { bytes += (unsigned)(ncb * Gr::ncomp(decltype(ac)::value) * ND * sizeof(R)); });
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(gbar), "r"(bytes) : "memory");
-    }
-    if constexpr (L::PADB == 0) {
-      if (lane == 0) {
-        sfor<Gi::NARR>([&](auto ac) {
-          constexpr int A = decltype(ac)::value;
-          constexpr int NC = Gr::ncomp(A);
-          constexpr int fb = [] { int b = 0; for (int a = 0; a < A; ++a) b += Gr::ncomp(a); return b; }();
-          const R* src = ptr.in[Gi::arr_base() + A] + (size_t)c0 * NC * ND;
-          const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + fb * CB * ND);
-          asm volatile(
-              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                  dst),
-              "l"(src), "r"((unsigned)(ncb * NC * ND * sizeof(R))), "r"(gbar)
-              : "memory");
-        });
-      }
-    } else {
-      // one copy per (array, cell), spread over the lanes of warp 0; every chunk and slot is a
-      // multiple of 16 bytes (ND * 8 = 288 bytes, slots of 304 and 592), so both addresses stay
-      // 16-byte aligned
-      __syncwarp();
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      sfor<Gi::NARR>([&](auto ac) {
-        constexpr int A = decltype(ac)::value;
-        constexpr int NC = Gr::ncomp(A);
-        constexpr int ab = [] { int b = 0; for (int a = 0; a < A; ++a) b += CB * L::slot(Gr::ncomp(a)); return b; }();
-        const R* src = ptr.in[Gi::arr_base() + A] + (size_t)c0 * NC * ND;
-        for (int cc = lane; cc < ncb; cc += 32) {
-          const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + ab + cc * L::slot(NC));
-          asm volatile(
-              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                  dst),
-              "l"(src + (size_t)cc * NC * ND), "r"((unsigned)(NC * ND * sizeof(R))), "r"(gbar)
-              : "memory");
-        }
+      sfor<Phys::NG>([&](auto gc) {
+        constexpr int G = decltype(gc)::value;
+        if constexpr (I::batch_of(G) == B) bytes += (unsigned)(ncb * GroupInfo<Phys, G>::NF * ND * sizeof(R));
       });
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
     }
-  };
-  // neighbours' face nodes of a face group (L2-resident), ordered along the face parameter, by
-  // per-element asynchronous copies; one element per thread for each (face, field):
-  // CB * P1 <= NT for every degree
-  auto gather_neighbours = [&](auto gc) {
-    constexpr int G = decltype(gc)::value;
-    using Gi = GroupInfo<Phys, G>;
-    using Gr = typename Phys::template Grp<G>;
-    constexpr int NF = Gi::NF;
-    static_assert(CB * P1 <= NT, "neighbour staging assumes one element per thread");
-    const int tid = threadIdx.x;
-    const int cc = tid / P1, i = tid % P1;
-    if (tid < CB * P1) {
-      int nbs[4];
-      cell_neighbours(mesh, c0 + (cc < ncb ? cc : ncb - 1), nbs);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        const int nb = nbs[f];
-        const bool ok = nb >= 0 && cc < ncb;
-        const int kk = f == 0 ? i * P1 + P : (f == 1 ? i * P1 : (f == 2 ? P * P1 + i : i));
+    if constexpr (L::PADB > 0) __syncwarp();
+    sfor<Phys::NG>([&](auto gc) {
+      constexpr int G = decltype(gc)::value;
+      if constexpr (I::batch_of(G) == B) {
+        using Gi = GroupInfo<Phys, G>;
         sfor<Gi::NARR>([&](auto ac) {
           constexpr int A = decltype(ac)::value;
-          constexpr int NC = Gr::ncomp(A);
-          constexpr int fb = [] { int b = 0; for (int a = 0; a < A; ++a) b += Gr::ncomp(a); return b; }();
-          const R* base = ptr.in[Gi::arr_base() + A];
-#pragma unroll
-          for (int d = 0; d < NC; ++d) {
-            R* dst = &s_nb[((f * NF + fb + d) * CB + cc) * L::P1P + i];
-            if (ok) cp_async_el(dst, base + (size_t)nb * NC * ND + d * ND + kk);
-            else *dst = 0.0;
-          }
+          constexpr int NC = Gi::Gr::ncomp(A);
+          const R* src = ptr.in[I::arr_base(G) + A] + (size_t)c0 * NC * ND;
+          const unsigned dst = (unsigned)__cvta_generic_to_shared(buf + L::template line_base<G>(A) * L::LS);
+          // one copy per array, or one per line (every chunk and slot a multiple of 16 bytes)
+          for (int cc = tid; cc < (L::PADB ? ncb * NC : 1); cc += 32)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                    dst + (unsigned)(cc * L::LS * (int)sizeof(R))),
+                "l"(src + (size_t)cc * ND), "r"((unsigned)((L::PADB ? 1 : ncb * NC) * ND * sizeof(R))), "r"(bar)
+                : "memory");
         });
       }
-    }
+    });
   };
-  // shared-memory offset of field fi (group-local) of cell cl_ in the staged nodes of group G
-  auto field_offset = [&](auto gc, int fi, int cl_) -> int {
-    constexpr int G = decltype(gc)::value;
-    using Gi = GroupInfo<Phys, G>;
-    using Gr = typename Phys::template Grp<G>;
-    if constexpr (!L::BULK) {
-      return (fi * CB + cl_) * L::NDP;
-    } else {
-      int off = 0, fb = 0, ab = 0;
-#pragma unroll
-      for (int a = 0; a < Gi::NARR; ++a) {
-        const int nc = Gr::ncomp(a);
-        if (fi >= fb && fi < fb + nc) off = ab + cl_ * L::slot(nc) + (fi - fb) * ND;
-        fb += nc;
-        ab += CB * L::slot(nc);
-      }
-      return off;
-    }
-  };
-  // numerical flux of face group G on face f of this thread's cell at face point q, times the
-  // face JxW: the own trace from the group's staged nodes, the neighbour's from its gathered
-  // face nodes; sq = the basis at point q
-  auto face_flux = [&](auto gc, int f, int q, const R* sq, R* fo) {
-    constexpr int G = decltype(gc)::value;
-    constexpr int NF = GroupInfo<Phys, G>::NF;
-    const R* sin = (L::PREFETCH && (G & 1)) ? s_in2 : s_in0;
-    const int cl_ = threadIdx.x % CB;
-    const R* g = s_geo + cl_ * L::GS;
-    const int nb = get_index(g[20 + f]);
-    R vp[NF], vm[NF];
-#pragma unroll
-    for (int fi = 0; fi < NF; ++fi) {
-      const R* cell = sin + field_offset(gc, fi, cl_);
-      const R* nbv = s_nb + ((f * NF + fi) * CB + cl_) * L::P1P;
-      R a = 0.0, b = 0.0;
-#pragma unroll
-      for (int i = 0; i < P1; ++i) {
-        const int kk = f == 0 ? i * P1 : (f == 1 ? i * P1 + P : (f == 2 ? i : P * P1 + i));
-        a = fmaR(sq[i], cell[kk], a);
-        b = fmaR(sq[i], nbv[i], b);
-      }
-      vp[fi] = a;
-      vm[fi] = b;
-    }
-    const R n[2] = {g[8 + 3 * f], g[9 + 3 * f]};
-    const R jxw = g[10 + 3 * f] * s_w[q];
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) fo[o] = 0.0;
-    if (nb >= 0) Phys::template face<G>(prm, vp, vm, n, fo);
-    else Phys::template boundary<G>(prm, vp, n, fo);
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) fo[o] *= jxw;
-  };
-  // per barrier: the phase a wait expects, and whether copies were issued and not yet waited for
-  unsigned ph[2] = {0u, 0u};
-  bool pending[2] = {false, false};
+  // copies were issued and not yet waited for; their phase
+  bool pending = L::BULK && bulk;
+  unsigned phase = 0u;
   if constexpr (L::BULK) {
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
-      if (L::PREFETCH) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar2) : "memory");
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
-    pending[0] = bulk;
+    if (L::PADB > 0 && tid < 32) __syncwarp();
   }
 
   bool abort = false;
@@ -718,34 +750,30 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
   bool epi_bulk = false;
   const R* epi_src[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t epi_bytes = 0;
-  int epi_ncb = 0;
   if constexpr (L::EPI != 0) {
-    const int c0e = mesh.cell0 + blockIdx.x * CB;
-    epi_ncb = min(CB, ncell - c0e);
-    epi_bytes = sizeof(R) * (size_t)epi_ncb * ND;
-    epi_src[0] = prm.inv + (size_t)c0e * ND;
+    epi_bytes = sizeof(R) * (size_t)ncb * ND;
+    epi_src[0] = prm.inv + (size_t)c0 * ND;
     if constexpr (L::EPI >= 2) {
-      epi_src[1] = prm.r + (size_t)c0e * ND;
-      epi_src[2] = prm.din + (size_t)c0e * ND;
-      epi_src[3] = prm.x + (size_t)c0e * ND;
+      epi_src[1] = prm.r + (size_t)c0 * ND;
+      epi_src[2] = prm.din + (size_t)c0 * ND;
+      epi_src[3] = prm.x + (size_t)c0 * ND;
     }
     epi_bulk = epi_bytes % 16 == 0;
 #pragma unroll
     for (int k = 0; k < L::NE; ++k) epi_bulk = epi_bulk && (reinterpret_cast<size_t>(epi_src[k]) & 15) == 0;
-    if (epi_bulk && threadIdx.x == 0) {
+    if (epi_bulk && tid == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_e) : "memory");
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
   }
-  // the copies that read what earlier kernels wrote: group 0's own-cell chunks (bulk layout)
-  // and the epilogue's chunks
+  // the copies that read what earlier kernels wrote: batch 0 (bulk layout) and the epilogue's chunks
   auto issue_inputs = [&]() {
     if constexpr (L::BULK) {
-      if (threadIdx.x < L::ISSUE_LANES && bulk) issue_group(std::integral_constant<int, 0>{});
+      if (tid < L::ISSUE_LANES && bulk) issue_batch(std::integral_constant<int, 0>{});
     }
     if constexpr (L::EPI != 0) {
       if (epi_bulk) {
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar_e),
                        "r"((unsigned)(epi_bytes * L::NE))
                        : "memory");
@@ -760,7 +788,7 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
       } else {
 #pragma unroll
         for (int k = 0; k < L::NE; ++k)
-          for (int e = threadIdx.x; e < epi_ncb * ND; e += L::NT) cp_async_el(&s_minv[k * CB * ND + e], epi_src[k] + e);
+          for (int e = tid; e < ncb * ND; e += NT) cp_async_el(&s_minv[k * CB * ND + e], epi_src[k] + e);
       }
     }
   };
@@ -771,45 +799,74 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
     issue_inputs();
   }
 
-  const int tid = threadIdx.x;
-  const int m = tid / CB;   // member: row / column / face point
-  const int cl = tid % CB;  // cell within the block
-  const int c = c0 + (cl < ncb ? cl : ncb - 1);
+  // two maps of the threads: point map (cell cl, point m) of the z pass and the faces; line map
+  // (cell ct, line mt + NQ k) of the 1D contractions, consecutive threads on consecutive cells
+  const int cl = tid / NQ, m = tid % NQ;
+  const int mt = tid / CB, ct = tid % CB;
+  const int cg = c0 + (ct < ncb ? ct : ncb - 1);  // global index of cell ct
+  const int gi = cg % mesh.nx, gj = cg / mesh.nx;
+  const int clast = c0 + ncb - 1;
 
-  // ---- per-cell geometry and neighbours, spread over the cell's threads (task f < 4: face f,
-  //      task 4: the bilinear map and the neighbour indices); basis copy for runtime indexing
-  for (int k = tid; k < NQ * P1; k += NT) s_S[k] = tb.S[k / P1][k % P1];
-  for (int k = tid; k < NQ; k += NT) s_w[k] = tb.w[k];
-  for (int task = m; task < 5; task += NQ) {
-    const int i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
-    R* g = s_geo + cl * L::GS;
-    if (task == 4) {
-      const double2 v0 = mesh.vtx[j * W + i], v1 = mesh.vtx[j * W + i + 1];
-      const double2 v2 = mesh.vtx[(j + 1) * W + i], v3 = mesh.vtx[(j + 1) * W + i + 1];
-      g[0] = v1.x - v0.x; g[1] = v1.y - v0.y;                        // A = x_xi at eta = 0
-      g[2] = v3.x - v2.x - v1.x + v0.x; g[3] = v3.y - v2.y - v1.y + v0.y;  // B (bilinear term)
-      g[4] = v2.x - v0.x; g[5] = v2.y - v0.y;                        // C = x_eta at xi = 0
-      g[6] = v0.x; g[7] = v0.y;
-      int nb[4];
-      cell_neighbours(mesh, c, nb);
-      put_index(g[20], nb[0]); put_index(g[21], nb[1]); put_index(g[22], nb[2]); put_index(g[23], nb[3]);
-    } else {
-      // faces: 0 (xi=0, edge v0->v2), 1 (xi=1, v1->v3), 2 (eta=0, v0->v1), 3 (eta=1, v2->v3);
-      // a face's normal is formed from its two vertices the same way by both cells
-      const int f = task;
-      const int ia = (f == 1) ? i + 1 : i, ja = (f == 3) ? j + 1 : j;                       // first vertex
-      const int ib = (f == 0) ? i : i + 1, jb = (f == 2) ? j : j + 1;                       // second vertex
-      const double2 a = mesh.vtx[ja * W + ia], b = mesh.vtx[jb * W + ib];
-      const double tx = b.x - a.x, tz = b.y - a.y, len = sqrt(tx * tx + tz * tz);
-      const double sg = (f == 0 || f == 3) ? 1.0 : -1.0;  // outward: (-tz, tx) on faces 0 and 3
-      const double il = sg / len;
-      g[8 + 3 * f] = -tz * il;
-      g[9 + 3 * f] = tx * il;
-      g[10 + 3 * f] = len;
+  // ---- per-cell geometry and neighbours (one row of the line map), tables of the line tasks
+  if (mt == NQ - 1) {
+    const int W = mesh.nx + 1;
+    const double2* v = mesh.vtx + (size_t)gj * W + gi;
+    const double2 v0 = v[0], v1 = v[1], v2 = v[W], v3 = v[W + 1];
+    R* g = s_geo + ct * L::GS;
+    g[0] = v1.x - v0.x; g[1] = v1.y - v0.y;                              // A = x_xi at eta = 0
+    g[2] = v3.x - v2.x - v1.x + v0.x; g[3] = v3.y - v2.y - v1.y + v0.y;  // B (bilinear term)
+    g[4] = v2.x - v0.x; g[5] = v2.y - v0.y;                              // C = x_eta at xi = 0
+    g[6] = v0.x; g[7] = v0.y;
+    // the edges of the faces xi = 1 and eta = 1; those of xi = 0 and eta = 0 are C and A.  A
+    // face's normal is formed from its two vertices the same way by both cells.
+    g[8] = v3.x - v1.x; g[9] = v3.y - v1.y;
+    g[10] = v3.x - v2.x; g[11] = v3.y - v2.y;
+    if constexpr (Phys::FACES) {
+      // x-neighbours in the CTA: their own trace slot; outside it: two extra slots per side, the
+      // first for the cell before (after) the CTA, the second for a periodic one
+      const int nl = gi > 0 ? cg - 1 : (mesh.periodic_x ? cg + mesh.nx - 1 : -1);
+      const int nr = gi < mesh.nx - 1 ? cg + 1 : (mesh.periodic_x ? cg - mesh.nx + 1 : -1);
+      s_nb[4 * ct] = nl < 0 ? -1 : ((nl >= c0 && nl <= clast) ? nl - c0 : CB + (gi > 0 ? 0 : 1));
+      s_nb[4 * ct + 1] = nr < 0 ? -1 : ((nr >= c0 && nr <= clast) ? nr - c0 : CB + (gi < mesh.nx - 1 ? 0 : 1));
+      s_nb[4 * ct + 2] = gj > 0 ? 0 : -1;
+      s_nb[4 * ct + 3] = gj < mesh.nz - 1 ? 0 : -1;
     }
   }
-  if (Phys::FACES) {
-    for (int k = tid; k < L::R_FLUX; k += NT) s_flux[k] = 0.0;
+  sfor<Phys::NG>([&](auto gc) {
+    constexpr int G = decltype(gc)::value, B = I::batch_of(G);
+    using Gi = GroupInfo<Phys, G>;
+    using F = FaceInfo<Phys, Gi::FACE ? G : -1>;
+    sfor<Gi::NARR>([&](auto ac) {
+      constexpr int A = decltype(ac)::value, NC = Gi::Gr::ncomp(A), f0 = Gi::first_field(A);
+      constexpr bool cell_field = !Gi::Gr::face_only(A), face_field = Gi::FACE && FaceFieldOf<Phys>::get(G, f0);
+      constexpr int k0 = F::before(f0);  // face fields before this array's
+      static_assert(!cell_field || L::template line_base<G>(A) + CB * NC <= L::NTL, "line outside its table");
+      static_assert(!face_field || k0 * CB + CB * NC <= L::NTT, "face line outside its table");
+      for (int t = tid; t < CB * NC; t += NT) {
+        const int cc = t / NC, d = t % NC, line = L::template line_base<G>(A) + t;
+        if (cell_field) s_line[B * L::NTL + line] = (unsigned short)((I::slot_offset(G) + f0 + d) * L::SLS + cc * NQP);
+        if (face_field) {
+          s_tsrc[B * L::NTT + k0 * CB + t] = (unsigned short)(line * L::LS);
+          s_tdst[B * L::NTT + k0 * CB + t] = (unsigned short)((k0 + d) * L::TXS + cc * NQP);
+        }
+      }
+      if constexpr (face_field) {
+        if (tid < NC) {
+          s_tc[B * L::NTF + k0 + tid] = NC;
+          s_tp[B * L::NTF + k0 + tid] = ptr.in[I::arr_base(G) + A] + tid * ND;
+        }
+      }
+    });
+  });
+  if (tid < 32) {
+    sfor<Phys::NOUT_ARR>([&](auto oc) {
+      constexpr int OA = decltype(oc)::value, NC = Phys::out_ncomp(OA);
+      constexpr int ob = [] { int b = 0; for (int a = 0; a < OA; ++a) b += Phys::out_ncomp(a); return b; }();
+      sfor<NC>([&](auto dc) {
+        constexpr int d = decltype(dc)::value;
+        if (tid == ob + d) s_to[ob + d] = L::EPI ? ((ob + d) * CB * L::NDP) | (L::NDP << 20) : (ob * CB * ND + d * ND) | ((NC * ND) << 20);
+      });
+    });
   }
   // geometry-first prologue: everything above read only the mesh vertices and the constant
   // tables, which no kernel writes just before a cell-operator launch; from here on the
@@ -818,138 +875,9 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
     pdl_wait_previous();
     issue_inputs();
   }
+  __syncthreads();  // geometry and tables visible
 
-  // ================= per group: stage, x pass (to region A), face terms =================
-  sfor<Phys::NG>([&](auto gc) {
-    constexpr int G = decltype(gc)::value;
-    using Gi = GroupInfo<Phys, G>;
-    using Gr = typename Phys::template Grp<G>;
-    constexpr int NF = Gi::NF, NFC = Gi::NF_CELL;
-    constexpr int EOFF = PhysInfo<Phys>::eo_offset(G);
-    constexpr bool GFACE = Phys::FACES && Gr::FACE;
-
-    constexpr int B = (L::PREFETCH && (G & 1)) ? 1 : 0;  // this group's input buffer and barrier
-    R* const s_in = B ? s_in2 : s_in0;
-
-    if (abort) return;
-    __syncthreads();  // the buffer of group G-1 and the neighbour area free / geometry visible
-    if (bulk) {
-      // group 0 was issued at kernel entry; with prefetch, group G+1 goes into the other buffer
-      // now (group G-1 has finished reading it), otherwise group G is issued here
-      if constexpr (L::PREFETCH) {
-        if constexpr (G + 1 < Phys::NG) {
-          if (tid < L::ISSUE_LANES) issue_group(std::integral_constant<int, G + 1>{});
-          pending[B ^ 1] = true;
-        }
-      } else if constexpr (G > 0) {
-        if (tid < L::ISSUE_LANES) issue_group(std::integral_constant<int, G>{});
-        pending[0] = true;
-      }
-    } else {
-      sfor<Gi::NARR>([&](auto ac) {
-        constexpr int A = decltype(ac)::value;
-        constexpr int NC = Gr::ncomp(A);
-        constexpr int fb = [] { int b = 0; for (int a = 0; a < A; ++a) b += Gr::ncomp(a); return b; }();
-        const R* src = ptr.in[Gi::arr_base() + A] + (size_t)c0 * NC * ND;
-        for (int e = tid; e < ncb * NC * ND; e += NT) {
-          if constexpr (L::BULK) {
-            // [cell][comp][node] in the slots of the bulk layout
-            constexpr int ab = [] { int b = 0; for (int a = 0; a < A; ++a) b += CB * L::slot(Gr::ncomp(a)); return b; }();
-            cp_async_el(&s_in[ab + (e / (NC * ND)) * L::slot(NC) + e % (NC * ND)], src + e);
-          } else {
-            const int cc = e / (NC * ND), r = e % (NC * ND);
-            cp_async_el(&s_in[((fb + r / ND) * CB + cc) * L::NDP + r % ND], src + e);
-          }
-        }
-      });
-    }
-    auto foff = [&](int fi, int cl_) -> int { return field_offset(gc, fi, cl_); };
-    if constexpr (GFACE) gather_neighbours(gc);
-    cp_async_wait_all();
-    if (bulk) {
-      const bool ok = mbar_wait(B ? bar2 : bar, ph[B]);
-      if (ok) {
-        ph[B] ^= 1u;
-        pending[B] = false;
-      }
-      if (!ok) report_status(mesh.status, kStatusStageTimeout);
-      if (__syncthreads_or(!ok)) {  // every thread leaves together, nothing waits on a barrier
-        abort = true;
-        return;
-      }
-    } else {
-      __syncthreads();
-    }
-    // ---- X pass: rows (k, P-k) even/odd, contracted along x, for the cell fields (S) and
-    //      again for the gradient fields (D, slots NFC..NFC+NFG-1)
-    {
-      constexpr int NPR = H + (MIDN ? 1 : 0);
-      constexpr int NFG = Gi::NF_GRAD;
-      for (int task = m; task < (NFC + NFG) * NPR; task += NQ) {
-        const int fi = task / NPR, k = task % NPR;
-        const bool dxi = NFG > 0 && fi >= NFC;
-        const int src = dxi ? fi - NFG : fi;  // gradient fields are the last NFG cell fields
-        const R* cell = s_in + foff(src, cl);
-        R* eo = s_eo + ((EOFF + fi) * CB + cl) * L::EOS;
-        R r[P1], y[NQ];
-        auto contract = [&]() {
-          if (NFG > 0 && dxi) contract_eo_D<P, R, NQ>(r, y);
-          else contract_eo<P, R, NQ>(r, y);
-        };
-        if (k < H) {
-#pragma unroll
-          for (int ix = 0; ix < P1; ++ix) r[ix] = cell[k * P1 + ix] + cell[(P - k) * P1 + ix];
-          contract();
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) eo[k * NQ + q] = y[q];
-#pragma unroll
-          for (int ix = 0; ix < P1; ++ix) r[ix] = cell[k * P1 + ix] - cell[(P - k) * P1 + ix];
-          contract();
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) eo[(H + k) * NQ + q] = y[q];
-        } else {
-#pragma unroll
-          for (int ix = 0; ix < P1; ++ix) r[ix] = cell[(P / 2) * P1 + ix];
-          contract();
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) eo[(2 * H) * NQ + q] = y[q];
-        }
-      }
-    }
-    // ---- faces (same phase: reads region B only): member = face quadrature point; the
-    //      z-faces of a folding layout come after the z pass
-    if constexpr (GFACE) {
-      const int q = m;
-      R sq[P1];
-#pragma unroll
-      for (int i = 0; i < P1; ++i) sq[i] = s_S[q * P1 + i];
-#pragma unroll
-      for (int f = 0; f < (L::FOLD_Z ? 2 : 4); ++f) {
-        R fo[NOUT];
-        face_flux(gc, f, q, sq, fo);
-#pragma unroll
-        for (int o = 0; o < NOUT; ++o) s_flux[((f * NOUT + o) * CB + cl) * NQ + q] += fo[o];
-      }
-    }
-  });
-  if (abort) {  // a staging wait gave up: wait (bounded) for this CTA's copies before leaving
-    if (tid == 0) {
-      if (pending[0]) mbar_wait(bar, ph[0]);
-      if (pending[1]) mbar_wait(bar2, ph[1]);
-      if (epi_bulk) mbar_wait(bar_e, 0);
-    }
-    return;
-  }
-  __syncthreads();
-
-  // ================= merged z pass: member = quadrature column qx =================
-  // All groups' fields are evaluated at each point, their integrands summed, and the sum
-  // is mapped to reference coordinates and contracted along z once.  The contraction of a
-  // point pair (q, NQ-1-q) goes into even/odd accumulators of the node pairs (i, P-i):
-  //   S terms:  E_i += Se[q][i] (f1 + f2),  O_i += So[q][i] (f1 - f2),  mid += Sm[q] (f1 + f2)
-  //   D terms:  E_i += De[q][i] (g1 - g2),  O_i += Do[q][i] (g1 + g2),  mid += Dm[q] (g1 - g2)
-  // (S[NQ-1-q][i] = S[q][P-i], D[NQ-1-q][i] = -D[q][P-i]); node i gets E_i + O_i, node P-i
-  // gets E_i - O_i.  A middle point is a pair with f2 = g2 = 0.
+  // accumulators of the z pass (see below)
   constexpr int HE = H > 0 ? H : 1;
   R aE[NOUT][HE], aO[NOUT][HE], aM[NOUT], bE[NOUT][HE], bO[NOUT][HE], bM[NOUT];
 #pragma unroll
@@ -958,206 +886,449 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
     for (int i = 0; i < HE; ++i) aE[o][i] = aO[o][i] = bE[o][i] = bO[o][i] = R(0);
     aM[o] = bM[o] = R(0);
   }
-  {
-    const int qx = m;
-    const R* g = s_geo + cl * L::GS;
-    const R xi = tb.x[qx];
-    const R wx = s_w[qx];
-    const R J01 = fmaR(g[2], xi, g[4]);  // x_eta (x component)
-    const R J11 = fmaR(g[3], xi, g[5]);  // x_eta (z component)
-    const bool need_x = Phys::NEED_X && PositionUse<typename Phys::Params>::get(prm);
-    constexpr int NFG_ALL = PhysInfo<Phys>::NFG_TOTAL;
-    // the mapped integrands of one point: fv (tested with phi), fx, fe (with d/dxi, d/deta phi)
-    auto integrand = [&](const R* v, const R* deta, const int qz, R* fvo, R* fxo, R* feo) {
-      const R eta = tb.x[qz];
-      const R J00 = fmaR(g[2], eta, g[0]);
-      const R J10 = fmaR(g[3], eta, g[1]);
-      const R w = wx * tb.w[qz];
-      const R dw = (J00 * J11 - J01 * J10) * w;
-      PointGeo pg;
-      if (need_x) {
-        pg.X[0] = g[6] + g[0] * xi + g[4] * eta + g[2] * xi * eta;
-        pg.X[1] = g[7] + g[1] * xi + g[5] * eta + g[3] * xi * eta;
-      }
-      if constexpr (NFG_ALL > 0) {
-        pg.J[0] = J00; pg.J[1] = J01; pg.J[2] = J10; pg.J[3] = J11;
-      }
-      if constexpr (MappedOf<Phys>::value) {  // the policy maps its own integrand
-        const R A[4] = {J11 * w, J01 * w, J10 * w, J00 * w};
+
+  sfor<NB>([&](auto bc) {
+    constexpr int B = decltype(bc)::value;
+    using Bt = typename L::template Batch<B>;
+    using F = typename Bt::F;
+    constexpr int FG = Bt::FG, NFF = F::NF;
+    R* const s_in = smem + L::O_IN;
+    if (abort) return;
+    if (B > 0) __syncthreads();  // the rows and traces of the batch before are free
+
+    // ---- traces of the neighbours' faces, straight from their nodes (L2-resident): one line per
+    //      (z-side, field, cell), and per field up to two cells on either side of the CTA
+    if constexpr (FG >= 0) {
+      constexpr int NZT = (2 * NFF + NQ - 1) / NQ;  // rounds of the z-sides' lines
+      constexpr int NXT = (4 * NFF + NT - 1) / NT;  // rounds of the outer x-neighbours' lines
+#pragma unroll 1
+      for (int t = 0; t < NZT + NXT; ++t) {
+        int k, nb = -1, start, stride;
+        R* dst;
+        if (t < NZT) {
+          const int e = mt + t * NQ, top = e >= NFF ? 1 : 0;
+          k = e - top * NFF;
+          if (e < 2 * NFF) nb = top ? (gj < mesh.nz - 1 ? cg + mesh.nx : -1) : (gj > 0 ? cg - mesh.nx : -1);
+          start = top ? 0 : P * P1;
+          stride = 1;
+          dst = s_tr + Bt::NX + (e * CB + ct) * NQP;
+        } else {
+          const int e = NT - 1 - tid + (t - NZT) * NT, x = e & 3;
+          k = e >> 2;
+          const int first = c0 - c0 % mesh.nx, lrow = clast - clast % mesh.nx;  // rows of the first and last cell
+          if (e >= 4 * NFF) nb = -1;
+          else if (x == 0) nb = c0 > first ? c0 - 1 : -1;
+          else if (x == 1) nb = mesh.periodic_x && lrow >= c0 && lrow + mesh.nx - 1 > clast ? lrow + mesh.nx - 1 : -1;
+          else if (x == 2) nb = clast < lrow + mesh.nx - 1 ? clast + 1 : -1;
+          else nb = mesh.periodic_x && first + mesh.nx - 1 <= clast && first < c0 ? first : -1;
+          start = x < 2 ? P : 0;  // a left neighbour's right face, a right neighbour's left face
+          stride = P1;
+          dst = s_tr + ((x < 2 ? 1 : 0) * NFF + k) * L::TXS + (CB + (x & 1)) * NQP;
+        }
+        if (nb >= 0) {
+          const R* src = s_tp[B * L::NTF + k] + (size_t)nb * (s_tc[B * L::NTF + k] * ND) + start;
+          R r[P1], y[NQ];
 #pragma unroll
-        for (int o = 0; o < NOUT; ++o) fvo[o] = fxo[o] = feo[o] = R(0);
-        sfor<Phys::NG>([&](auto gc) {
-          constexpr int G = decltype(gc)::value;
-          Phys::template point_mapped<G>(prm, v + PhysInfo<Phys>::eo_offset(G), pg, A, dw, fvo, fxo, feo);
-        });
-        return;
-      }
-      R val[NOUT], gr[NOUT][2];
+          for (int i = 0; i < P1; ++i) r[i] = src[i * stride];
+          contract_eo<P, R, NQ>(r, y);
 #pragma unroll
-      for (int o = 0; o < NOUT; ++o) { val[o] = 0.0; gr[o][0] = gr[o][1] = 0.0; }
+          for (int q = 0; q < NQ; ++q) dst[q] = y[q];
+        }
+      }
+    }
+
+    // ---- the own cells' nodes
+    bool ok = true;
+    if (bulk) {
+      ok = mbar_wait(bar, phase);
+      if (ok) {
+        phase ^= 1u;
+        pending = false;
+      } else {
+        report_status(mesh.status, kStatusStageTimeout);
+      }
+    } else {
       sfor<Phys::NG>([&](auto gc) {
         constexpr int G = decltype(gc)::value;
-        if constexpr (NFG_ALL > 0)
-          Phys::template point<G>(prm, v + PhysInfo<Phys>::eo_offset(G), deta + PhysInfo<Phys>::grad_offset(G), pg,
-                                  val, gr);
-        else
-          Phys::template point<G>(prm, v + PhysInfo<Phys>::eo_offset(G), pg, val, gr);
-      });
-      const R a00 = J11 * w, a01 = J01 * w, a10 = J10 * w, a11 = J00 * w;  // adj(J) w
-#pragma unroll
-      for (int o = 0; o < NOUT; ++o) {
-        fvo[o] = val[o] * dw;
-        fxo[o] = a00 * gr[o][0] - a01 * gr[o][1];
-        feo[o] = a11 * gr[o][1] - a10 * gr[o][0];
-      }
-    };
-#pragma unroll kZUnroll
-    for (int k = 0; k < T::QE; ++k) {
-      const bool pair = k < QH;
-      R v1[NFC_ALL], v2[NFC_ALL];
-#pragma unroll
-      for (int fi = 0; fi < NFC_ALL; ++fi) {
-        const R* eo = s_eo + (fi * CB + cl) * L::EOS + qx;
-        R e = 0.0, o = 0.0;
-#pragma unroll
-        for (int i = 0; i < H; ++i) {
-          e = fmaR(tb.Se[k][i], eo[i * NQ], e);
-          if (pair) o = fmaR(tb.So[k][i], eo[(H + i) * NQ], o);
-        }
-        if (MIDN) e = fmaR(tb.Sm[k], eo[(2 * H) * NQ], e);
-        v1[fi] = e + o;
-        v2[fi] = e - o;
-      }
-      // d/deta of the gradient fields: their S-row slots contracted with D along z
-      R d1[NFG_ALL > 0 ? NFG_ALL : 1], d2[NFG_ALL > 0 ? NFG_ALL : 1];
-      if constexpr (NFG_ALL > 0) {
-        sfor<Phys::NG>([&](auto gc) {
-          constexpr int G = decltype(gc)::value;
+        if constexpr (I::batch_of(G) == B) {
           using Gi = GroupInfo<Phys, G>;
-          constexpr int NFG = Gi::NF_GRAD;
+          sfor<Gi::NARR>([&](auto ac) {
+            constexpr int A = decltype(ac)::value;
+            constexpr int NC = Gi::Gr::ncomp(A);
+            const R* src = ptr.in[I::arr_base(G) + A] + (size_t)c0 * NC * ND;
+            for (int e = tid; e < ncb * NC * ND; e += NT)
+              cp_async_el(&s_in[(L::template line_base<G>(A) + e / ND) * L::LS + e % ND], src + e);
+          });
+        }
+      });
+      cp_async_wait_all();
+      __syncthreads();
+    }
+
+    // ---- line tasks on them: the rows (k, P-k) of every line, even/odd, contracted along x
+    auto load = [&](const R* src, int st, R* r) {
 #pragma unroll
-          for (int kk = 0; kk < NFG; ++kk) {
-            const int slot = PhysInfo<Phys>::eo_offset(G) + Gi::NF_CELL - NFG + kk;
-            const R* eo = s_eo + (slot * CB + cl) * L::EOS + qx;
-            R e = 0.0, o = 0.0;
+      for (int i = 0; i < P1; ++i) r[i] = src[i * st];
+    };
+    auto store = [&](R* dst, const R* y) {
 #pragma unroll
-            for (int i = 0; i < H; ++i) {
-              e = fmaR(tb.De[k][i], eo[i * NQ], e);
-              o = fmaR(tb.Do[k][i], eo[(H + i) * NQ], o);  // at the middle point only o remains
+      for (int q = 0; q < NQ; ++q) dst[q] = y[q];
+    };
+    auto row_pair = [&](int line, int k, auto der) {
+      R a[P1], b[P1], r[P1], y[NQ];
+      load(s_in + line * L::LS + k * P1, 1, a);
+      load(s_in + line * L::LS + (P - k) * P1, 1, b);
+      R* dst = s_eo + s_line[B * L::NTL + line] + (decltype(der)::value ? Bt::NG * L::SLS : 0) + k * RS;
+#pragma unroll
+      for (int i = 0; i < P1; ++i) r[i] = a[i] + b[i];
+      if constexpr (decltype(der)::value) contract_eo_D<P, R, NQ>(r, y);
+      else contract_eo<P, R, NQ>(r, y);
+      store(dst, y);
+#pragma unroll
+      for (int i = 0; i < P1; ++i) r[i] = a[i] - b[i];
+      if constexpr (decltype(der)::value) contract_eo_D<P, R, NQ>(r, y);
+      else contract_eo<P, R, NQ>(r, y);
+      store(dst + H * RS, y);
+    };
+    for (int e = tid; e < H * Bt::NLC; e += NT) row_pair(e % Bt::NLC, e / Bt::NLC, std::false_type{});
+    if constexpr (Bt::NG > 0) {
+      for (int e = tid; e < H * Bt::NLG; e += NT)
+        row_pair(Bt::NLC - Bt::NLG + e % Bt::NLG, e / Bt::NLG, std::true_type{});
+    }
+    //      the middle rows, the traces of the x-faces and of the z-faces of face-only fields (from the
+    //      other end of the CTA, which has fewer row pairs)
+    constexpr int NM = MIDN ? Bt::NLC : 0, NLO = (NFF - F::NC) * CB, NLX = Bt::NLF;
+    for (int e = NT - 1 - tid; e < NM + 2 * NLX + 2 * NLO; e += NT) {
+      const R* src;
+      R* dst;
+      int st = 1;
+      if (e < NM) {
+        src = s_in + e * L::LS + (P / 2) * P1;
+        dst = s_eo + s_line[B * L::NTL + e] + 2 * H * RS;
+      } else if (e < NM + 2 * NLX) {
+        const int f = e >= NM + NLX ? 1 : 0, t = e - NM - f * NLX;
+        src = s_in + s_tsrc[B * L::NTT + t] + f * P;
+        dst = s_tr + s_tdst[B * L::NTT + t] + f * NFF * L::TXS;
+        st = P1;
+      } else {
+        const int f = e >= NM + 2 * NLX + NLO ? 1 : 0, o = e - NM - 2 * NLX - f * NLO, t = NLX - NLO + o;
+        const int p = s_tdst[B * L::NTT + t], k = p / L::TXS;  // face field of the line
+        src = s_in + s_tsrc[B * L::NTT + t] + f * P * P1;
+        dst = s_tr + Bt::NX + Bt::NZ + (f * (NFF - F::NC) + k - F::NC) * RS + (p - k * L::TXS);
+      }
+      R r[P1], y[NQ];
+      load(src, st, r);
+      contract_eo<P, R, NQ>(r, y);
+      store(dst, y);
+    }
+    if constexpr (Bt::NG > 0 && MIDN) {
+      for (int e = NT - 1 - tid; e < Bt::NLG; e += NT) {
+        const int line = Bt::NLC - Bt::NLG + e;
+        R r[P1], y[NQ];
+        load(s_in + line * L::LS + (P / 2) * P1, 1, r);
+        contract_eo_D<P, R, NQ>(r, y);
+        store(s_eo + s_line[B * L::NTL + line] + Bt::NG * L::SLS + 2 * H * RS, y);
+      }
+    }
+    if (__syncthreads_or(!ok)) {  // a staging wait gave up: every thread leaves together
+      abort = true;
+      return;
+    }
+    if constexpr (B + 1 < NB) {  // the line tasks have consumed the buffer: the next batch's nodes
+      if (bulk) {
+        if (tid < L::ISSUE_LANES) issue_batch(std::integral_constant<int, B + 1>{});
+        pending = true;
+      }
+    }
+
+    // ---- faces: numerical flux at face point m of cell cl.  The fluxes are linear in the normal's
+    //      length, so the edge vector times the quadrature weight serves as normal times JxW.  The
+    //      z-faces go into the accumulators of node rows 0 and P (whose weight is theirs, w_m), the
+    //      x-faces to shared memory.
+    const R* const g = s_geo + cl * L::GS;
+    const int pt = cl * NQP + m;
+    if constexpr (FG >= 0) {
+      constexpr int NFG_ = GroupInfo<Phys, FG>::NF;
+      const R wq = tb.w[m];
+      R zb[NFF], zt[NFF];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        if (f == 2) {  // the own traces on eta = 0 and 1: half the sum and difference of the rows 0 +- P
+          sfor<NFF>([&](auto kc) {
+            constexpr int k = decltype(kc)::value;
+            if constexpr (k < F::NC) {
+              const R* e = s_eo + (I::slot_offset(FG) + F::field(k)) * L::SLS + pt;
+              const R a = R(0.5) * e[0], b = e[H * RS];
+              zb[k] = fmaR(R(0.5), b, a);
+              zt[k] = fmaR(R(-0.5), b, a);
+            } else {
+              const R* e = s_tr + Bt::NX + Bt::NZ + (k - F::NC) * RS + pt;
+              zb[k] = e[0];
+              zt[k] = e[(NFF - F::NC) * RS];
             }
-            if (MIDN) e = fmaR(tb.Dm[k], eo[(2 * H) * NQ], e);
-            d1[PhysInfo<Phys>::grad_offset(G) + kk] = e + o;
-            d2[PhysInfo<Phys>::grad_offset(G) + kk] = o - e;
+          });
+        }
+        R vp[NFG_], vm[NFG_], fo[NOUT];
+        const int nb = s_nb[4 * cl + f];
+        if (f < 2) {
+          const R* own = s_tr + f * NFF * L::TXS + pt;
+          const R* oth = s_tr + (1 - f) * NFF * L::TXS + (nb < 0 ? 0 : nb) * NQP + m;
+          sfor<NFF>([&](auto kc) {
+            constexpr int k = decltype(kc)::value;
+            vp[F::field(k)] = own[k * L::TXS];
+            vm[F::field(k)] = oth[k * L::TXS];
+          });
+        } else {
+          sfor<NFF>([&](auto kc) {
+            constexpr int k = decltype(kc)::value;
+            vp[F::field(k)] = f == 2 ? zb[k] : zt[k];
+            vm[F::field(k)] = s_tr[Bt::NX + ((f - 2) * NFF + k) * RS + pt];
+          });
+        }
+        constexpr int E0[4] = {4, 8, 0, 10};
+        // outward: (-tz, tx) on faces 0 and 3
+        const R sw = (f == 0 || f == 3 ? R(1) : R(-1)) * (f < 2 ? wq : R(1));
+        const R n[2] = {-sw * g[E0[f] + 1], sw * g[E0[f]]};
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) fo[o] = R(0);
+        if (nb >= 0) Phys::template face<FG>(prm, vp, vm, n, fo);
+        else Phys::template boundary<FG>(prm, vp, n, fo);
+#pragma unroll
+        for (int o = 0; o < NOUT; ++o) {
+          if (f < 2) {
+            R* d = s_fx + (f * NOUT + o) * RS + pt;
+            *d = B > 0 ? *d + fo[o] : fo[o];
+          } else {
+            aE[o][0] += R(0.5) * fo[o];
+            aO[o][0] += (f == 2 ? R(0.5) : R(-0.5)) * fo[o];
+          }
+        }
+        asm volatile("" ::: "memory");  // one face's traces at a time in registers
+      }
+    } else if constexpr (Phys::FACES && B == 0) {
+#pragma unroll
+      for (int o = 0; o < 2 * NOUT; ++o) s_fx[o * RS + pt] = R(0);
+    }
+
+    // ---- z pass: member = quadrature column qx = m.  All fields of the batch are evaluated at each
+    // point, their integrands summed, and the sum is mapped to reference coordinates and
+    // contracted along z once.  The contraction of a point pair (q, NQ-1-q) goes into even/odd
+    // accumulators of the node pairs (i, P-i) (tables with the z weight folded in; the x weight
+    // multiplies the accumulators at the end):
+    //   S terms:  E_i += Se[q][i] (f1 + f2),  O_i += So[q][i] (f1 - f2),  mid += Sm[q] (f1 + f2)
+    //   D terms:  E_i += De[q][i] (g1 - g2),  O_i += Do[q][i] (g1 + g2),  mid += Dm[q] (g1 - g2)
+    // (S[NQ-1-q][i] = S[q][P-i], D[NQ-1-q][i] = -D[q][P-i]); node i gets E_i + O_i, node P-i
+    // gets E_i - O_i.  A middle point is a pair with f2 = g2 = 0.
+    {
+      constexpr int NS = Bt::NS, NGR = Bt::NG;
+      const R xi = tb.x[m];
+      const R J01 = fmaR(g[2], xi, g[4]);  // x_eta (x component)
+      const R J11 = fmaR(g[3], xi, g[5]);  // x_eta (z component)
+      const bool need_x = Phys::NEED_X && PositionUse<typename Phys::Params>::get(prm);
+      const R* const eo = s_eo + pt;
+      // the mapped integrands of one point, up to the quadrature weights: fv (tested with phi), fx,
+      // fe (with d/dxi, d/deta phi)
+      auto integrand = [&](const R* v, const R* deta, const int qz, R* fvo, R* fxo, R* feo) {
+        const R eta = tb.x[qz];
+        const R a11 = fmaR(g[2], eta, g[0]), a10 = fmaR(g[3], eta, g[1]);  // x_xi, z_xi
+        const R dw = a11 * J11 - a10 * J01;
+        PointGeo pg;
+        if (need_x) {
+          pg.X[0] = g[6] + g[0] * xi + g[4] * eta + g[2] * xi * eta;
+          pg.X[1] = g[7] + g[1] * xi + g[5] * eta + g[3] * xi * eta;
+        }
+        if constexpr (NGR > 0) {
+          pg.J[0] = a11; pg.J[1] = J01; pg.J[2] = a10; pg.J[3] = J11;
+        }
+        if constexpr (MappedOf<Phys>::value) {  // the policy maps its own integrand
+          const R A[4] = {J11, J01, a10, a11};
+#pragma unroll
+          for (int o = 0; o < NOUT; ++o) fvo[o] = fxo[o] = feo[o] = R(0);
+          sfor<Phys::NG>([&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            if constexpr (I::batch_of(G) == B)
+              Phys::template point_mapped<G>(prm, v + I::slot_offset(G), pg, A, dw, fvo, fxo, feo);
+          });
+        } else {
+          R val[NOUT], gr[NOUT][2];
+#pragma unroll
+          for (int o = 0; o < NOUT; ++o) { val[o] = 0.0; gr[o][0] = gr[o][1] = 0.0; }
+          sfor<Phys::NG>([&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            if constexpr (I::batch_of(G) == B) {
+              if constexpr (NfgOf<Phys>::any)
+                Phys::template point<G>(prm, v + I::slot_offset(G), deta + I::grad_offset(G), pg, val, gr);
+              else
+                Phys::template point<G>(prm, v + I::slot_offset(G), pg, val, gr);
+            }
+          });
+#pragma unroll
+          for (int o = 0; o < NOUT; ++o) {
+            fvo[o] = val[o] * dw;
+            fxo[o] = J11 * gr[o][0] - J01 * gr[o][1];
+            feo[o] = a11 * gr[o][1] - a10 * gr[o][0];
+          }
+        }
+      };
+#pragma unroll 1
+      for (int k = 0; k < T::QE; ++k) {
+        const bool pair = k < QH;
+        asm volatile("" ::: "memory");  // keeps the rows in shared memory: hoisted, they spill
+        R v1[NS], v2[NS];
+#pragma unroll
+        for (int fi = 0; fi < NS; ++fi) {
+          const R* row = eo + fi * L::SLS;
+          R e = MIDN ? tb.Sm[k] * row[2 * H * RS] : R(0), o = R(0);
+#pragma unroll
+          for (int i = 0; i < H; ++i) {
+            e = fmaR(tb.Se[k][i], row[i * RS], e);
+            o = fmaR(tb.So[k][i], row[(H + i) * RS], o);  // (0 at a middle point)
+          }
+          v1[fi] = e + o;
+          v2[fi] = e - o;
+        }
+        // d/deta of the gradient fields: their S-row slots contracted with D along z
+        R d1[NGR > 0 ? NGR : 1], d2[NGR > 0 ? NGR : 1];
+        if constexpr (NGR > 0) {
+          sfor<Phys::NG>([&](auto gc) {
+            constexpr int G = decltype(gc)::value;
+            if constexpr (I::batch_of(G) == B) {
+              using Gi = GroupInfo<Phys, G>;
+#pragma unroll
+              for (int kk = 0; kk < Gi::NF_GRAD; ++kk) {
+                const R* row = eo + (I::slot_offset(G) + Gi::NF_CELL - Gi::NF_GRAD + kk) * L::SLS;
+                R e = 0.0, o = 0.0;
+#pragma unroll
+                for (int i = 0; i < H; ++i) {
+                  e = fmaR(tb.De[k][i], row[i * RS], e);
+                  o = fmaR(tb.Do[k][i], row[(H + i) * RS], o);  // at the middle point only o remains
+                }
+                if (MIDN) e = fmaR(tb.Dm[k], row[2 * H * RS], e);
+                d1[I::grad_offset(G) + kk] = e + o;
+                d2[I::grad_offset(G) + kk] = o - e;
+              }
+            }
+          });
+        }
+        R fv1[NOUT], fx1[NOUT], fe1[NOUT], fv2[NOUT], fx2[NOUT], fe2[NOUT];
+        integrand(v1, d1, k, fv1, fx1, fe1);
+        if (pair) {
+          integrand(v2, d2, NQ - 1 - k, fv2, fx2, fe2);
+        } else {
+#pragma unroll
+          for (int o = 0; o < NOUT; ++o) fv2[o] = fx2[o] = fe2[o] = R(0);
+        }
+        sfor<NOUT>([&](auto oc) {
+          constexpr int o = decltype(oc)::value;
+          constexpr bool hv = TermsOf<Phys>::val(B, o), hg = TermsOf<Phys>::grad(B, o);
+          const R se = hv ? fv1[o] + fv2[o] : R(0), so = hv ? fv1[o] - fv2[o] : R(0);
+          const R ge = hg ? fe1[o] - fe2[o] : R(0), go = hg ? fe1[o] + fe2[o] : R(0);
+          const R xe = hg ? fx1[o] + fx2[o] : R(0), xo = hg ? fx1[o] - fx2[o] : R(0);
+#pragma unroll
+          for (int i = 0; i < H; ++i) {
+            if (hv) {
+              aE[o][i] = fmaR(tb.SeW[k][i], se, aE[o][i]);
+              aO[o][i] = fmaR(tb.SoW[k][i], so, aO[o][i]);
+            }
+            if (hg) {
+              aE[o][i] = fmaR(tb.DeW[k][i], ge, aE[o][i]);
+              aO[o][i] = fmaR(tb.DoW[k][i], go, aO[o][i]);
+              bE[o][i] = fmaR(tb.SeW[k][i], xe, bE[o][i]);
+              bO[o][i] = fmaR(tb.SoW[k][i], xo, bO[o][i]);
+            }
+          }
+          if (MIDN) {
+            if (hv) aM[o] = fmaR(tb.SmW[k], se, aM[o]);
+            if (hg) {
+              aM[o] = fmaR(tb.DmW[k], ge, aM[o]);
+              bM[o] = fmaR(tb.SmW[k], xe, bM[o]);
+            }
           }
         });
       }
-      R fv1[NOUT], fx1[NOUT], fe1[NOUT], fv2[NOUT], fx2[NOUT], fe2[NOUT];
-      integrand(v1, d1, k, fv1, fx1, fe1);
-      if (pair) {
-        integrand(v2, d2, NQ - 1 - k, fv2, fx2, fe2);
-      } else {
-#pragma unroll
-        for (int o = 0; o < NOUT; ++o) fv2[o] = fx2[o] = fe2[o] = R(0);
-      }
-#pragma unroll
-      for (int o = 0; o < NOUT; ++o) {
-        const bool hv = Phys::has_val(o), hg = Phys::has_grad(o);
-        const R se = hv ? fv1[o] + fv2[o] : R(0), so = hv ? fv1[o] - fv2[o] : R(0);
-        const R ge = hg ? fe1[o] - fe2[o] : R(0), go = hg ? fe1[o] + fe2[o] : R(0);
-        const R xe = fx1[o] + fx2[o], xo = fx1[o] - fx2[o];
-#pragma unroll
-        for (int i = 0; i < H; ++i) {
-          if (hv) {
-            aE[o][i] = fmaR(tb.Se[k][i], se, aE[o][i]);
-            aO[o][i] = fmaR(tb.So[k][i], so, aO[o][i]);
-          }
-          if (hg) {
-            aE[o][i] = fmaR(tb.De[k][i], ge, aE[o][i]);
-            aO[o][i] = fmaR(tb.Do[k][i], go, aO[o][i]);
-            bE[o][i] = fmaR(tb.Se[k][i], xe, bE[o][i]);
-            bO[o][i] = fmaR(tb.So[k][i], xo, bO[o][i]);
-          }
-        }
-        if (MIDN) {
-          if (hv) aM[o] = fmaR(tb.Sm[k], se, aM[o]);
-          if (hg) {
-            aM[o] = fmaR(tb.Dm[k], ge, aM[o]);
-            bM[o] = fmaR(tb.Sm[k], xe, bM[o]);
-          }
-        }
-      }
     }
+  });
+  if (abort) {  // a staging wait gave up: wait (bounded) for this CTA's copies before leaving
+    if (tid == 0) {
+      if (pending) mbar_wait(bar, phase);
+      if (epi_bulk) mbar_wait(bar_e, 0);
+    }
+    return;
   }
-  // node values of the accumulators
-  R acc_a[NOUT][P1], acc_b[NOUT][P1];
-#pragma unroll
-  for (int o = 0; o < NOUT; ++o) {
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      acc_a[o][i] = aE[o][i] + aO[o][i];
-      acc_a[o][P - i] = aE[o][i] - aO[o][i];
-      acc_b[o][i] = bE[o][i] + bO[o][i];
-      acc_b[o][P - i] = bE[o][i] - bO[o][i];
-    }
-    if (MIDN) {
-      acc_a[o][P / 2] = aM[o];
-      acc_b[o][P / 2] = bM[o];
-    }
-  }
-  if constexpr (L::FOLD_Z) {  // z-faces at face point qx = m, into node rows 0 (face 2) and P (3)
-    R sq[P1];
-#pragma unroll
-    for (int i = 0; i < P1; ++i) sq[i] = s_S[m * P1 + i];
-#pragma unroll
-    for (int f = 2; f < 4; ++f) {
-      R fo[NOUT];
-      face_flux(std::integral_constant<int, L::FACE_G>{}, f, m, sq, fo);
-#pragma unroll
-      for (int o = 0; o < NOUT; ++o) acc_a[o][f == 2 ? 0 : P] += fo[o];
-    }
-  }
-  __syncthreads();  // region A: x-contracted rows consumed -> accumulators
+  __syncthreads();  // the x-contracted rows are consumed -> accumulators
   {
-    const int qx = m;
+    const int pt = cl * NQP + m;
+    const R wx = tb.w[m];
 #pragma unroll
     for (int o = 0; o < NOUT; ++o) {
-      R* A = s_acc + ((o * 2 + 0) * CB + cl) * L::EOS;
-      R* B = s_acc + ((o * 2 + 1) * CB + cl) * L::EOS;
+      R* A = s_acc + (o * P1) * RS + pt;           // [output][row], tested with phi
+      R* Bx = s_acc + ((NOUT + o) * P1) * RS + pt;  // [output][row], tested with d/dxi phi
+      const bool hg = Phys::has_grad(o);
 #pragma unroll
-      for (int iz = 0; iz < P1; ++iz) {
-        A[iz * NQ + qx] = acc_a[o][iz];
-        B[iz * NQ + qx] = acc_b[o][iz];
+      for (int i = 0; i < H; ++i) {
+        A[i * RS] = wx * (aE[o][i] + aO[o][i]);
+        A[(P - i) * RS] = wx * (aE[o][i] - aO[o][i]);
+        if (hg) {
+          Bx[i * RS] = wx * (bE[o][i] + bO[o][i]);
+          Bx[(P - i) * RS] = wx * (bE[o][i] - bO[o][i]);
+        }
       }
+      if (MIDN) {
+        A[(P / 2) * RS] = wx * aM[o];
+        if (hg) Bx[(P / 2) * RS] = wx * bM[o];
+      }
+    }
+  }
+  if constexpr (Phys::FACES) {  // the x-face fluxes contracted along z: line = (face, output)
+    for (int e = mt; e < 2 * NOUT; e += NQ) {
+      R f[NQ], y[P1];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) f[q] = s_fx[e * RS + ct * NQP + q];
+      contract_eo_T<P, R, NQ>(f, y);
+#pragma unroll
+      for (int i = 0; i < P1; ++i) s_acc[L::O_XF + (e * P1 + i) * CB + ct] = y[i];
     }
   }
   __syncthreads();
-  // ---- XT pass: task (output, row iz) -> P1 outputs, plus face terms on face nodes
-  for (int task = m; task < NOUT * P1; task += NQ) {
-    const int o = task / P1, iz = task % P1;
-    const R* A = s_acc + ((o * 2 + 0) * CB + cl) * L::EOS + iz * NQ;
-    const R* B = s_acc + ((o * 2 + 1) * CB + cl) * L::EOS + iz * NQ;
+  // ---- x-transpose pass: line (output, row iz) -> P1 outputs, plus the x-faces' nodes
+  for (int row = mt; row < NOUT * P1; row += NQ) {
+    const int o = row / P1, iz = row % P1;
+    const R* A = s_acc + row * RS + ct * NQP;
+    const R* Bx = A + NOUT * P1 * RS;
+    const bool hg = Phys::has_grad(0);  // (the same for every output of a policy)
     R oE[H > 0 ? H : 1], oO[H > 0 ? H : 1], oM = 0.0;
 #pragma unroll
     for (int i = 0; i < H; ++i) oE[i] = oO[i] = 0.0;
 #pragma unroll
     for (int k = 0; k < QH; ++k) {
-      const R a1 = A[k], a2 = A[NQ - 1 - k], b1 = B[k], b2 = B[NQ - 1 - k];
-      const R As = a1 + a2, Ad = a1 - a2, Bs = b1 + b2, Bd = b1 - b2;
+      const R a1 = A[k], a2 = A[NQ - 1 - k];
+      const R As = a1 + a2, Ad = a1 - a2;
+      R Bs = R(0), Bd = R(0);
+      if (hg) {
+        const R b1 = Bx[k], b2 = Bx[NQ - 1 - k];
+        Bs = b1 + b2;
+        Bd = b1 - b2;
+      }
 #pragma unroll
       for (int i = 0; i < H; ++i) {
         oE[i] = fmaR(tb.Se[k][i], As, oE[i]);
-        oE[i] = fmaR(tb.De[k][i], Bd, oE[i]);
         oO[i] = fmaR(tb.So[k][i], Ad, oO[i]);
-        oO[i] = fmaR(tb.Do[k][i], Bs, oO[i]);
+        if (hg) {
+          oE[i] = fmaR(tb.De[k][i], Bd, oE[i]);
+          oO[i] = fmaR(tb.Do[k][i], Bs, oO[i]);
+        }
       }
-      if (MIDN) { oM = fmaR(tb.Sm[k], As, oM); oM = fmaR(tb.Dm[k], Bd, oM); }
+      if (MIDN) {
+        oM = fmaR(tb.Sm[k], As, oM);
+        if (hg) oM = fmaR(tb.Dm[k], Bd, oM);
+      }
     }
     if constexpr (T::QMID) {  // the middle point: even part of S, odd part of D
-      const R am = A[QH], bm = B[QH];
+      const R am = A[QH], bm = hg ? Bx[QH] : R(0);
 #pragma unroll
       for (int i = 0; i < H; ++i) {
         oE[i] = fmaR(tb.Se[QH][i], am, oE[i]);
-        oO[i] = fmaR(tb.Do[QH][i], bm, oO[i]);
+        if (hg) oO[i] = fmaR(tb.Do[QH][i], bm, oO[i]);
       }
       if (MIDN) oM = fmaR(tb.Sm[QH], am, oM);
     }
@@ -1168,30 +1339,12 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
       out[P - i] = oE[i] - oO[i];
     }
     if (MIDN) out[P / 2] = oM;
-    if (Phys::FACES) {
-      const R* F0 = s_flux + ((0 * NOUT + o) * CB + cl) * NQ;
-      const R* F1 = s_flux + ((1 * NOUT + o) * CB + cl) * NQ;
-      R l = 0.0, r = 0.0;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        const R s = s_S[q * P1 + iz];
-        l = fmaR(s, F0[q], l);
-        r = fmaR(s, F1[q], r);
-      }
-      out[0] += l;
-      out[P] += r;
-      if (!L::FOLD_Z && (iz == 0 || iz == P)) {
-        const R* F = s_flux + (((iz == 0 ? 2 : 3) * NOUT + o) * CB + cl) * NQ;
-#pragma unroll
-        for (int ix = 0; ix < P1; ++ix) {
-          R s = 0.0;
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) s = fmaR(tb.S[q][ix], F[q], s);
-          out[ix] += s;
-        }
-      }
+    if constexpr (Phys::FACES) {
+      out[0] += s_acc[L::O_XF + row * CB + ct];
+      out[P] += s_acc[L::O_XF + (NOUT * P1 + row) * CB + ct];
     }
-    R* dst = s_out + (o * CB + cl) * L::NDP + iz * P1;
+    const int w = s_to[o];
+    R* dst = s_out + (w & 0xfffff) + ct * (w >> 20) + iz * P1;
     if constexpr (L::EPI == 1 || L::EPI == 3) {
       // the epilogue's first change-of-basis pass on the row in registers:
       // u[iz][qx] = sum_ix Vi[ix][qx] out[ix], stored in place of the row
@@ -1208,22 +1361,44 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
       for (int ix = 0; ix < P1; ++ix) dst[ix] = out[ix];
     }
   }
-  __syncthreads();
   if constexpr (L::EPI == 0) {
-    // ---- store (coalesced)
-    sfor<Phys::NOUT_ARR>([&](auto oc) {
-      constexpr int OA = decltype(oc)::value;
-      constexpr int NC = Phys::out_ncomp(OA);
-      constexpr int ob = [] { int b = 0; for (int a = 0; a < OA; ++a) b += Phys::out_ncomp(a); return b; }();
-      R* dst = ptr.out[OA] + (size_t)c0 * NC * ND;
-      for (int e = tid; e < ncb * NC * ND; e += NT) {
-        const int cc = e / (NC * ND), r = e % (NC * ND);
-        const R v = s_out[((ob + r / ND) * CB + cc) * L::NDP + r % ND];
-        if (Phys::ACCUMULATE) dst[e] += v;
-        else dst[e] = v;
+    // ---- store: the shared-memory image of an output equals its global chunk, so one bulk copy
+    //      per array writes it when the chunk starts and ends on 16 bytes
+    bool bst = !Phys::ACCUMULATE && ((size_t)ncb * ND * sizeof(R)) % 16 == 0 && (CB * ND * sizeof(R)) % 16 == 0;
+#pragma unroll
+    for (int a = 0; a < Phys::NOUT_ARR; ++a)
+      bst = bst && (reinterpret_cast<size_t>(ptr.out[a] + (size_t)c0 * Phys::out_ncomp(a) * ND) & 15) == 0;
+    if (bst) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    if (bst) {
+      if (tid == 0) {
+        sfor<Phys::NOUT_ARR>([&](auto oc) {
+          constexpr int OA = decltype(oc)::value;
+          constexpr int NC = Phys::out_ncomp(OA);
+          constexpr int ob = [] { int b = 0; for (int a = 0; a < OA; ++a) b += Phys::out_ncomp(a); return b; }();
+          asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(
+                           ptr.out[OA] + (size_t)c0 * NC * ND),
+                       "r"((unsigned)__cvta_generic_to_shared(s_out + ob * CB * ND)), "r"((unsigned)(ncb * NC * ND * sizeof(R)))
+                       : "memory");
+        });
+        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
       }
-    });
+    } else {
+      sfor<Phys::NOUT_ARR>([&](auto oc) {
+        constexpr int OA = decltype(oc)::value;
+        constexpr int NC = Phys::out_ncomp(OA);
+        constexpr int ob = [] { int b = 0; for (int a = 0; a < OA; ++a) b += Phys::out_ncomp(a); return b; }();
+        R* dst = ptr.out[OA] + (size_t)c0 * NC * ND;
+        for (int e = tid; e < ncb * NC * ND; e += NT) {
+          const R v = s_out[ob * CB * ND + e];
+          if (Phys::ACCUMULATE) dst[e] += v;
+          else dst[e] = v;
+        }
+      });
+    }
   } else {
+    __syncthreads();
     // ---- cell-local epilogue: the inverse weights (copied since kernel start)
     if (epi_bulk) {
       const bool ok = mbar_wait(bar_e, 0);
@@ -1344,7 +1519,7 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
   }
 }
 
-template <int P, class Phys, int CB_ = cells_per_block<P>(), int MINB = min_blocks_per_sm<P>()>
+template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>(), int MINB = Layout<P, Phys, CB_>::CTAS>
 cudaError_t launch_cellop(const MeshDev& mesh,
                           const ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>>& ptr,
                           const typename Phys::Params& prm, int ncell, cudaStream_t stream) {
@@ -1362,7 +1537,7 @@ cudaError_t launch_cellop(const MeshDev& mesh,
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit, std::memory_order_release);
   }
-  if (mesh.cell0 % L::CB != 0 || mesh.cell0 < 0) return cudaErrorInvalidValue;
+  if (mesh.cell0 < 0) return cudaErrorInvalidValue;
   if (ncell <= mesh.cell0) return cudaSuccess;
   const int nblk = (ncell - mesh.cell0 + L::CB - 1) / L::CB;
   if constexpr (!kPDL) {

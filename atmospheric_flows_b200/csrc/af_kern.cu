@@ -53,7 +53,7 @@ namespace {
 constexpr int P = AF_P;
 // cells per CTA of the reduced-quadrature (P+1 points) B kernel: its CTAs have NQ = P+1
 // threads per cell, about half of the full-quadrature kernel's
-constexpr int kReducedCB = P == 4 ? 32 : cells_per_block<P>();
+constexpr int kReducedCB = P == 1 ? 64 : (P == 2 ? 42 : (P <= 4 ? 32 : (P == 5 ? 20 : 18)));
 
 cudaError_t upload_tables() {
   static const Tab<P> t = host::make_tab<P>();
@@ -75,10 +75,10 @@ cudaError_t upload_tables() {
   return e;
 }
 
-template <int STAGE, int MASK>
+template <int STAGE, int MASK, bool GEN>
 cudaError_t rhs_mask(const MeshDev& mesh, const RhsSources& s, const RhsParams& prm, double* o_rho, double* o_u,
                      double* o_p, int ncell, cudaStream_t st) {
-  using Ph = RhsPhys<STAGE, MASK>;
+  using Ph = RhsPhys<STAGE, MASK, GEN>;
   ArgPtrs<PhysInfo<Ph>::NARR_TOTAL, Ph::NOUT_ARR> a{};
   int k = 0;
   for (int j = 0; j < STAGE; ++j) {
@@ -102,25 +102,31 @@ cudaError_t rhs_mask(const MeshDev& mesh, const RhsSources& s, const RhsParams& 
   return launch_cellop<P, Ph>(mesh, a, prm, ncell, st);
 }
 
-template <int STAGE>
+template <int STAGE, bool GEN>
 cudaError_t rhs_stage(const MeshDev& mesh, int mask, const RhsSources& s, const RhsParams& prm, double* o_rho,
                       double* o_u, double* o_p, int ncell, cudaStream_t st) {
   switch (mask) {
-    case 1: return rhs_mask<STAGE, 1>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
-    case 2: return rhs_mask<STAGE, 2>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
-    case 4: return rhs_mask<STAGE, 4>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
-    case 6: return rhs_mask<STAGE, 6>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
-    case 7: return rhs_mask<STAGE, 7>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
+    case 1: return rhs_mask<STAGE, 1, GEN>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
+    case 2: return rhs_mask<STAGE, 2, GEN>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
+    case 4: return rhs_mask<STAGE, 4, GEN>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
+    case 6: return rhs_mask<STAGE, 6, GEN>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
+    case 7: return rhs_mask<STAGE, 7, GEN>(mesh, s, prm, o_rho, o_u, o_p, ncell, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t rhs(const MeshDev& mesh, int stage, int mask, const RhsSources& s, const RhsParams& prm, double* o_rho,
                 double* o_u, double* o_p, int ncell, cudaStream_t st) {
+  const bool gen = prm.radial || prm.sponge;
+  auto run = [&](auto sc) {
+    constexpr int S = decltype(sc)::value;
+    return gen ? rhs_stage<S, true>(mesh, mask, s, prm, o_rho, o_u, o_p, ncell, st)
+               : rhs_stage<S, false>(mesh, mask, s, prm, o_rho, o_u, o_p, ncell, st);
+  };
   switch (stage) {
-    case 1: return rhs_stage<1>(mesh, mask, s, prm, o_rho, o_u, o_p, ncell, st);
-    case 2: return rhs_stage<2>(mesh, mask, s, prm, o_rho, o_u, o_p, ncell, st);
-    case 3: return rhs_stage<3>(mesh, mask, s, prm, o_rho, o_u, o_p, ncell, st);
+    case 1: return run(std::integral_constant<int, 1>{});
+    case 2: return run(std::integral_constant<int, 2>{});
+    case 3: return run(std::integral_constant<int, 3>{});
     default: return cudaErrorInvalidValue;
   }
 }
@@ -700,18 +706,18 @@ __global__ void k_inject(const double* __restrict__ ff, double* __restrict__ fc,
 }
 
 // ------------------------------------------------------------------ adjoint
-constexpr int kAdjCells = P <= 2 ? 16 : 8;
+constexpr int kAdjCells = P <= 2 ? 16 : 10;
 cudaError_t rhs_adjoint1(const MeshDev& mesh, const double* const* in, const double* const* ybar,
                          double* const* xbar, const RhsParams& prm, int ncell, cudaStream_t st) {
   ArgPtrs<8, 5> a{{in[0], in[1], in[2], in[3], in[4], ybar[0], ybar[1], ybar[2]},
                   {xbar[0], xbar[1], xbar[2], xbar[3], xbar[4]}};
-  return launch_cellop<P, RhsAdj1Phys, kAdjCells, 2>(mesh, a, prm, ncell, st);
+  return launch_cellop<P, RhsAdj1Phys, fit_cells<P, RhsAdj1Phys, kAdjCells>()>(mesh, a, prm, ncell, st);
 }
 
 cudaError_t rhs_tangent1(const MeshDev& mesh, const double* const* in, const double* const* din, double* const* dy,
                          const RhsParams& prm, int ncell, cudaStream_t st) {
   ArgPtrs<10, 3> a{{in[0], in[1], in[2], in[3], in[4], din[0], din[1], din[2], din[3], din[4]}, {dy[0], dy[1], dy[2]}};
-  return launch_cellop<P, RhsTlm1Phys, kAdjCells, 2>(mesh, a, prm, ncell, st);
+  return launch_cellop<P, RhsTlm1Phys, fit_cells<P, RhsTlm1Phys, kAdjCells>()>(mesh, a, prm, ncell, st);
 }
 
 // ---- automatic tangents and adjoints of the fused rhs triple of any stage (dual numbers).
@@ -740,7 +746,7 @@ cudaError_t rhs_tangent_s(const MeshDev& mesh, const double* const* in, const do
   a.out[2] = dy[2];
   for (int i = 0; i < k; ++i)
     if (!a.in[i]) return cudaErrorInvalidValue;
-  return launch_cellop<P, Ph, kAdjCells, 2>(mesh, a, prm, ncell, st);
+  return launch_cellop<P, Ph, fit_cells<P, Ph, kAdjCells>()>(mesh, a, prm, ncell, st);
 }
 
 template <int STAGE, int G>
@@ -760,7 +766,7 @@ cudaError_t rhs_adj_group(const MeshDev& mesh, const double* const* in, const do
     a.in[Ph::NBC + 3] = in[1];
     a.out[Ph::NBC] = scratch;
   }
-  return launch_cellop<P, Ph, kAdjCells, 2>(mesh, a, prm, ncell, st);
+  return launch_cellop<P, Ph, fit_cells<P, Ph, kAdjCells>()>(mesh, a, prm, ncell, st);
 }
 
 __global__ void k_add(const double* __restrict__ x, double* __restrict__ y, const long n) {
@@ -961,9 +967,10 @@ cudaError_t cob_cheb(const R* W, const R* r, R alpha, R s, R* d, R* x, int first
 // Launch shapes of the two FP32 smoother kernels at p = 4 (1024x256, us per launch):
 // cells per CTA / CTAs per SM  16/2: B+A^-1 190.6, residual+Chebyshev 258.2;  32/2: 176.4,
 // 237.7;  32/3: 172.5, 240.5;  8/8: 215.1, 314.7;  64/1: 209.1, 372.2.
-constexpr int kFusedCB = P == 4 ? 32 : cells_per_block<P>();
-constexpr int kBInvMinB = P == 4 ? 3 : min_blocks_per_sm<P>();
-constexpr int kResChebMinB = min_blocks_per_sm<P>();
+constexpr int kFusedCB = P == 4 ? 32 : cells_per_block<P, float>();
+constexpr int kFusedMinB = P == 3 || P == 5 ? 3 : 2;
+constexpr int kBInvMinB = P == 4 ? 3 : kFusedMinB;
+constexpr int kResChebMinB = kFusedMinB;
 template <class R>
 cudaError_t b_inv(const MeshDev& mesh, const R* p, R c, const R* WA, R scale, R* w, int ncell, cudaStream_t st) {
   ArgPtrs<1, 1, R> a{{p}, {w}};
@@ -1134,7 +1141,7 @@ const DegreeOps kOps = {upload_tables,     rhs,
                         mass,              op_B,
                         op_C,              inv_diag,
                         mass_factor,       mass_solve,
-                        cells_per_block<P>(), kNPK,
+                        kND % 2 ? 2 : 1, kNPK,
                         mg_res<double>,    mg_res<float>,
                         cheb<double>,
                         prolong<double>,   prolong<float>,

@@ -14,9 +14,10 @@
 //   MassPhys<NC, W>       assemble_cell_term_{rho_update,internal_energy,velocity_fixed}
 //                         (:715-740, :1386-1408, :2330-2357)
 //
-// Conventions of the cell-centric kernel: the calling cell is always the "+" side, n its
-// outward unit normal, and the returned flux is the integrand tested against the cell's
-// own basis functions on that face (already carrying the reference's phi_p sign).
+// Conventions of the cell-centric kernel: the calling cell is always the "+" side, n an
+// outward normal of any length (a flux is linear in it), and the returned flux is the integrand
+// tested against the cell's own basis functions on that face (already carrying the reference's
+// phi_p sign).
 // Integrands are algebraically equal to the reference's (e.g. rho*(p/((g-1) rho)) is
 // formed as p/(g-1)); the oracle keeps the literal forms and parity is checked at 1e-12.
 #pragma once
@@ -30,6 +31,12 @@ struct RhsParams {
   double g1, gg;          // 1/(gamma-1), gamma/(gamma-1)
   double ca[3], ct[3];    // explicit weights a_j and a~_j of the stage's explicit terms
   double cg[3], cgI;      // gravity weights of the explicit terms and of the implicit one
+  // products of the above that the point and face functions read, formed once on the host so that
+  // the kernel takes them from the parameter bank instead of holding them in registers:
+  // a_j dt, a~_j dt / Ma^2, gravity / Fr^2 and Ma^2 / Fr^2, a_j dt Ma^2 / 2, a~_j dt gamma/(gamma-1),
+  // halves of the face weights, a~_j dt / (2 (gamma-1))
+  double r_[3], p_[3], f_[3], e_[3], k_[3], h_[3], fI, eI, hMa2;
+  double r2_[3], p2_[3], k2_[3], h2_[3], j_[3];
   int radial;             // 0: e_z, |g| const; 1: e_r = X/|X|, factor a^2/|X|^2
   // Rayleigh damping of the momentum towards (sp_u, 0) (the 2D hill case's upper sponge and
   // lateral relaxation zones; no counterpart in the reference): rate tau(x, z) of sponge_rate
@@ -96,13 +103,15 @@ __device__ __forceinline__ double amax(double a, double b) { return fmax(a, b); 
 __device__ __forceinline__ Dual aabs(Dual x) { return x.v > 0.0 ? x : (x.v < 0.0 ? -x : Dual{0.0, 0.0}); }
 __device__ __forceinline__ Dual amax(Dual a, Dual b) { return a.v >= b.v ? a : b; }
 
-template <int STAGE, int MASK>
+// GEN: radial gravity or the sponge may be on.  Without them (the hill's vertical gravity) a policy
+// compiled for that alone leaves out their branches, which cost the point loop registers: at degree
+// 4 the fused stage-1 kernel spills with them at three CTAs per SM and does not without.
+template <int STAGE, int MASK, bool GEN = true>
 struct RhsPhys {
   static constexpr bool RHO = (MASK & 1) != 0, VEL = (MASK & 2) != 0, PRES = (MASK & 4) != 0;
   static constexpr bool HAS_I = STAGE < 3 ? (VEL || PRES) : PRES;
   static constexpr int NG = STAGE + (HAS_I ? 1 : 0);
-  static constexpr bool FACES = true, NEED_X = true, ACCUMULATE = false;
-  static constexpr bool FOLD = true;  // z-face folding (Layout::FOLD_Z) measured faster here
+  static constexpr bool FACES = true, NEED_X = GEN, ACCUMULATE = false;
   static constexpr int NOUT_ARR = (RHO ? 1 : 0) + (VEL ? 1 : 0) + (PRES ? 1 : 0);
   static constexpr int NOUT = (RHO ? 1 : 0) + (VEL ? 2 : 0) + (PRES ? 1 : 0);
   static constexpr int O_RHO = 0, O_U = RHO ? 1 : 0, O_P = (RHO ? 1 : 0) + (VEL ? 2 : 0);
@@ -115,6 +124,15 @@ struct RhsPhys {
   }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return true; }
+
+  // With several explicit groups every group is a batch of its own (PhysInfo): the first feeds all
+  // values, the others the gravity terms (and the sponge), the implicit one values only.
+  static constexpr bool val_in(int b, int o) {
+    if (STAGE == 1 || b == 0 || (PRES && o == O_P)) return true;
+    if (RHO && o == O_RHO) return false;
+    return (o == O_U + 1 || GEN) && (b < STAGE || STAGE < 3);
+  }
+  static constexpr bool grad_in(int b, int) { return STAGE == 1 || b < STAGE; }
 
   static constexpr bool quirk_group(int g) { return STAGE == 2 && PRES && g == 1; }
   static constexpr int narr_of(int g) {
@@ -218,17 +236,17 @@ struct RhsPhys {
 
   // The integrand of point_t mapped to the reference cell (see MappedOf in af_cellop.cuh):
   // every flux of the explicit group is a multiple of the velocity u_j plus pressure times the
-  // identity, so its mapped form shares the contravariant velocity (U1, U2) = adj(J) w u_j:
+  // identity, so its mapped form shares the contravariant velocity (U1, U2) = adj(J) u_j:
   //   rho:       ca rho (U1, U2)
   //   rho u_x:   ca rho u_x (U1, U2) + pt (A0, -A2)      rho u_z: ca rho u_z (U1, U2) + pt (-A1, A3)
   //   pressure:  s (U1, U2)
-  // (ca = a_j dt, pt = a~_j dt p_j / Ma^2, s as in point_t); values are multiplied by |J| w.
+  // (ca = a_j dt, pt = a~_j dt p_j / Ma^2, s as in point_t); values are multiplied by |J|.
   static constexpr bool MAPPED = true;
   template <int G>
   __device__ __forceinline__ static void point_mapped(const Params& prm, const double* v, const PointGeo& pg,
                                                       const double (&A)[4], double dw, double* fv, double* fx,
                                                       double* fe) {
-    if (prm.radial) point_mapped_g<G, true>(prm, v, pg, A, dw, fv, fx, fe);
+    if (GEN && prm.radial) point_mapped_g<G, true>(prm, v, pg, A, dw, fv, fx, fe);
     else point_mapped_g<G, false>(prm, v, pg, A, dw, fv, fx, fe);
   }
   template <int G, bool RADIAL>
@@ -239,33 +257,31 @@ struct RhsPhys {
     if constexpr (RADIAL) gravity_dir(prm, pg, e0, e1, fac);
     if constexpr (G < STAGE) {
       const double rho = v[0], ux = v[1], uz = v[2];
-      const double ca = prm.ca[G] * prm.dt, cg = prm.cg[G] * prm.dt;
       const double U1 = A[0] * ux - A[1] * uz, U2 = A[3] * uz - A[2] * ux;
-      const double cr = ca * rho;
+      const double cr = prm.r_[G] * rho;
+      const double rdw = rho * dw;
       if constexpr (RHO) {
-        if (G == 0) fv[O_RHO] += rho * dw;
+        if (G == 0) fv[O_RHO] += rdw;
         fx[O_RHO] += cr * U1;
         fe[O_RHO] += cr * U2;
       }
       if constexpr (VEL || PRES) {
         const double p = v[3];
-        const double ct = prm.ct[G] * prm.dt;
         if constexpr (VEL) {
-          const double rdw = rho * dw;
           if (G == 0) { fv[O_U] += rdw * ux; fv[O_U + 1] += rdw * uz; }
           if constexpr (RADIAL) {
-            const double gfac = cg * prm.invFr2 * rdw * fac;
+            const double gfac = prm.f_[G] * rdw * fac;
             fv[O_U] -= gfac * e0;
             fv[O_U + 1] -= gfac * e1;
           } else {
-            fv[O_U + 1] -= cg * prm.invFr2 * rdw;
+            fv[O_U + 1] -= prm.f_[G] * rdw;
           }
-          if (prm.sponge) {  // -dt a_j tau rho_j (u_j - u_ref)
-            const double ct_ = ca * sponge_rate(prm, pg) * rdw;
+          if (GEN && prm.sponge) {  // -dt a_j tau rho_j (u_j - u_ref)
+            const double ct_ = prm.r_[G] * sponge_rate(prm, pg) * rdw;
             fv[O_U] -= ct_ * (ux - prm.sp_u);
             fv[O_U + 1] -= ct_ * uz;
           }
-          const double pt = ct * prm.invMa2 * p;
+          const double pt = prm.p_[G] * p;
           const double cx = cr * ux, cz = cr * uz;
           fx[O_U] += cx * U1 + pt * A[0];
           fe[O_U] += cx * U2 - pt * A[2];
@@ -274,35 +290,36 @@ struct RhsPhys {
         }
         if constexpr (PRES) {
           const double uu = ux * ux + uz * uz;
-          double val = G == 0 ? p * prm.g1 + 0.5 * prm.Ma2 * rho * uu : 0.0;
-          if constexpr (RADIAL) val -= cg * prm.Ma2Fr2 * rho * (ux * e0 + uz * e1) * fac;
-          else val -= cg * prm.Ma2Fr2 * rho * uz;
-          fv[O_P] += val * dw;
-          const double s = 0.5 * ca * prm.Ma2 * uu * rho + ct * prm.gg * p;
+          // gravity and kinetic part times rho |J| w, the internal energy times |J| w
+          double val = G == 0 ? prm.hMa2 * uu : 0.0;
+          if constexpr (RADIAL) val -= prm.e_[G] * fac * (ux * e0 + uz * e1);
+          else val -= prm.e_[G] * uz;
+          fv[O_P] += val * rdw;
+          if (G == 0) fv[O_P] += prm.g1 * dw * p;
+          const double s = prm.k_[G] * uu * rho + prm.h_[G] * p;
           fx[O_P] += s * U1;
           fe[O_P] += s * U2;
         }
       }
     } else {
-      const double rc = v[0];
-      const double cgI = prm.cgI * prm.dt;
+      const double rdw = v[0] * dw;
       if constexpr (VEL && STAGE < 3) {
         if constexpr (RADIAL) {
-          const double gfac = cgI * prm.invFr2 * rc * fac * dw;
+          const double gfac = prm.fI * rdw * fac;
           fv[O_U] -= gfac * e0;
           fv[O_U + 1] -= gfac * e1;
         } else {
-          fv[O_U + 1] -= cgI * prm.invFr2 * rc * dw;
+          fv[O_U + 1] -= prm.fI * rdw;
         }
       }
       if constexpr (PRES) {
         const double fxv = v[1], fzv = v[2];
-        double val = 0.5 * rc * prm.Ma2 * (fxv * fxv + fzv * fzv);
+        double val = prm.hMa2 * (fxv * fxv + fzv * fzv);
         if (STAGE < 3) {
-          if constexpr (RADIAL) val += cgI * prm.Ma2Fr2 * rc * (fxv * e0 + fzv * e1) * fac;
-          else val += cgI * prm.Ma2Fr2 * rc * fzv;
+          if constexpr (RADIAL) val += prm.eI * fac * (fxv * e0 + fzv * e1);
+          else val += prm.eI * fzv;
         }
-        fv[O_P] -= val * dw;
+        fv[O_P] -= val * rdw;
       }
     }
   }
@@ -315,38 +332,30 @@ struct RhsPhys {
       const T rm = vm[0], umx = vm[1], umz = vm[2];
       const T unp = upx * n[0] + upz * n[1], unm = umx * n[0] + umz * n[1];
       const T lam = amax(aabs(unp), aabs(unm));
-      const double ca = prm.ca[G] * prm.dt;
-      if constexpr (RHO) {  // :519-526
-        const T F = ca * (0.5 * (rp * unp + rm * unm) + 0.5 * lam * (rp - rm));
-        flux[O_RHO] = -F;
-      }
+      // the mass fluxes and the dissipation of both sides: rho u.n +- lambda rho share one product
+      const T mp = rp * (unp + lam), mm = rm * (unm - lam);
+      if constexpr (RHO) flux[O_RHO] = -prm.r2_[G] * (mp + mm);  // :519-526
       if constexpr (VEL || PRES) {
         const T pp = vp[3], pm = vm[3];
-        const double ct = prm.ct[G] * prm.dt;
         if constexpr (VEL) {  // :1938-1950
-          const T pa = ct * prm.invMa2 * 0.5 * (pp + pm);
-          const T Fx = ca * 0.5 * (rp * upx * unp + rm * umx * unm) + pa * n[0] + ca * 0.5 * lam * (rp * upx - rm * umx);
-          const T Fz = ca * 0.5 * (rp * upz * unp + rm * umz * unm) + pa * n[1] + ca * 0.5 * lam * (rp * upz - rm * umz);
-          flux[O_U] = -Fx;
-          flux[O_U + 1] = -Fz;
+          const T pa = prm.p2_[G] * (pp + pm);
+          flux[O_U] = -(prm.r2_[G] * (mp * upx + mm * umx) + pa * n[0]);
+          flux[O_U + 1] = -(prm.r2_[G] * (mp * upz + mm * umz) + pa * n[1]);
         }
         if constexpr (PRES) {  // :1057-1079 (stage 1), :1141-1194 (2), :1275-1355 (3)
           const T uup = upx * upx + upz * upz, uum = umx * umx + umz * umz;
-          const T kin = 0.5 * (0.5 * uup * rp * unp + 0.5 * uum * rm * unm);
-          const T ent = 0.5 * prm.gg * (pp * unp + pm * unm);
           T F;
           if constexpr (STAGE < 3) {
-            T jk;
-            if constexpr (quirk_group(G)) {  // :1182-1183 uses u_tmp_2 . u_old
-              jk = rp * 0.5 * (upx * vp[4] + upz * vp[5]) - rm * 0.5 * (umx * vm[4] + umz * vm[5]);
+            T K;  // kinetic flux and dissipation
+            if constexpr (quirk_group(G)) {  // :1182-1183 uses u_tmp_2 . u_old in the jump
+              const T qp = upx * vp[4] + upz * vp[5], qm = umx * vm[4] + umz * vm[5];
+              K = rp * (unp * uup + lam * qp) + rm * (unm * uum - lam * qm);
             } else {
-              jk = rp * 0.5 * uup - rm * 0.5 * uum;
+              K = mp * uup + mm * uum;
             }
-            const T je = prm.g1 * (pp - pm);
-            F = ca * prm.Ma2 * (kin + 0.5 * lam * jk) + ct * (ent + 0.5 * lam * je);
+            F = prm.k2_[G] * K + prm.h2_[G] * (pp * unp + pm * unm) + prm.j_[G] * lam * (pp - pm);
           } else {
-            const T jE = prm.g1 * (pp - pm) + 0.5 * prm.Ma2 * (rp * uup - rm * uum);
-            F = ca * prm.Ma2 * kin + ca * ent + ca * 0.5 * lam * jE;
+            F = prm.k2_[G] * (mp * uup + mm * uum) + prm.h2_[G] * (pp * unp + pm * unm) + prm.j_[G] * lam * (pp - pm);
           }
           flux[O_P] = -F;
         }
@@ -358,7 +367,7 @@ struct RhsPhys {
   __device__ __forceinline__ static void boundary_t(const Params& prm, const T* vp, const double* n, T* flux) {
     if constexpr (G < STAGE && VEL) {  // :2189-2305, p_D = p
       const T pp = vp[3];
-      const T s = prm.ct[G] * prm.dt * prm.invMa2 * (0.5 * (pp + pp));
+      const T s = prm.p2_[G] * (pp + pp);
       flux[O_U] = -s * n[0];
       flux[O_U + 1] = -s * n[1];
     }

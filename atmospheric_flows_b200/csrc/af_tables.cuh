@@ -33,6 +33,10 @@ struct TabT {
   R Se[QE][H > 0 ? H : 1], So[QE][H > 0 ? H : 1];
   R De[QE][H > 0 ? H : 1], Do[QE][H > 0 ? H : 1];
   R Sm[QE], Dm[QE];
+  // the even/odd tables times the quadrature weight of their point (test-function contractions)
+  R SeW[QE][H > 0 ? H : 1], SoW[QE][H > 0 ? H : 1];
+  R DeW[QE][H > 0 ? H : 1], DoW[QE][H > 0 ? H : 1];
+  R SmW[QE], DmW[QE];
   R w[NQ], x[NQ];
 };
 template <int P>
@@ -168,9 +172,15 @@ inline TabT<P, R, NQ> make_tab() {
       t.So[q][i] = (R)((S[q][i] - S[q][P - i]) / 2);
       t.De[q][i] = (R)((D[q][i] + D[q][P - i]) / 2);
       t.Do[q][i] = (R)((D[q][i] - D[q][P - i]) / 2);
+      t.SeW[q][i] = (R)(w[q] * (S[q][i] + S[q][P - i]) / 2);
+      t.SoW[q][i] = (R)(w[q] * (S[q][i] - S[q][P - i]) / 2);
+      t.DeW[q][i] = (R)(w[q] * (D[q][i] + D[q][P - i]) / 2);
+      t.DoW[q][i] = (R)(w[q] * (D[q][i] - D[q][P - i]) / 2);
     }
     t.Sm[q] = T::MIDN ? (R)S[q][P / 2] : R(0);
     t.Dm[q] = T::MIDN ? (R)D[q][P / 2] : R(0);
+    t.SmW[q] = T::MIDN ? (R)(w[q] * S[q][P / 2]) : R(0);
+    t.DmW[q] = T::MIDN ? (R)(w[q] * D[q][P / 2]) : R(0);
   }
   for (int q = 0; q < T::NQ; ++q) {
     t.w[q] = (R)w[q];
