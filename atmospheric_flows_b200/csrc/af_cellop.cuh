@@ -130,22 +130,6 @@ struct EpiOf<Phys, std::void_t<decltype(Phys::EPI)>> {
   static constexpr int value = Phys::EPI;
 };
 
-// Cell indices kept in the real-typed geometry block, stored bit for bit (a float holds
-// integers exactly only up to 2^24, fewer than the cells of a large mesh).
-__device__ __forceinline__ void put_index(float& s, int v) { s = __int_as_float(v); }
-__device__ __forceinline__ void put_index(double& s, int v) { s = __longlong_as_double((long long)v); }
-__device__ __forceinline__ int get_index(float s) { return __float_as_int(s); }
-__device__ __forceinline__ int get_index(double s) { return (int)__double_as_longlong(s); }
-
-// Face neighbours of cell c (faces 0: xi=0, 1: xi=1, 2: eta=0, 3: eta=1); -1 on a wall.
-__device__ __forceinline__ void cell_neighbours(const MeshDev& mesh, int c, int nb[4]) {
-  const int i = c % mesh.nx, j = c / mesh.nx;
-  nb[0] = i > 0 ? c - 1 : (mesh.periodic_x ? c + mesh.nx - 1 : -1);
-  nb[1] = i < mesh.nx - 1 ? c + 1 : (mesh.periodic_x ? c - mesh.nx + 1 : -1);
-  nb[2] = j > 0 ? c - mesh.nx : -1;
-  nb[3] = j < mesh.nz - 1 ? c + mesh.nx : -1;
-}
-
 template <int N, class F, int... I>
 __device__ __forceinline__ void sfor_impl(F& f, std::integer_sequence<int, I...>) {
   (f(std::integral_constant<int, I>{}), ...);

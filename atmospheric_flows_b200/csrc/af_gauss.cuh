@@ -18,579 +18,535 @@
 // Per cell, the operators need the values of their inputs at the volume points (the
 // coefficients themselves: no contraction) and their traces on the faces; test functions
 // enter through Dg[q][i] = L_i'(g_q) (volume gradients) and L_i(0), L_i(1) (faces).  A face
-// trace is an extrapolation along the normal line: u(0, g_q) = sum_i L_i(0) u_g[q][i].  Each
-// kernel writes the face traces of its output, which the next kernel reads for its own and
-// its neighbours' faces (the neighbour's trace on the shared face: 4 (P+1) values per cell
-// and field, as many as the nodal kernels gather).
-//   trace layout: tr[((f * NC + comp) * ncell + cell) * (P+1) + point], faces 0 (xi = 0),
-//   1 (xi = 1), 2 (eta = 0), 3 (eta = 1); the point runs along the face (eta for faces 0, 1,
-//   xi for faces 2, 3), so a face and the neighbour's opposite face share point indices.
-// CTA: GS_CB cells x (P+1) threads; thread (cell, m) owns the column m (x index) of its cell in
-// the volume pass and the row m in the passes along x.
+// trace is an extrapolation along the normal line: u(0, g_q) = sum_i L_i(0) u_g[q][i].
+//
+// Layout: every array of the recurrence is tiled by 32 consecutive cells, the cell fastest:
+//   field  v[(tile * ND + node) * 32 + lane],  node = qz (P+1) + qx
+//   faces  t[((tile * 4 + face) * (P+1) + point) * 32 + lane]
+// faces 0 (xi = 0), 1 (xi = 1), 2 (eta = 0), 3 (eta = 1); the point runs along the face, so a face
+// and the neighbour's opposite face share point indices.  A CTA is one tile, lane = cell, warp m =
+// column qx = m of the cells: every load and store of a warp is one aligned line of 32 cells, there
+// is no index arithmetic per element, the column's work stays in registers, the tables are indexed
+// by warp-uniform values, and only the contraction along x passes through shared memory (cell
+// fastest: no bank conflicts).  The edge vectors of a face serve as its normal (the fluxes are
+// linear in it), so a cell's geometry is six floats, formed once per mesh.
+//
+// The kernels pass between them what the next one needs and no more: k_gs_binv does not write w but
+// the two mapped fluxes of C0 at the points (p_f w contracted with adj(J)) and one value per face
+// point, p_f (w . n), so k_gs_zstep reads neither p_f nor the traces of w: its face flux is the own
+// value minus the neighbour's.  x takes two directions every second step.
+//
+// The kernels of the chain overlap by programmatic dependent launch and read what the kernel before
+// wrote, so none of their arrays is declared const __restrict__: such loads count as invariant over
+// the kernel and the compiler may move them above griddepcontrol.wait (small meshes then read the
+// previous step's values).
+//
+// Measured at 512x256, p = 4 (131072 cells), us per launch in a chain, before (cell-major arrays,
+// element-wise copies through shared memory: 21.7 M and 26.6 M warp instructions) and now:
+//   k_gs_binv 32.9 -> 23.5, k_gs_zstep 46.9 -> 20.5 (the mixed IMEX step 70.2 -> 45.5 ms)
+// The step moves about 250 MB through L2 (164 MB of it DRAM) at 1024x256 in 37 us, 6.8 TB/s: it is
+// bound by memory; k_gs_binv (200 MB, 41 us) by issue (0.66 of the cycles) and latency.
 #pragma once
 
 #include "af_cellop.cuh"
 
 namespace af {
 
-template <int P>
-constexpr int gs_cells() { return P <= 4 ? 32 : 16; }
+constexpr int kGsTile = 32;  // cells per tile (one warp of lanes)
+constexpr int kGsGeo = 6;    // floats per cell: A, C, B of the bilinear map x = v0 + A xi + C eta + B xi eta
 
-// per cell: bilinear map A, B, C (6), four faces (normal x, z, length) (12), neighbours (4);
-// an odd stride against bank conflicts
-constexpr int kGsGeo = 23;
+// n / d for 0 <= n < 2^31 by one multiplication (Granlund and Montgomery, "Division by invariant
+// integers using multiplication", 1994): m = floor(2^(31+l) / d) + 1, l = ceil(log2 d)
+struct FastDiv {
+  unsigned m;
+  int l, d;
+  static FastDiv make(int d) {
+    int l = 0;
+    while ((1LL << l) < d) ++l;
+    return {(unsigned)((1ULL << (31 + l)) / (unsigned)d + 1), l, d};
+  }
+  __device__ __forceinline__ int div(int n) const { return (int)(__umulhi((unsigned)n << 1, m) >> l); }
+};
+
+struct GsMesh {
+  const float* geo;  // [tile][kGsGeo][32]
+  FastDiv nx;
+  int nz, periodic_x, ncell;
+};
 
 template <int P>
 struct GsShape {
-  static constexpr int P1 = P + 1, ND = P1 * P1, CB = gs_cells<P>(), NT = CB * P1;
-  static constexpr int NDS = ND | 1;  // per-cell stride of nodal arrays in shared memory
-  static constexpr int P1S = P1 | 1;  // per-cell stride of face arrays
+  static constexpr int P1 = P + 1, ND = P1 * P1, NT = kGsTile * P1;
+  // CTAs per SM asked of the compiler.  Degree 4, (k_gs_binv, k_gs_zstep), the mixed IMEX step at
+  // 512x256: (4, 6) 46.3 ms, (5, 6) 45.4, (5, 7) 45.2, (6, 6) 46.8 (k_gs_binv spills at 64 registers).
+  static constexpr int CTAS_B = 800 / NT, CTAS_Z = (P <= 4 ? 1120 : 900) / NT;
+  // the thread's element of node or point 0 .. and the strides between its nodes (column m) and faces
+  __device__ __forceinline__ static size_t column(int tile, int m, int lane) {
+    return (size_t)tile * (ND * kGsTile) + (m * kGsTile + lane);
+  }
+  static constexpr int SN = P1 * kGsTile, SF = P1 * kGsTile;
+  __device__ __forceinline__ static size_t point(int tile, int m, int lane) {
+    return (size_t)tile * (4 * P1 * kGsTile) + (m * kGsTile + lane);
+  }
 };
 
-// the cell map, face normals and lengths and the neighbours of cell c, spread over the
-// cell's threads: task 4 the map and neighbours, task f < 4 face f (as the cell kernel)
+// what a thread knows of its cell and column
 template <int P>
-__device__ __forceinline__ void gs_geometry(const MeshDev& mesh, int c, int m, float* g) {
-  constexpr int P1 = P + 1;
-  const int i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
-  for (int task = m; task < 5; task += P1) {
-    if (task == 4) {
-      const double2 v0 = mesh.vtx[j * W + i], v1 = mesh.vtx[j * W + i + 1];
-      const double2 v2 = mesh.vtx[(j + 1) * W + i], v3 = mesh.vtx[(j + 1) * W + i + 1];
-      g[0] = (float)(v1.x - v0.x);
-      g[1] = (float)(v1.y - v0.y);
-      g[2] = (float)(v3.x - v2.x - v1.x + v0.x);
-      g[3] = (float)(v3.y - v2.y - v1.y + v0.y);
-      g[4] = (float)(v2.x - v0.x);
-      g[5] = (float)(v2.y - v0.y);
-      int nb[4];
-      cell_neighbours(mesh, c, nb);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) put_index(g[18 + f], nb[f]);
-    } else {
-      const int f = task;
-      const int ia = (f == 1) ? i + 1 : i, ja = (f == 3) ? j + 1 : j;
-      const int ib = (f == 0) ? i : i + 1, jb = (f == 2) ? j : j + 1;
-      const double2 a = mesh.vtx[ja * W + ia], b = mesh.vtx[jb * W + ib];
-      const double tx = b.x - a.x, tz = b.y - a.y, len = sqrt(tx * tx + tz * tz);
-      const double il = ((f == 0 || f == 3) ? 1.0 : -1.0) / len;
-      g[6 + 3 * f] = (float)(-tz * il);
-      g[7 + 3 * f] = (float)(tx * il);
-      g[8 + 3 * f] = (float)len;
-    }
-  }
-}
-
-// own and neighbour traces of NC components of a field into s_own / s_nb
-// [face][comp][cell][point] (point stride P1S), by asynchronous element copies (the caller
-// waits for them before its barrier); a boundary face takes the own trace as the
-// neighbour's (B's wall flux uses it so; C0 has no wall flux).  Thread t copies point
-// t % (P+1) of cell t / (P+1) for every face and component: consecutive threads read
-// consecutive elements.  The neighbours come from the CTA's geometry block (complete).
-template <int P, int NC>
-__device__ __forceinline__ void gs_load_traces(const float* __restrict__ tr, const float* s_geo, int c0, int ncb,
-                                               int ncell, float* s_own, float* s_nb) {
-  using S = GsShape<P>;
-  const int cc = threadIdx.x / S::P1, p = threadIdx.x % S::P1;
-  if (cc >= ncb) return;
-  const int c = c0 + cc;
+struct GsThread {
+  int lane, m, tile, c;
+  bool live;
+  float Ax, Az, Cx, Cz, Bx, Bz;
   int nb[4];
-#pragma unroll
-  for (int f = 0; f < 4; ++f) nb[f] = get_index(s_geo[cc * kGsGeo + 18 + f]);
-#pragma unroll
-  for (int fc = 0; fc < 4 * NC; ++fc) {
-    const int f = fc / NC, comp = fc % NC;
-    const int o = (fc * S::CB + cc) * S::P1S + p;
-    const float* own = tr + ((size_t)(f * NC + comp) * ncell + c) * S::P1 + p;
-    const float* oth = nb[f] >= 0 ? tr + ((size_t)((f ^ 1) * NC + comp) * ncell + nb[f]) * S::P1 + p : own;
-    cp_async_el(&s_own[o], own);
-    cp_async_el(&s_nb[o], oth);
+  __device__ __forceinline__ explicit GsThread(const GsMesh& g) {
+    lane = threadIdx.x & 31;
+    m = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // warp-uniform
+    tile = blockIdx.x;
+    c = tile * kGsTile + lane;
+    live = c < g.ncell;
   }
+  __device__ __forceinline__ void geometry(const GsMesh& g) {
+    const float* s = g.geo + (size_t)tile * kGsGeo * kGsTile + lane;
+    Ax = s[0]; Az = s[kGsTile]; Cx = s[2 * kGsTile]; Cz = s[3 * kGsTile]; Bx = s[4 * kGsTile]; Bz = s[5 * kGsTile];
+  }
+  __device__ __forceinline__ void neighbours(const GsMesh& g) {  // -1: wall (and past the last cell)
+    const int nx = g.nx.d, j = g.nx.div(c), i = c - j * nx;
+    nb[0] = i > 0 ? c - 1 : (g.periodic_x ? c + nx - 1 : -1);
+    nb[1] = i < nx - 1 ? c + 1 : (g.periodic_x ? c - nx + 1 : -1);
+    nb[2] = j > 0 ? c - nx : -1;
+    nb[3] = j < g.nz - 1 ? c + nx : -1;
+#pragma unroll
+    for (int f = 0; f < 4; ++f) nb[f] = live ? nb[f] : -1;
+  }
+  __device__ __forceinline__ float J01(float xi) const { return fmaf(Bx, xi, Cx); }
+  __device__ __forceinline__ float J11(float xi) const { return fmaf(Bz, xi, Cz); }
+  __device__ __forceinline__ float J00(float eta) const { return fmaf(Bx, eta, Ax); }
+  __device__ __forceinline__ float J10(float eta) const { return fmaf(Bz, eta, Az); }
+  // outward normal times length of face f: (-tz, tx) of the edge on faces 0 and 3, (tz, -tx) on 1, 2
+  __device__ __forceinline__ void normal(int f, float& n0, float& n1) const {
+    const float tx = f == 0 ? Cx : (f == 1 ? Cx + Bx : (f == 2 ? Ax : Ax + Bx));
+    const float tz = f == 0 ? Cz : (f == 1 ? Cz + Bz : (f == 2 ? Az : Az + Bz));
+    const float s = (f == 0 || f == 3) ? 1.f : -1.f;
+    n0 = -s * tz;
+    n1 = s * tx;
+  }
+};
+
+// neighbour's value of a face array at this thread's point (own: what a wall takes)
+template <int P>
+__device__ __forceinline__ float gs_other(const float* t, const GsThread<P>& th, int f, float own) {
+  const int nb = th.nb[f];
+  return nb >= 0 ? t[GsShape<P>::point(nb >> 5, th.m, nb & 31) + (f ^ 1) * GsShape<P>::SF] : own;
 }
 
-// the face traces of NC components of a cell field staged in shared memory (cell stride NDS,
-// component stride CB NDS) into s_t [face][comp][cell][point]: thread (cell, m) extrapolates
-// along row m (faces 0, 1) and column m (faces 2, 3)
-template <int P, int NC>
-__device__ __forceinline__ void gs_traces(const float* s_val, int cl, int m, float* s_t) {
-  using S = GsShape<P>;
+// the traces on faces 2 and 3 of a column, at its point
+template <int P>
+__device__ __forceinline__ void gs_ends(const float* col, float& lo, float& hi) {
   const CobT<P, float>& cb = cobr<P, float>();
+  lo = cb.lo[0] * col[0];
+  hi = cb.hi[0] * col[0];
 #pragma unroll
-  for (int comp = 0; comp < NC; ++comp) {
-    const float* cell = s_val + (comp * S::CB + cl) * S::NDS;
-    float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
-#pragma unroll
-    for (int i = 0; i < S::P1; ++i) {
-      t0 = fmaf(cb.lo[i], cell[m * S::P1 + i], t0);
-      t1 = fmaf(cb.hi[i], cell[m * S::P1 + i], t1);
-      t2 = fmaf(cb.lo[i], cell[i * S::P1 + m], t2);
-      t3 = fmaf(cb.hi[i], cell[i * S::P1 + m], t3);
-    }
-    s_t[((0 * NC + comp) * S::CB + cl) * S::P1S + m] = t0;
-    s_t[((1 * NC + comp) * S::CB + cl) * S::P1S + m] = t1;
-    s_t[((2 * NC + comp) * S::CB + cl) * S::P1S + m] = t2;
-    s_t[((3 * NC + comp) * S::CB + cl) * S::P1S + m] = t3;
+  for (int i = 1; i <= P; ++i) {
+    lo = fmaf(cb.lo[i], col[i], lo);
+    hi = fmaf(cb.hi[i], col[i], hi);
   }
 }
-
-// s_t [face][comp][cell][point] to the trace array, consecutive threads on consecutive elements
-template <int P, int NC>
-__device__ __forceinline__ void gs_store_traces(const float* s_t, int c0, int ncb, int ncell, float* __restrict__ tr) {
-  using S = GsShape<P>;
-  const int cc = threadIdx.x / S::P1, p = threadIdx.x % S::P1;
-  if (cc >= ncb) return;
+// the traces on faces 0 and 1 at point m from the rows of a field in shared memory [node][lane]
+template <int P>
+__device__ __forceinline__ void gs_row_ends(const float* s, int m, int lane, float& lo, float& hi) {
+  float row[P + 1];
 #pragma unroll
-  for (int fc = 0; fc < 4 * NC; ++fc)
-    tr[((size_t)fc * ncell + c0) * S::P1 + threadIdx.x] = s_t[(fc * S::CB + cc) * S::P1S + p];
+  for (int i = 0; i <= P; ++i) row[i] = s[(m * (P + 1) + i) * kGsTile + lane];
+  gs_ends<P>(row, lo, hi);
 }
 
-// ---------------------------------------------------------------- w = A^{-1} B d
-// d_g, its traces dtr -> w_g = scale diag(WA) B_g d_g (two components) and its traces wtr.
+// the geometry block of a mesh
+static __global__ void k_gs_geo(const MeshDev mesh, float* __restrict__ geo, const int ncell) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (ncell + kGsTile - 1) / kGsTile * kGsTile) return;
+  const int c = min(e, ncell - 1), i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
+  const double2* v = mesh.vtx + (size_t)j * W + i;
+  const double2 v0 = v[0], v1 = v[1], v2 = v[W], v3 = v[W + 1];
+  float* g = geo + (size_t)(e / kGsTile) * kGsGeo * kGsTile + e % kGsTile;
+  g[0] = (float)(v1.x - v0.x);
+  g[kGsTile] = (float)(v1.y - v0.y);
+  g[2 * kGsTile] = (float)(v2.x - v0.x);
+  g[3 * kGsTile] = (float)(v2.y - v0.y);
+  g[4 * kGsTile] = (float)(v3.x - v2.x - v1.x + v0.x);
+  g[5 * kGsTile] = (float)(v3.y - v2.y - v1.y + v0.y);
+}
+
+// ------------------------------------------- w = A^{-1} B d, handed on as the fluxes of C0 w
+// d_g and its traces dtr -> w_g = diag(WA) B_g d_g, then at the points the mapped fluxes of C0,
+//   (fx, fe) = -cdt gg p_f w_q (J11 w0 - J01 w1, J00 w1 - J10 w0),
+// and at the face points gf = cdt gg/2 p_f (w . n) w_q with the cell's outward normal.
 // B with coefficient cB (euler_operator.h:1536, 1574-1577, 1611-1613): volume
 // -cB d div(phi), face cB {{d}} phi . n, wall cB d+ phi . n.
-template <int P>
-__global__ void __launch_bounds__(GsShape<P>::NT)
-    k_gs_binv(const MeshDev mesh, const float* __restrict__ d, const float* __restrict__ dtr, const float cB,
-              const float* __restrict__ WA, const float scale, float* __restrict__ w, float* __restrict__ wtr,
-              const int ncell) {
-  using S = GsShape<P>;
-  constexpr int P1 = S::P1, ND = S::ND, CB = S::CB, NT = S::NT, NDS = S::NDS, P1S = S::P1S;
-  __shared__ float s_geo[CB * kGsGeo];
-  __shared__ float s_d[CB * NDS];
-  __shared__ float s_wa[CB * NDS];
-  __shared__ float s_tpm[2 * 4 * CB * P1S];  // own and neighbour traces of d
-  __shared__ float s_fx[2 * CB * NDS];
-  __shared__ float s_xf[2 * 2 * CB * P1S];  // x-face fluxes [face 0, 1][comp][cell][point]
-  __shared__ float s_out[2 * CB * NDS];
-  float* const s_tp = s_tpm;
-  float* const s_tm = s_tpm + 4 * CB * P1S;
-  // the traces of w take the place of d's traces, which the face terms read before the
-  // barrier that ends the volume and face phase: 30 KB instead of 35 KB per CTA, 7 CTAs per SM
-  float* const s_wt = s_tpm;
-  pdl_allow_next();
-  const CobT<P, float>& cb = cobr<P, float>();
-  const int tid = threadIdx.x, cl = tid % CB, m = tid / CB;
-  const int c0 = blockIdx.x * CB, ncb = min(CB, ncell - c0);
-  const bool live = cl < ncb;
-  const int c = c0 + (live ? cl : ncb - 1);
-  float* g = s_geo + cl * kGsGeo;
-  gs_geometry<P>(mesh, c, m, g);
-  pdl_wait_previous();
-  for (int e = tid; e < ncb * ND; e += NT) {
-    const int o = (e / ND) * NDS + e % ND;
-    cp_async_el(&s_d[o], d + (size_t)c0 * ND + e);
-    cp_async_el(&s_wa[o], WA + (size_t)c0 * ND + e);
-  }
-  __syncthreads();  // the geometry block (neighbours) complete
-  gs_load_traces<P, 1>(dtr, s_geo, c0, ncb, ncell, s_tp, s_tm);
-  cp_async_wait_all();
-  __syncthreads();
-  float acc[2][P1];
-#pragma unroll
-  for (int o = 0; o < 2; ++o)
-#pragma unroll
-    for (int i = 0; i < P1; ++i) acc[o][i] = 0.f;
-  if (live) {
-    // volume points of column qx = m: x-fluxes to shared memory, the z-derivative test in registers
-    const int qx = m;
-    const float xi = cb.g[qx], wx = cb.w[qx];
-    const float J01 = fmaf(g[2], xi, g[4]), J11 = fmaf(g[3], xi, g[5]);
-#pragma unroll
-    for (int qz = 0; qz < P1; ++qz) {
-      const float eta = cb.g[qz];
-      const float J00 = fmaf(g[2], eta, g[0]), J10 = fmaf(g[3], eta, g[1]);
-      const float sw = -cB * s_d[cl * NDS + qz * P1 + qx] * (wx * cb.w[qz]);
-      s_fx[(0 * CB + cl) * NDS + qz * P1 + qx] = J11 * sw;
-      s_fx[(1 * CB + cl) * NDS + qz * P1 + qx] = -J01 * sw;
-      const float fe0 = -J10 * sw, fe1 = J00 * sw;
-#pragma unroll
-      for (int iz = 0; iz < P1; ++iz) {
-        acc[0][iz] = fmaf(cb.Dg[qz][iz], fe0, acc[0][iz]);
-        acc[1][iz] = fmaf(cb.Dg[qz][iz], fe1, acc[1][iz]);
-      }
-    }
-    // z-faces at point qx (test L_iz(0) or L_iz(1) on the column), x-faces at point m
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const int p = m;
-      const float tp = s_tp[(f * CB + cl) * P1S + p], tm = s_tm[(f * CB + cl) * P1S + p];
-      const float a = cB * 0.5f * (tp + tm) * (g[8 + 3 * f] * cb.w[p]);
-      const float F0 = a * g[6 + 3 * f], F1 = a * g[7 + 3 * f];
-      if (f >= 2) {
-#pragma unroll
-        for (int iz = 0; iz < P1; ++iz) {
-          const float e = f == 2 ? cb.lo[iz] : cb.hi[iz];
-          acc[0][iz] = fmaf(e, F0, acc[0][iz]);
-          acc[1][iz] = fmaf(e, F1, acc[1][iz]);
-        }
-      } else {
-        s_xf[((f * 2 + 0) * CB + cl) * P1S + p] = F0;
-        s_xf[((f * 2 + 1) * CB + cl) * P1S + p] = F1;
-      }
-    }
-  }
-  __syncthreads();
-  if (live) {
-    // node (ix = m, iz): the x-derivative test along row iz, the x-face terms, A^{-1}
-    const int ix = m;
-#pragma unroll
-    for (int iz = 0; iz < P1; ++iz) {
-#pragma unroll
-      for (int o = 0; o < 2; ++o) {
-        float v = acc[o][iz];
-        const float* fx = s_fx + (o * CB + cl) * NDS + iz * P1;
-#pragma unroll
-        for (int qx = 0; qx < P1; ++qx) v = fmaf(cb.Dg[qx][ix], fx[qx], v);
-        v = fmaf(cb.lo[ix], s_xf[((0 * 2 + o) * CB + cl) * P1S + iz], v);
-        v = fmaf(cb.hi[ix], s_xf[((1 * 2 + o) * CB + cl) * P1S + iz], v);
-        s_out[(o * CB + cl) * NDS + iz * P1 + ix] = scale * s_wa[cl * NDS + iz * P1 + ix] * v;
-      }
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < ncb * 2 * ND; e += NT) {  // [cell][comp][node], coalesced
-    const int cc = e / (2 * ND), o = (e / ND) % 2, k = e % ND;
-    w[(size_t)c0 * 2 * ND + e] = s_out[(o * CB + cc) * NDS + k];
-  }
-  if (live) gs_traces<P, 2>(s_out, cl, m, s_wt);
-  __syncthreads();
-  gs_store_traces<P, 2>(s_wt, c0, ncb, ncell, wtr);
-}
-
-// ------------------------------------------------- the Chebyshev step on z = D^{-1} r
-// w_g (two components) and p_fixed (pg) with their traces -> y = C0_g w_g, then per node
-//   z' = z + g WM y - d,  d' = alpha d + s z',  x = d' (first) or x += d',
-// d' in place of d (each CTA reads only its own cells of d), and the traces of d'.
 // C0 (euler_operator.h:1444, 1494-1502 without the wave-speed term): volume
 // -cdt gg p_f w . grad(q), face cdt gg/2 (p_f+ w+ . n + p_f- w- . n) q, no wall term.
 template <int P>
-__global__ void __launch_bounds__(GsShape<P>::NT)
-    k_gs_zstep(const MeshDev mesh, const float* __restrict__ w, const float* __restrict__ wtr,
-               const float* __restrict__ pg, const float* __restrict__ ptr, const float cdt, const float gg,
-               const float* __restrict__ WM, const float gfac, const float alpha, const float s,
-               float* __restrict__ z, float* __restrict__ d, float* __restrict__ x, const int first,
-               float* __restrict__ dtr, const int ncell) {
+__global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_B)
+    k_gs_binv(const GsMesh mesh, const float* d, const float* dtr, const float cB,
+              const float* WA, const float* pg, const float* ptr,
+              const float cgg, float* fx, float* fe, float* gf) {
   using S = GsShape<P>;
-  constexpr int P1 = S::P1, ND = S::ND, CB = S::CB, NT = S::NT, NDS = S::NDS, P1S = S::P1S;
-  __shared__ float s_geo[CB * kGsGeo];
-  __shared__ float s_w[2 * CB * NDS];
-  __shared__ float s_p[CB * NDS];
-  __shared__ float s_twp[4 * 2 * CB * P1S], s_twm[4 * 2 * CB * P1S];
-  __shared__ float s_tpp[4 * CB * P1S], s_tpm[4 * CB * P1S];
-  __shared__ float s_fx[CB * NDS];
-  __shared__ float s_xf[2 * CB * P1S];
-  // C0 w and then d' take the place of w, and the traces of d' that of w's own traces; w and
-  // its traces are last read before the barrier that ends the volume and face phase (32 KB
-  // instead of 38 KB per CTA: 6 CTAs per SM instead of 5)
-  float* const s_out = s_w;
-  float* const s_dt = s_twp;
+  constexpr int P1 = S::P1, ND = S::ND;
+  __shared__ float s_sw[ND * kGsTile];        // weighted values of -cB d
+  __shared__ float s_xf[4 * P1 * kGsTile];    // x-face fluxes of B [face][component][point][lane]
+  __shared__ float s_w[2 * ND * kGsTile];     // w [component][node][lane]
   pdl_allow_next();
   const CobT<P, float>& cb = cobr<P, float>();
-  const int tid = threadIdx.x, cl = tid % CB, m = tid / CB;
-  const int c0 = blockIdx.x * CB, ncb = min(CB, ncell - c0);
-  const bool live = cl < ncb;
-  const int c = c0 + (live ? cl : ncb - 1);
-  float* g = s_geo + cl * kGsGeo;
-  gs_geometry<P>(mesh, c, m, g);
+  GsThread<P> th(mesh);
+  th.geometry(mesh);
+  th.neighbours(mesh);
+  const int lane = th.lane, m = th.m;
   pdl_wait_previous();
-  for (int e = tid; e < ncb * ND; e += NT) {
-    const int cc = e / ND, k = e % ND;
-    cp_async_el(&s_p[cc * NDS + k], pg + (size_t)c0 * ND + e);
+  const size_t oc = S::column(th.tile, m, lane), op = S::point(th.tile, m, lane);
+  const float *dB = d + oc, *wB = WA + oc, *pB = pg + oc, *tB = dtr + op, *qB = ptr + op;
+  float *fxB = fx + oc, *feB = fe + oc, *gB = gf + op;
+  float dc[P1], wa[P1], pc[P1], tm[4], tp[4], pt[4];
+#pragma unroll
+  for (int q = 0; q < P1; ++q) dc[q] = dB[q * S::SN];
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    tp[f] = tB[f * S::SF];
+    pt[f] = qB[f * S::SF];
   }
-  for (int e = tid; e < ncb * 2 * ND; e += NT) {
-    const int cc = e / (2 * ND), o = (e / ND) % 2, k = e % ND;
-    cp_async_el(&s_w[(o * CB + cc) * NDS + k], w + (size_t)c0 * 2 * ND + e);
+  gs_ends<P>(dc, tp[2], tp[3]);
+#pragma unroll
+  for (int f = 0; f < 4; ++f) tm[f] = gs_other<P>(dtr, th, f, tp[f]);
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {
+    wa[q] = wB[q * S::SN];
+    pc[q] = pB[q * S::SN];
   }
-  __syncthreads();  // the geometry block (neighbours) complete
-  gs_load_traces<P, 2>(wtr, s_geo, c0, ncb, ncell, s_twp, s_twm);
-  gs_load_traces<P, 1>(ptr, s_geo, c0, ncb, ncell, s_tpp, s_tpm);
-  // the epilogue's operands of this thread's elements (CB ND = (P+1) NT elements per CTA)
-  static_assert(CB * ND == P1 * NT, "P+1 epilogue elements per thread");
-  float ez[P1], ed[P1], ex[P1], ew[P1];
+  const float wx = cb.w[m];
+  float a0[P1], a1[P1];
+  {
+    float e0[P1], e1[P1];
 #pragma unroll
-  for (int k = 0; k < P1; ++k) {
-    const int e = tid + k * NT;
-    const size_t gi = (size_t)c0 * ND + (e < ncb * ND ? e : 0);
-    ez[k] = z[gi];
-    ed[k] = d[gi];
-    ex[k] = first ? 0.f : x[gi];
-    ew[k] = WM[gi];
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  float acc[P1];
-#pragma unroll
-  for (int i = 0; i < P1; ++i) acc[i] = 0.f;
-  if (live) {
-    const int qx = m;
-    const float xi = cb.g[qx], wx = cb.w[qx];
-    const float J01 = fmaf(g[2], xi, g[4]), J11 = fmaf(g[3], xi, g[5]);
-    const float k0 = -cdt * gg;
-#pragma unroll
-    for (int qz = 0; qz < P1; ++qz) {
-      const float eta = cb.g[qz];
-      const float J00 = fmaf(g[2], eta, g[0]), J10 = fmaf(g[3], eta, g[1]);
-      const int o = cl * NDS + qz * P1 + qx;
-      const float sv = k0 * s_p[o] * (wx * cb.w[qz]);
-      const float gr0 = sv * s_w[(0 * CB + cl) * NDS + qz * P1 + qx];
-      const float gr1 = sv * s_w[(1 * CB + cl) * NDS + qz * P1 + qx];
-      s_fx[o] = J11 * gr0 - J01 * gr1;
-      const float fe = J00 * gr1 - J10 * gr0;
-#pragma unroll
-      for (int iz = 0; iz < P1; ++iz) acc[iz] = fmaf(cb.Dg[qz][iz], fe, acc[iz]);
+    for (int q = 0; q < P1; ++q) {
+      const float sw = -cB * dc[q] * (wx * cb.w[q]);
+      s_sw[(q * P1 + m) * kGsTile + lane] = sw;
+      e0[q] = -th.J10(cb.g[q]) * sw;
+      e1[q] = th.J00(cb.g[q]) * sw;
     }
-    const float hg = 0.5f * cdt * gg;
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const int p = m;
-      float F = 0.f;
-      if (get_index(g[18 + f]) >= 0) {
-        const float nx = g[6 + 3 * f], nz = g[7 + 3 * f];
-        const float wnp = s_twp[((f * 2 + 0) * CB + cl) * P1S + p] * nx + s_twp[((f * 2 + 1) * CB + cl) * P1S + p] * nz;
-        const float wnm = s_twm[((f * 2 + 0) * CB + cl) * P1S + p] * nx + s_twm[((f * 2 + 1) * CB + cl) * P1S + p] * nz;
-        const float pp = s_tpp[(f * CB + cl) * P1S + p], pm = s_tpm[(f * CB + cl) * P1S + p];
-        F = hg * (pp * wnp + pm * wnm) * (g[8 + 3 * f] * cb.w[p]);
+    for (int i = 0; i < P1; ++i) {
+      a0[i] = cb.Dg[0][i] * e0[0];
+      a1[i] = cb.Dg[0][i] * e1[0];
+#pragma unroll
+      for (int q = 1; q < P1; ++q) {
+        a0[i] = fmaf(cb.Dg[q][i], e0[q], a0[i]);
+        a1[i] = fmaf(cb.Dg[q][i], e1[q], a1[i]);
       }
-      if (f >= 2) {
+    }
+  }
 #pragma unroll
-        for (int iz = 0; iz < P1; ++iz) acc[iz] = fmaf(f == 2 ? cb.lo[iz] : cb.hi[iz], F, acc[iz]);
-      } else {
-        s_xf[(f * CB + cl) * P1S + p] = F;
+  for (int f = 0; f < 4; ++f) {
+    float n0, n1;
+    th.normal(f, n0, n1);
+    const float a = cB * 0.5f * (tp[f] + tm[f]) * wx;
+    const float F0 = a * n0, F1 = a * n1;
+    if (f < 2) {
+      s_xf[((f * 2 + 0) * P1 + m) * kGsTile + lane] = F0;
+      s_xf[((f * 2 + 1) * P1 + m) * kGsTile + lane] = F1;
+    } else {
+#pragma unroll
+      for (int i = 0; i < P1; ++i) {
+        const float e = f == 2 ? cb.lo[i] : cb.hi[i];
+        a0[i] = fmaf(e, F0, a0[i]);
+        a1[i] = fmaf(e, F1, a1[i]);
       }
     }
   }
   __syncthreads();
-  if (live) {
-    const int ix = m;
+  // node (i, m): the x-derivative test along row i (adj(J)'s x part depends on qx alone), the
+  // x-face terms, A^{-1}; then the mapped fluxes of C0 at the point
+  {
+    float k0[P1], k1[P1];
 #pragma unroll
-    for (int iz = 0; iz < P1; ++iz) {
-      float v = acc[iz];
-      const float* fx = s_fx + cl * NDS + iz * P1;
+    for (int q = 0; q < P1; ++q) {
+      const float dg = cb.Dg[q][m];
+      k0[q] = dg * th.J11(cb.g[q]);
+      k1[q] = -dg * th.J01(cb.g[q]);
+    }
+    const float lo = cb.lo[m], hi = cb.hi[m];
+    const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]);
 #pragma unroll
-      for (int qx = 0; qx < P1; ++qx) v = fmaf(cb.Dg[qx][ix], fx[qx], v);
-      v = fmaf(cb.lo[ix], s_xf[(0 * CB + cl) * P1S + iz], v);
-      v = fmaf(cb.hi[ix], s_xf[(1 * CB + cl) * P1S + iz], v);
-      s_out[cl * NDS + iz * P1 + ix] = v;
+    for (int i = 0; i < P1; ++i) {
+      float v0 = a0[i], v1 = a1[i];
+#pragma unroll
+      for (int q = 0; q < P1; ++q) {
+        const float sw = s_sw[(i * P1 + q) * kGsTile + lane];
+        v0 = fmaf(k0[q], sw, v0);
+        v1 = fmaf(k1[q], sw, v1);
+      }
+      v0 = fmaf(lo, s_xf[(0 * P1 + i) * kGsTile + lane], v0);
+      v1 = fmaf(lo, s_xf[(1 * P1 + i) * kGsTile + lane], v1);
+      v0 = fmaf(hi, s_xf[(2 * P1 + i) * kGsTile + lane], v0);
+      v1 = fmaf(hi, s_xf[(3 * P1 + i) * kGsTile + lane], v1);
+      const float w0 = wa[i] * v0, w1 = wa[i] * v1;
+      a0[i] = w0;
+      a1[i] = w1;
+      s_w[(i * P1 + m) * kGsTile + lane] = w0;
+      s_w[(ND + i * P1 + m) * kGsTile + lane] = w1;
+      const float sv = -cgg * pc[i] * (wx * cb.w[i]);
+      fxB[i * S::SN] = sv * (J11 * w0 - J01 * w1);
+      feB[i * S::SN] = sv * (th.J00(cb.g[i]) * w1 - th.J10(cb.g[i]) * w0);
     }
   }
+  gs_ends<P>(pc, pt[2], pt[3]);
+  float t0[4], t1[4];
+  gs_ends<P>(a0, t0[2], t0[3]);
+  gs_ends<P>(a1, t1[2], t1[3]);
   __syncthreads();
-  // the update in global order (coalesced; element tid + k NT, k < P+1, of the CTA's chunk,
-  // its z, d, x and WM read at kernel start); d' back into s_out for its traces
+  gs_row_ends<P>(s_w, m, lane, t0[0], t0[1]);
+  gs_row_ends<P>(s_w + ND * kGsTile, m, lane, t1[0], t1[1]);
 #pragma unroll
-  for (int k = 0; k < P1; ++k) {
-    const int e = tid + k * NT;
-    if (e < ncb * ND) {
-      const int cc = e / ND, kk = e % ND;
-      const size_t gi = (size_t)c0 * ND + e;
-      const float y = s_out[cc * NDS + kk];
-      const float zn = ez[k] + gfac * ew[k] * y - ed[k];
-      const float nd = alpha * ed[k] + s * zn;
-      z[gi] = zn;
-      d[gi] = nd;
-      x[gi] = first ? nd : ex[k] + nd;
-      s_out[cc * NDS + kk] = nd;
-    }
+  for (int f = 0; f < 4; ++f) {
+    float n0, n1;
+    th.normal(f, n0, n1);
+    gB[f * S::SF] = 0.5f * cgg * wx * pt[f] * (t0[f] * n0 + t1[f] * n1);
+  }
+}
+
+// ------------------------------------------------- the Chebyshev step on z = D^{-1} r
+// The fluxes of C0 w (fx, fe at the points, gf at the face points) -> y = C0_g w_g, then per node
+//   z' = z + g y / JxW - d,  d' = alpha d + s z',
+// and the traces of d'.  xmode 0: x stays (its direction is added by the next step), 1: x += d + d',
+// 2: x += d'.  In place: each CTA reads only its own cells of z, d and x.
+template <int P>
+__global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
+    k_gs_zstep(const GsMesh mesh, const float* fx, const float* fe,
+               const float* gf, const float gfac, const float alpha, const float s,
+               float* z, float* d, float* x, const int xmode,
+               float* dtr) {
+  using S = GsShape<P>;
+  constexpr int P1 = S::P1, ND = S::ND;
+  __shared__ float s_fx[ND * kGsTile], s_d[ND * kGsTile], s_xf[2 * P1 * kGsTile];
+  pdl_allow_next();
+  const CobT<P, float>& cb = cobr<P, float>();
+  GsThread<P> th(mesh);
+  th.geometry(mesh);
+  th.neighbours(mesh);
+  const int lane = th.lane, m = th.m;
+  pdl_wait_previous();
+  const size_t oc = S::column(th.tile, m, lane), op = S::point(th.tile, m, lane);
+  const float *fxB = fx + oc, *feB = fe + oc, *gB = gf + op;
+  float *zB = z + oc, *dB = d + oc, *xB = x + oc, *tB = dtr + op;
+  float ec[P1], zc[P1], dc[P1], xc[P1], F[4];
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {
+    s_fx[(q * P1 + m) * kGsTile + lane] = fxB[q * S::SN];
+    ec[q] = feB[q * S::SN];
+  }
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {  // own minus the neighbour's (whose normal is the opposite); none at walls
+    const float own = gB[f * S::SF];
+    F[f] = own - gs_other<P>(gf, th, f, own);
+  }
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {
+    zc[q] = zB[q * S::SN];
+    dc[q] = dB[q * S::SN];
+    xc[q] = xmode ? xB[q * S::SN] : 0.f;
+  }
+  s_xf[m * kGsTile + lane] = F[0];
+  s_xf[(P1 + m) * kGsTile + lane] = F[1];
+  float a[P1];
+#pragma unroll
+  for (int i = 0; i < P1; ++i) {
+    a[i] = fmaf(cb.hi[i], F[3], cb.lo[i] * F[2]);
+#pragma unroll
+    for (int q = 0; q < P1; ++q) a[i] = fmaf(cb.Dg[q][i], ec[q], a[i]);
   }
   __syncthreads();
-  if (live) gs_traces<P, 1>(s_out, cl, m, s_dt);
+  const float lo = cb.lo[m], hi = cb.hi[m];
+  const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]), gw = 1.f / cb.w[m];
+#pragma unroll
+  for (int i = 0; i < P1; ++i) {
+    float y = a[i];
+#pragma unroll
+    for (int q = 0; q < P1; ++q) y = fmaf(cb.Dg[q][m], s_fx[(i * P1 + q) * kGsTile + lane], y);
+    y = fmaf(lo, s_xf[i * kGsTile + lane], y);
+    y = fmaf(hi, s_xf[(P1 + i) * kGsTile + lane], y);
+    const float det = th.J00(cb.g[i]) * J11 - th.J10(cb.g[i]) * J01;
+    const float zn = zc[i] + __fdividef(gfac * gw * y, det * cb.w[i]) - dc[i];
+    const float nd = alpha * dc[i] + s * zn;
+    zB[i * S::SN] = zn;
+    dB[i * S::SN] = nd;
+    if (xmode == 1) xB[i * S::SN] = (xc[i] + dc[i]) + nd;
+    else if (xmode == 2) xB[i * S::SN] = xc[i] + nd;
+    s_d[(i * P1 + m) * kGsTile + lane] = nd;
+    dc[i] = nd;
+  }
+  float t[4];
+  gs_ends<P>(dc, t[2], t[3]);
   __syncthreads();
-  gs_store_traces<P, 1>(s_dt, c0, ncb, ncell, dtr);
+  gs_row_ends<P>(s_d, m, lane, t[0], t[1]);
+#pragma unroll
+  for (int f = 0; f < 4; ++f) tB[f * S::SF] = t[f];
 }
 
 // ------------------------------------------------------------ basis changes
 // The preconditioner's input: v (FP64, a residual: dual, nodal) -> b_g = (Vi x Vi)^T v,
-// d = x = sc WM b_g, z = theta d and the traces of d.
+// d = x = sc b_g / JxW, z = theta d and the traces of d.
 template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT)
-    k_gs_entry(const double* __restrict__ v, const float* __restrict__ WM, const float sc, const float theta,
-               float* __restrict__ z, float* __restrict__ d, float* __restrict__ x, float* __restrict__ dtr,
-               const int ncell) {
+    k_gs_entry(const GsMesh mesh, const double* v, const float sc, const float theta,
+               float* z, float* d, float* x, float* dtr) {
   using S = GsShape<P>;
-  constexpr int P1 = S::P1, ND = S::ND, CB = S::CB, NT = S::NT, NDS = S::NDS;
-  __shared__ float s_a[CB * NDS];
-  __shared__ float s_t[4 * CB * S::P1S];
+  constexpr int P1 = S::P1, ND = S::ND, NDS = ND | 1;
+  __shared__ float s_v[kGsTile * NDS], s_t[ND * kGsTile];
   pdl_allow_next();
-  pdl_wait_previous();
   const CobT<P, float>& cb = cobr<P, float>();
-  const int tid = threadIdx.x, cl = tid % CB, m = tid / CB;
-  const int c0 = blockIdx.x * CB, ncb = min(CB, ncell - c0);
-  const bool live = cl < ncb;
-  for (int e = tid; e < ncb * ND; e += NT) s_a[(e / ND) * NDS + e % ND] = (float)v[(size_t)c0 * ND + e];
+  GsThread<P> th(mesh);
+  th.geometry(mesh);
+  const int lane = th.lane, m = th.m;
+  const int n = min(kGsTile, mesh.ncell - th.tile * kGsTile) * ND;
+  const size_t oc = S::column(th.tile, m, lane);
+  float *zB = z + oc, *dB = d + oc, *xB = x + oc, *tB = dtr + S::point(th.tile, m, lane);
+  pdl_wait_previous();
+  for (int e = threadIdx.x; e < n; e += S::NT) s_v[(e / ND) * NDS + e % ND] = (float)v[(size_t)th.tile * kGsTile * ND + e];
   __syncthreads();
-  float t[P1];
-  if (live) {  // along x on row iz = m: t[qx] = sum_ix Vi[ix][qx] v[iz][ix]
-    const float* row = s_a + cl * NDS + m * P1;
-    float r[P1];
 #pragma unroll
-    for (int i = 0; i < P1; ++i) r[i] = row[i];
+  for (int qx = 0; qx < P1; ++qx) {  // along x on row m
+    float t = 0.f;
 #pragma unroll
-    for (int qx = 0; qx < P1; ++qx) {
-      float a = 0.f;
-#pragma unroll
-      for (int ix = 0; ix < P1; ++ix) a = fmaf(cb.Vi[ix][qx], r[ix], a);
-      t[qx] = a;
-    }
+    for (int i = 0; i < P1; ++i) t = fmaf(cb.Vi[i][qx], s_v[lane * NDS + m * P1 + i], t);
+    s_t[(m * P1 + qx) * kGsTile + lane] = t;
   }
   __syncthreads();
-  if (live) {
+  float u[P1], dc[P1];
 #pragma unroll
-    for (int qx = 0; qx < P1; ++qx) s_a[cl * NDS + m * P1 + qx] = t[qx];
+  for (int i = 0; i < P1; ++i) u[i] = s_t[(i * P1 + m) * kGsTile + lane];
+  __syncthreads();
+  const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]);
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {  // along z on column m, then the weights
+    float b = 0.f;
+#pragma unroll
+    for (int i = 0; i < P1; ++i) b = fmaf(cb.Vi[i][q], u[i], b);
+    const float det = th.J00(cb.g[q]) * J11 - th.J10(cb.g[q]) * J01;
+    dc[q] = __fdividef(sc * b, det * (cb.w[m] * cb.w[q]));
+    dB[q * S::SN] = dc[q];
+    xB[q * S::SN] = dc[q];
+    zB[q * S::SN] = theta * dc[q];
+    s_t[(q * P1 + m) * kGsTile + lane] = dc[q];
   }
+  float t[4];
+  gs_ends<P>(dc, t[2], t[3]);
   __syncthreads();
-  if (live) {  // along z on column qx = m, then the weights
-    const int qx = m;
-    float u[P1];
+  gs_row_ends<P>(s_t, m, lane, t[0], t[1]);
 #pragma unroll
-    for (int iz = 0; iz < P1; ++iz) u[iz] = s_a[cl * NDS + iz * P1 + qx];
-#pragma unroll
-    for (int qz = 0; qz < P1; ++qz) {
-      float a = 0.f;
-#pragma unroll
-      for (int iz = 0; iz < P1; ++iz) a = fmaf(cb.Vi[iz][qz], u[iz], a);
-      t[qz] = a;
-    }
-  }
-  __syncthreads();
-  if (live) {
-#pragma unroll
-    for (int qz = 0; qz < P1; ++qz) s_a[cl * NDS + qz * P1 + m] = t[qz];
-  }
-  __syncthreads();
-  for (int e = tid; e < ncb * ND; e += NT) {
-    const size_t gi = (size_t)c0 * ND + e;
-    const float dv = sc * WM[gi] * s_a[(e / ND) * NDS + e % ND];
-    d[gi] = dv;
-    x[gi] = dv;
-    z[gi] = theta * dv;
-    s_a[(e / ND) * NDS + e % ND] = dv;
-  }
-  __syncthreads();
-  if (live) gs_traces<P, 1>(s_a, cl, m, s_t);
-  __syncthreads();
-  gs_store_traces<P, 1>(s_t, c0, ncb, ncell, dtr);
+  for (int f = 0; f < 4; ++f) tB[f * S::SF] = t[f];
 }
 
 // The preconditioner's output: x = (Vi x Vi) x_g (nodal, FP64).
 template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT)
-    k_gs_exit(const float* __restrict__ xg, double* __restrict__ out, const int ncell) {
+    k_gs_exit(const float* xg, double* out, const int ncell) {
   using S = GsShape<P>;
-  constexpr int P1 = S::P1, ND = S::ND, CB = S::CB, NT = S::NT, NDS = S::NDS;
-  __shared__ float s_a[CB * NDS];
+  constexpr int P1 = S::P1, ND = S::ND, NDS = ND | 1;
+  __shared__ float s_v[kGsTile * NDS], s_t[ND * kGsTile];
   pdl_allow_next();
-  pdl_wait_previous();
   const CobT<P, float>& cb = cobr<P, float>();
-  const int tid = threadIdx.x, cl = tid % CB, m = tid / CB;
-  const int c0 = blockIdx.x * CB, ncb = min(CB, ncell - c0);
-  const bool live = cl < ncb;
-  for (int e = tid; e < ncb * ND; e += NT) s_a[(e / ND) * NDS + e % ND] = xg[(size_t)c0 * ND + e];
-  __syncthreads();
-  float t[P1];
-  if (live) {  // along z on column qx = m: t[iz] = sum_qz Vi[iz][qz] x_g[qz][qx]
-    float u[P1];
+  const int lane = threadIdx.x & 31, m = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), tile = blockIdx.x;
+  const int n = min(kGsTile, ncell - tile * kGsTile) * ND;
+  pdl_wait_previous();
+  float u[P1];
 #pragma unroll
-    for (int qz = 0; qz < P1; ++qz) u[qz] = s_a[cl * NDS + qz * P1 + m];
+  for (int q = 0; q < P1; ++q) u[q] = xg[S::column(tile, m, lane) + q * S::SN];
 #pragma unroll
-    for (int iz = 0; iz < P1; ++iz) {
-      float a = 0.f;
+  for (int i = 0; i < P1; ++i) {  // along z on column m
+    float t = 0.f;
 #pragma unroll
-      for (int qz = 0; qz < P1; ++qz) a = fmaf(cb.Vi[iz][qz], u[qz], a);
-      t[iz] = a;
-    }
+    for (int q = 0; q < P1; ++q) t = fmaf(cb.Vi[i][q], u[q], t);
+    s_t[(i * P1 + m) * kGsTile + lane] = t;
   }
   __syncthreads();
-  if (live) {
 #pragma unroll
-    for (int iz = 0; iz < P1; ++iz) s_a[cl * NDS + iz * P1 + m] = t[iz];
+  for (int q = 0; q < P1; ++q) u[q] = s_t[(m * P1 + q) * kGsTile + lane];
+#pragma unroll
+  for (int i = 0; i < P1; ++i) {  // along x on row m
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < P1; ++q) t = fmaf(cb.Vi[i][q], u[q], t);
+    s_v[lane * NDS + m * P1 + i] = t;
   }
   __syncthreads();
-  if (live) {  // along x on row iz = m
-    float r[P1];
-#pragma unroll
-    for (int qx = 0; qx < P1; ++qx) r[qx] = s_a[cl * NDS + m * P1 + qx];
-#pragma unroll
-    for (int ix = 0; ix < P1; ++ix) {
-      float a = 0.f;
-#pragma unroll
-      for (int qx = 0; qx < P1; ++qx) a = fmaf(cb.Vi[ix][qx], r[qx], a);
-      t[ix] = a;
-    }
-  }
-  __syncthreads();
-  if (live) {
-#pragma unroll
-    for (int ix = 0; ix < P1; ++ix) s_a[cl * NDS + m * P1 + ix] = t[ix];
-  }
-  __syncthreads();
-  for (int e = tid; e < ncb * ND; e += NT) out[(size_t)c0 * ND + e] = (double)s_a[(e / ND) * NDS + e % ND];
+  for (int e = threadIdx.x; e < n; e += S::NT)
+    out[(size_t)tile * kGsTile * ND + e] = (double)s_v[(e / ND) * NDS + e % ND];
 }
 
-// A coefficient field (FP64, nodal) at the Gauss points, pg = (V x V) p, and its traces.
+// A coefficient field (FP64, nodal) at the Gauss points, pg = (V x V) p, and its traces on faces 0, 1
+// (those on faces 2 and 3 are formed from the columns where they are used); and, given rho, the
+// Gauss-point inverse weights of A, WA = 1 / (rho JxW).
 template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT)
-    k_gs_values(const double* __restrict__ p, float* __restrict__ pg, float* __restrict__ ptr, const int ncell) {
+    k_gs_values(const MeshDev mesh, const double* __restrict__ p, const double* __restrict__ rho,
+                float* __restrict__ pg, float* __restrict__ ptr, float* __restrict__ WA, const int ncell) {
   using S = GsShape<P>;
-  constexpr int P1 = S::P1, ND = S::ND, CB = S::CB, NT = S::NT, NDS = S::NDS;
-  __shared__ double s_a[CB * NDS];
+  constexpr int P1 = S::P1, ND = S::ND, NDS = ND | 1;
+  __shared__ double s_v[kGsTile * NDS], s_t[ND * kGsTile];
   const CobT<P, double>& cb = cobr<P, double>();
-  const int tid = threadIdx.x, cl = tid % CB, m = tid / CB;
-  const int c0 = blockIdx.x * CB, ncb = min(CB, ncell - c0);
-  const bool live = cl < ncb;
-  const int c = c0 + (live ? cl : ncb - 1);
-  for (int e = tid; e < ncb * ND; e += NT) s_a[(e / ND) * NDS + e % ND] = p[(size_t)c0 * ND + e];
-  __syncthreads();
-  double t[P1];
-  if (live) {  // along x on row iz = m: t[qx] = sum_ix V[qx][ix] p[iz][ix]
+  const int lane = threadIdx.x & 31, m = threadIdx.x >> 5, tile = blockIdx.x;
+  const int n = min(kGsTile, ncell - tile * kGsTile) * ND;
+  const int c = min(tile * kGsTile + lane, ncell - 1);
+  // the values of a nodal field at the points of column m
+  auto values = [&](const double* __restrict__ v, double* u) {
+    for (int e = threadIdx.x; e < n; e += S::NT) s_v[(e / ND) * NDS + e % ND] = v[(size_t)tile * kGsTile * ND + e];
+    __syncthreads();
     double r[P1];
 #pragma unroll
-    for (int i = 0; i < P1; ++i) r[i] = s_a[cl * NDS + m * P1 + i];
+    for (int i = 0; i < P1; ++i) r[i] = s_v[lane * NDS + m * P1 + i];
 #pragma unroll
-    for (int qx = 0; qx < P1; ++qx) {
-      double a = 0.0;
+    for (int q = 0; q < P1; ++q) {  // along x on row m
+      double t = 0.0;
 #pragma unroll
-      for (int ix = 0; ix < P1; ++ix) a = fma(cb.V[qx][ix], r[ix], a);
-      t[qx] = a;
+      for (int i = 0; i < P1; ++i) t = fma(cb.V[q][i], r[i], t);
+      s_t[(m * P1 + q) * kGsTile + lane] = t;
     }
-  }
-  __syncthreads();
-  if (live) {
+    __syncthreads();
 #pragma unroll
-    for (int qx = 0; qx < P1; ++qx) s_a[cl * NDS + m * P1 + qx] = t[qx];
-  }
-  __syncthreads();
-  if (live) {  // along z on column qx = m
-    double u[P1];
+    for (int i = 0; i < P1; ++i) r[i] = s_t[(i * P1 + m) * kGsTile + lane];
+    __syncthreads();
 #pragma unroll
-    for (int iz = 0; iz < P1; ++iz) u[iz] = s_a[cl * NDS + iz * P1 + m];
+    for (int q = 0; q < P1; ++q) {  // along z on column m
+      double t = 0.0;
 #pragma unroll
-    for (int qz = 0; qz < P1; ++qz) {
-      double a = 0.0;
-#pragma unroll
-      for (int iz = 0; iz < P1; ++iz) a = fma(cb.V[qz][iz], u[iz], a);
-      t[qz] = a;
+      for (int i = 0; i < P1; ++i) t = fma(cb.V[q][i], r[i], t);
+      u[q] = t;
     }
+  };
+  double u[P1];
+  values(p, u);
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {
+    pg[S::column(tile, m, lane) + q * S::SN] = (float)u[q];
+    s_t[(q * P1 + m) * kGsTile + lane] = u[q];
   }
   __syncthreads();
-  if (live) {
+  double lo = 0.0, hi = 0.0;
 #pragma unroll
-    for (int qz = 0; qz < P1; ++qz) s_a[cl * NDS + qz * P1 + m] = t[qz];
+  for (int i = 0; i < P1; ++i) {
+    lo = fma(cb.lo[i], s_t[(m * P1 + i) * kGsTile + lane], lo);
+    hi = fma(cb.hi[i], s_t[(m * P1 + i) * kGsTile + lane], hi);
   }
+  ptr[S::point(tile, m, lane)] = (float)lo;
+  ptr[S::point(tile, m, lane) + S::SF] = (float)hi;
   __syncthreads();
-  for (int e = tid; e < ncb * ND; e += NT) pg[(size_t)c0 * ND + e] = (float)s_a[(e / ND) * NDS + e % ND];
-  if (live) {
-    const double* cell = s_a + cl * NDS;
-    double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
+  values(rho, u);
+  const int i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
+  const double2* v = mesh.vtx + (size_t)j * W + i;
+  const double2 v0 = v[0], v1 = v[1], v2 = v[W], v3 = v[W + 1];
+  const double Ax = v1.x - v0.x, Az = v1.y - v0.y, Cx = v2.x - v0.x, Cz = v2.y - v0.y;
+  const double Bx = v3.x - v2.x - v1.x + v0.x, Bz = v3.y - v2.y - v1.y + v0.y;
+  const double xi = cb.g[m], J01 = fma(Bx, xi, Cx), J11 = fma(Bz, xi, Cz);
 #pragma unroll
-    for (int i = 0; i < P1; ++i) {
-      t0 = fma(cb.lo[i], cell[m * P1 + i], t0);
-      t1 = fma(cb.hi[i], cell[m * P1 + i], t1);
-      t2 = fma(cb.lo[i], cell[i * P1 + m], t2);
-      t3 = fma(cb.hi[i], cell[i * P1 + m], t3);
-    }
-    ptr[((size_t)0 * ncell + c) * P1 + m] = (float)t0;
-    ptr[((size_t)1 * ncell + c) * P1 + m] = (float)t1;
-    ptr[((size_t)2 * ncell + c) * P1 + m] = (float)t2;
-    ptr[((size_t)3 * ncell + c) * P1 + m] = (float)t3;
+  for (int q = 0; q < P1; ++q) {
+    const double eta = cb.g[q], J00 = fma(Bx, eta, Ax), J10 = fma(Bz, eta, Az);
+    WA[S::column(tile, m, lane) + q * S::SN] = (float)(1.0 / (u[q] * ((J00 * J11 - J01 * J10) * cb.w[m] * cb.w[q])));
   }
 }
 

@@ -129,22 +129,27 @@ struct DegreeOps {
   cudaError_t (*res_chebz_f)(const MeshDev&, const float* w, const float* pf, const float* din,
                              const CParamsT<float>&, const float* WM, float g, float alpha, float s, float* z,
                              float* dout, float* x, int first, int reduced, int ncell, cudaStream_t);
-  // ---- the same smoother in the Gauss-point basis (af_gauss.cuh): vectors hold values at the
-  // (P+1)^2 Gauss points, face traces tr[face][comp][cell][P+1] go with them
-  //   entry: d = x = sc WM (Vi x Vi)^T v (v FP64 nodal), z = theta d, dtr = traces of d
-  cudaError_t (*gs_entry)(const double* v, const float* WM, float sc, float theta, float* z, float* d, float* x,
-                          float* dtr, int ncell, cudaStream_t);
-  //   w = scale diag(WA) B_g d (two components) and its traces
-  cudaError_t (*gs_binv)(const MeshDev&, const float* d, const float* dtr, float c, const float* WA, float scale,
-                         float* w, float* wtr, int ncell, cudaStream_t);
-  //   z += g WM C0_g(w; pg) - d;  d = alpha d + s z (in place);  x += d;  dtr = traces of d
-  cudaError_t (*gs_zstep)(const MeshDev&, const float* w, const float* wtr, const float* pg, const float* ptr,
-                          float cdt, float gg, const float* WM, float g, float alpha, float s, float* z, float* d,
+  // ---- the same smoother in the Gauss-point basis (af_gauss.cuh): fields and face arrays in its
+  // layout, tiled by gs_tile cells; geo: the mesh's geometry block (kGsGeo floats per cell)
+  cudaError_t (*gs_geo)(const MeshDev&, float* geo, int ncell, cudaStream_t);
+  //   entry: d = x = sc (Vi x Vi)^T v / JxW (v FP64 nodal), z = theta d, dtr = traces of d
+  cudaError_t (*gs_entry)(const MeshDev&, const float* geo, const double* v, float sc, float theta, float* z, float* d,
                           float* x, float* dtr, int ncell, cudaStream_t);
+  //   w = diag(WA) B_g d, written as the mapped fluxes of C0 w at the points (fx, fe) and on the
+  //   faces (gf); pg, ptr: p_fixed at the points and on the x-faces; cgg = cdt gamma/(gamma-1)
+  cudaError_t (*gs_binv)(const MeshDev&, const float* geo, const float* d, const float* dtr, float cB, const float* WA,
+                         const float* pg, const float* ptr, float cgg, float* fx, float* fe, float* gf, int ncell,
+                         cudaStream_t);
+  //   z += g C0_g w / JxW - d;  d = alpha d + s z (in place);  x += 0, d_old + d, d (xmode 0, 1, 2);
+  //   dtr = traces of d
+  cudaError_t (*gs_zstep)(const MeshDev&, const float* geo, const float* fx, const float* fe, const float* gf, float g,
+                          float alpha, float s, float* z, float* d, float* x, int xmode, float* dtr, int ncell,
+                          cudaStream_t);
   //   out = (Vi x Vi) x (FP64 nodal)
   cudaError_t (*gs_exit)(const float* x, double* out, int ncell, cudaStream_t);
-  //   a coefficient at the Gauss points and its traces: pg = (V x V) p
-  cudaError_t (*gs_values)(const double* p, float* pg, float* ptr, int ncell, cudaStream_t);
+  //   the coefficients: pg = (V x V) p, its x-face traces, WA = 1 / (rho JxW)
+  cudaError_t (*gs_values)(const MeshDev&, const double* p, const double* rho, float* pg, float* ptr, float* WA,
+                           int ncell, cudaStream_t);
 };
 
 const DegreeOps* degree_ops(int P);  // null if the degree was not compiled

@@ -1069,12 +1069,11 @@ cudaError_t res_chebz_f(const MeshDev& mesh, const float* w, const float* pf, co
 // ------------------------------------------------------------------ Gauss-point smoother
 template <class K, class... A>
 cudaError_t launch_gs(K kernel, int ncell, cudaStream_t st, bool pdl, A... args) {
-  using S = GsShape<P>;
-  const int nblk = (ncell + S::CB - 1) / S::CB;
+  const int nblk = (ncell + kGsTile - 1) / kGsTile;
   if (ncell <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)nblk);
-  cfg.blockDim = dim3((unsigned)S::NT);
+  cfg.blockDim = dim3((unsigned)GsShape<P>::NT);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1083,27 +1082,34 @@ cudaError_t launch_gs(K kernel, int ncell, cudaStream_t st, bool pdl, A... args)
   cfg.numAttrs = (kPDL && pdl) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
-cudaError_t gs_entry(const double* v, const float* WM, float sc, float theta, float* z, float* d, float* x,
-                     float* dtr, int ncell, cudaStream_t st) {
-  return launch_gs(k_gs_entry<P>, ncell, st, true, v, WM, sc, theta, z, d, x, dtr, ncell);
+GsMesh gs_mesh(const MeshDev& m, const float* geo, int ncell) {
+  return {geo, FastDiv::make(m.nx), m.nz, m.periodic_x, ncell};
 }
-cudaError_t gs_binv(const MeshDev& mesh, const float* d, const float* dtr, float c, const float* WA, float scale,
-                    float* w, float* wtr, int ncell, cudaStream_t st) {
-  if (mesh.cell0 != 0) return cudaErrorInvalidValue;
-  return launch_gs(k_gs_binv<P>, ncell, st, true, mesh, d, dtr, c, WA, scale, w, wtr, ncell);
+cudaError_t gs_geo(const MeshDev& mesh, float* geo, int ncell, cudaStream_t st) {
+  k_gs_geo<<<(ncell + 255) / 256, 256, 0, st>>>(mesh, geo, ncell);
+  return cudaGetLastError();
 }
-cudaError_t gs_zstep(const MeshDev& mesh, const float* w, const float* wtr, const float* pg, const float* ptr,
-                     float cdt, float gg, const float* WM, float g, float alpha, float s, float* z, float* d,
+cudaError_t gs_entry(const MeshDev& mesh, const float* geo, const double* v, float sc, float theta, float* z, float* d,
                      float* x, float* dtr, int ncell, cudaStream_t st) {
-  if (mesh.cell0 != 0) return cudaErrorInvalidValue;
-  return launch_gs(k_gs_zstep<P>, ncell, st, true, mesh, w, wtr, pg, ptr, cdt, gg, WM, g, alpha, s, z, d, x, 0, dtr,
-                   ncell);
+  return launch_gs(k_gs_entry<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), v, sc, theta, z, d, x, dtr);
+}
+cudaError_t gs_binv(const MeshDev& mesh, const float* geo, const float* d, const float* dtr, float cB, const float* WA,
+                    const float* pg, const float* ptr, float cgg, float* fx, float* fe, float* gf, int ncell,
+                    cudaStream_t st) {
+  return launch_gs(k_gs_binv<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), d, dtr, cB, WA, pg, ptr, cgg, fx, fe, gf);
+}
+cudaError_t gs_zstep(const MeshDev& mesh, const float* geo, const float* fx, const float* fe, const float* gf, float g,
+                     float alpha, float s, float* z, float* d, float* x, int xmode, float* dtr, int ncell,
+                     cudaStream_t st) {
+  return launch_gs(k_gs_zstep<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), fx, fe, gf, g, alpha, s, z, d, x, xmode,
+                   dtr);
 }
 cudaError_t gs_exit(const float* x, double* out, int ncell, cudaStream_t st) {
   return launch_gs(k_gs_exit<P>, ncell, st, true, x, out, ncell);
 }
-cudaError_t gs_values(const double* p, float* pg, float* ptr, int ncell, cudaStream_t st) {
-  return launch_gs(k_gs_values<P>, ncell, st, false, p, pg, ptr, ncell);
+cudaError_t gs_values(const MeshDev& mesh, const double* p, const double* rho, float* pg, float* ptr, float* WA,
+                      int ncell, cudaStream_t st) {
+  return launch_gs(k_gs_values<P>, ncell, st, false, mesh, p, rho, pg, ptr, WA, ncell);
 }
 
 cudaError_t op_A_rho_T(const MeshDev& mesh, const double* x, const double* y, double* rhobar, int ncell,
@@ -1156,9 +1162,10 @@ const DegreeOps kOps = {upload_tables,     rhs,
                         b_inv_fr,          res_cheb_fr,
                         op_A_rho_T,        op_C_pf_T,
                         rhs_tangent,       rhs_adjoint,
-                        res_chebz_f,       gs_entry,
-                        gs_binv,           gs_zstep,
-                        gs_exit,           gs_values};
+                        res_chebz_f,       gs_geo,
+                        gs_entry,          gs_binv,
+                        gs_zstep,          gs_exit,
+                        gs_values};
 
 }  // namespace
 

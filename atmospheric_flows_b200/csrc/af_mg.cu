@@ -161,9 +161,10 @@ struct Level {
   void* LA = nullptr;
   void* LM = nullptr;
   void *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *u = nullptr, *w = nullptr;
-  // the Gauss-point smoother (af_gauss.cuh): face traces of d and w, p_fixed at the Gauss
-  // points and its traces
-  float *gdtr = nullptr, *gwtr = nullptr, *gpg = nullptr, *gptr = nullptr;
+  // the Gauss-point smoother (af_gauss.cuh), in its tiled layout: the geometry block, face traces of
+  // d, face fluxes of w, p_fixed at the Gauss points and its x-face traces, inverse weights of A; its
+  // fields d, x, z and the fluxes of w use the vectors above (allocated for whole tiles)
+  float *ggeo = nullptr, *gdtr = nullptr, *gwf = nullptr, *gpg = nullptr, *gptr = nullptr, *gWA = nullptr;
   double lmax = 0.0;
 };
 
@@ -423,8 +424,12 @@ int setup_levels(af_schur_solver* s, bool estimate) {
       MG_CU(k->inject(F.pf, L.pf, L.nx, L.nz, o->stream));
       o->launches += 2;
     }
+    if (s->gauss) {
+      MG_CU(k->gs_values(L.mesh, L.pf, L.rho, L.gpg, L.gptr, L.gWA, L.ncell, o->stream));
+      o->launches += 1;
+      if (!estimate) continue;  // the nodal coefficients below serve the eigenvalue estimate alone
+    }
     k_convert<double, R><<<nblocks(L.ns), kThreads, 0, o->stream>>>(L.pf, (R*)L.pfR, L.ns);
-    if (s->gauss) MG_CU(k->gs_values(L.pf, L.gpg, L.gptr, L.ncell, o->stream));
     if (sizeof(R) == sizeof(float)) {  // Gauss-point inverse weights of A
       MG_CU(k->cob_weights_f(L.mesh, L.rho, (float*)L.LA, L.ncell, o->stream));
     } else if (l == 0) {  // the operator's own inverse of A (built once per rho_for_fixed)
@@ -464,6 +469,9 @@ int build_mass_inverses(af_schur_solver* s) {
   return AF_OK;
 }
 
+// elements of a field of the Gauss-point smoother: whole tiles of 32 cells
+size_t gs_padded(int ncell, int nd) { return (size_t)(ncell + 31) / 32 * 32 * nd; }
+
 // z = the single-level FP32 Chebyshev polynomial in the Gauss-point basis applied to v (FP64 in
 // and out): the iteration of chebyshev() on z = D^{-1} r (zero start, no final residual), with
 // the basis changed at entry and exit (af_gauss.cuh)
@@ -477,19 +485,21 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
   float* zg = (float*)L.r;
   float* d = (float*)L.d;
   float* x = (float*)L.x;
-  const float* WM = (const float*)L.LM;
+  float *fx = (float*)L.w, *fe = fx + gs_padded(L.ncell, o->nd);
   // d = x = D^{-1} v / theta;  z = D^{-1} v = theta d
-  MG_CU(k->gs_entry(v, WM, (float)(ginv / theta), (float)theta, zg, d, x, L.gdtr, L.ncell, o->stream));
+  MG_CU(k->gs_entry(L.mesh, L.ggeo, v, (float)(ginv / theta), (float)theta, zg, d, x, L.gdtr, L.ncell, o->stream));
   o->launches += 1;
   double rho_old = 1.0 / sigma;
-  for (int it = 1; it < s->opt.coarse_degree; ++it) {
+  const int last = s->opt.coarse_degree - 1;
+  for (int it = 1; it <= last; ++it) {
     const double rho = 1.0 / (2.0 * sigma - rho_old);
     const double a = rho * rho_old, sc = 2.0 * rho / delta;
-    // w = A^{-1} B d;  z += D^{-1} C0 w - d;  d = a d + sc z;  x += d  (two launches)
-    MG_CU(k->gs_binv(L.mesh, d, L.gdtr, (float)s->cB, (const float*)L.LA, 1.0f, (float*)L.w, L.gwtr, L.ncell,
-                     o->stream));
-    MG_CU(k->gs_zstep(L.mesh, (const float*)L.w, L.gwtr, L.gpg, L.gptr, (float)s->cdt, (float)kGG, WM, (float)ginv,
-                      (float)a, (float)sc, zg, d, x, L.gdtr, L.ncell, o->stream));
+    // w = A^{-1} B d;  z += D^{-1} C0 w - d;  d = a d + sc z;  x += d (two launches; x takes the
+    // directions of an odd step and the next one together)
+    MG_CU(k->gs_binv(L.mesh, L.ggeo, d, L.gdtr, (float)s->cB, L.gWA, L.gpg, L.gptr, (float)(s->cdt * kGG), fx, fe,
+                     L.gwf, L.ncell, o->stream));
+    MG_CU(k->gs_zstep(L.mesh, L.ggeo, fx, fe, L.gwf, (float)ginv, (float)a, (float)sc, zg, d, x,
+                      it % 2 == 0 ? 1 : (it == last ? 2 : 0), L.gdtr, L.ncell, o->stream));
     o->launches += 2;
     rho_old = rho;
   }
@@ -624,16 +634,21 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
     if ((r = alloc(s, &L.pfR, rs * L.ns)) != AF_OK) return cleanup(r);
     if ((r = alloc(s, &L.LA, rs * nf)) != AF_OK) return cleanup(r);
     if ((r = alloc(s, &L.LM, rs * nf)) != AF_OK) return cleanup(r);
+    const size_t nv = s->gauss ? gs_padded(L.ncell, nd) : (size_t)L.ns;
     for (void** p : {&L.x, &L.b, &L.r, &L.d})
-      if ((r = alloc(s, p, rs * L.ns)) != AF_OK) return cleanup(r);
+      if ((r = alloc(s, p, rs * nv)) != AF_OK) return cleanup(r);
     for (void** p : {&L.u, &L.w})
-      if ((r = alloc(s, p, rs * 2 * L.ns)) != AF_OK) return cleanup(r);
+      if ((r = alloc(s, p, rs * 2 * nv)) != AF_OK) return cleanup(r);
     if (s->gauss) {
-      const size_t nt = sizeof(float) * 4 * (size_t)L.ncell * (op->P + 1);
-      if ((r = alloc(s, (void**)&L.gdtr, nt)) != AF_OK) return cleanup(r);
-      if ((r = alloc(s, (void**)&L.gwtr, 2 * nt)) != AF_OK) return cleanup(r);
-      if ((r = alloc(s, (void**)&L.gptr, nt)) != AF_OK) return cleanup(r);
-      if ((r = alloc(s, (void**)&L.gpg, sizeof(float) * L.ns)) != AF_OK) return cleanup(r);
+      const size_t cells = gs_padded(L.ncell, 1), nt = 4 * cells * (op->P + 1);
+      if ((r = alloc(s, (void**)&L.ggeo, sizeof(float) * 6 * cells)) != AF_OK) return cleanup(r);
+      for (float** p : {&L.gdtr, &L.gwf, &L.gptr})
+        if ((r = alloc(s, (void**)p, sizeof(float) * nt)) != AF_OK) return cleanup(r);
+      for (float** p : {&L.gpg, &L.gWA})
+        if ((r = alloc(s, (void**)p, sizeof(float) * nv)) != AF_OK) return cleanup(r);
+      if (op->ops->gs_geo(L.mesh, L.ggeo, L.ncell, op->stream) != cudaSuccess)
+        return cleanup(merr(AF_CUDA, "af_schur_solver_create: geometry block"));
+      op->launches += 1;
     }
   }
   s->nact = (int)s->lv.size();
