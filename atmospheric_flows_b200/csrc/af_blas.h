@@ -34,16 +34,36 @@ cudaError_t cg_start(KrylovState* s, const double* b, const double* Ax, const do
 cudaError_t cg_after_apply(KrylovState* s, double* x, double* r, double* z, double* p, const double* Ap,
                            const double* invd, long n, double* part, int maxit, cudaStream_t st);
 
-// GMRES / fixed-point helpers
-// out[j] = V_j . w, j < k, V_j = V + j*ldv  (partial needs k * reduce_blocks(n) <= 4*kMaxPartials doubles)
-cudaError_t mdot(const double* V, long ldv, int k, const double* w, long n, double* partial, double* out,
-                 cudaStream_t st);
-cudaError_t maxpy(const double* V, long ldv, int k, const double* h, double* w, long n, cudaStream_t st);  // w -= V h
+// ---- Krylov basis kernels.  One KrylovWork per solver: reduction partials, the block counter of
+// the finishing block, the results on the device and, in mapped pinned memory, on the host (read
+// after a stream synchronisation, no copy).
+constexpr int kKrylovMax = 64;  // basis vectors
+struct KrylovWork {
+  double* dev = nullptr;     // partials, then h1[kKrylovMax], h2[kKrylovMax], norm^2 (slot 0, 1)
+  unsigned* count = nullptr;
+  double* host = nullptr;    // h[kKrylovMax], then kHostSlots scalars
+  double* host_dev = nullptr;  // the same memory as the device sees it
+  static constexpr int kHostSlots = 8;
+  double h(int j) const { return static_cast<const volatile double*>(host)[j]; }
+  double slot(int s) const { return static_cast<const volatile double*>(host)[kKrylovMax + s]; }
+  double* slot_dev(int s) const { return host_dev + kKrylovMax + s; }
+};
+cudaError_t krylov_create(KrylovWork* k);
+void krylov_destroy(KrylovWork* k);
+// w orthogonalised against V_0 .. V_{k-1} (V_j = V + j*ldv; k <= kKrylovMax) by classical Gram-Schmidt
+// applied twice, w = pre .* w first when pre is given; then w scaled by 1/|w| (when |w| > 0).  Host:
+// h(j) = the sum of both passes' coefficients, slot(0) = |w|^2 before the scaling.
+cudaError_t gram_schmidt(const KrylovWork& kw, const double* V, long ldv, int k, double* w, const double* pre, long n,
+                         cudaStream_t st);
+constexpr int kGramSchmidtLaunches = 4;
+// r = b - r (pre .* (b - r) when pre is given);  v = r / |r| (when |r| > 0);  slot(1) = |r|^2
+cudaError_t residual_start(const KrylovWork& kw, const double* b, double* r, const double* pre, double* v, long n,
+                           cudaStream_t st);
+// slot(s) = |x|^2, s >= 2
+cudaError_t norm2_host(const KrylovWork& kw, const double* x, long n, int s, cudaStream_t st);
 cudaError_t mcombine(const double* V, long ldv, int k, const double* y_host, double* x, long n,
                      cudaStream_t st);  // x += V y
-cudaError_t scale(double a, const double* x, double* y, long n, cudaStream_t st);   // y = a x
 cudaError_t dmul(const double* d, const double* x, double* z, long n, cudaStream_t st);  // z = d .* x
-cudaError_t sub(const double* x, const double* y, double* z, long n, cudaStream_t st);   // z = x - y
 // out[0] = max|x|, out[1] = max|x - y| (0 when y is null); partial needs 2*kMaxPartials doubles
 cudaError_t maxabs2(const double* x, const double* y, long n, double* partial, double* out, cudaStream_t st);
 // state->tol2 = eps^2 * bb[0]  (bb a device scalar, e.g. |b|^2 from dot)

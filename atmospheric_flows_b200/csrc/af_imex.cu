@@ -44,7 +44,8 @@ struct af_imex {
   // CG workspace and inverse diagonals
   double *cg_r, *cg_z, *cg_p, *cg_Ap, *invd_u, *invd_M, *invd_D;
   // GMRES workspace
-  double *V, *gw, *d_h, *scal;
+  double *V, *gw, *scal;
+  KrylovWork kw;
   double* part;
   KrylovState* kst;
   af_schur_solver* schur = nullptr;  // FGMRES + Jacobi/multigrid (schur_preconditioner >= 0)
@@ -120,54 +121,43 @@ static int cg_solve(af_imex* h, const Apply& A, const double* invd, double* x, c
   return AF_OK;
 }
 
-// GMRES with left Jacobi preconditioning (deal.II SolverGMRES defaults), |P^{-1} r| <= tol
-static int gmres_solve(af_imex* h, const Apply& A, const double* invd, double* x, const double* b, long n, double tol,
+// GMRES with left Jacobi preconditioning (deal.II SolverGMRES defaults), |P^{-1} r| <= eps |b|
+static int gmres_solve(af_imex* h, const Apply& A, const double* invd, double* x, const double* b, long n, double eps,
                        int* its_out) {
   cudaStream_t st = h->op->stream;
   const int m = h->opt.gmres_restart;
   const long ld = krylov_stride(n);  // basis vectors start on 16-byte boundaries
   int total = 0;
-  std::vector<double> H((m + 1) * m), cs(m), sn(m), g(m + 1), hh(2 * (m + 1));
+  std::vector<double> H((m + 1) * m), cs(m), sn(m), g(m + 1);
   auto Hs = [&](int i, int j) -> double& { return H[i * m + j]; };
-  double res = 0.0;
+  double res = 0.0, tol = -1.0;
   bool converged = false;
+  // |b|^2 arrives with the first residual's norm
+  IM_CU(norm2_host(h->kw, b, n, 2, st));
+  h->op->launches += 1;
   while (true) {
     IM_AF(A(x, h->gw));
-    IM_CU(sub(b, h->gw, h->gw, n, st));
-    IM_CU(dmul(invd, h->gw, h->gw, n, st));
-    IM_CU(dot(h->gw, nullptr, n, h->part, h->scal, st));
-    double beta2 = 0.0;
-    IM_CU(cudaMemcpyAsync(&beta2, h->scal, sizeof(double), cudaMemcpyDeviceToHost, st));
+    IM_CU(residual_start(h->kw, b, h->gw, invd, h->V, n, st));  // V_0 = P^{-1} r / |P^{-1} r|
+    h->op->launches += 2;
     IM_AF(sync_checked(h->op, st));
-    h->op->launches += 4;
-    const double beta = std::sqrt(beta2);
+    if (tol < 0.0) tol = eps * std::sqrt(h->kw.slot(2));
+    const double beta = std::sqrt(h->kw.slot(1));
     res = beta;
     if (!std::isfinite(beta)) return ierr(AF_NAN, "GMRES: NaN residual");
     if (beta <= tol) { converged = true; break; }
     if (total >= h->opt.max_iterations) break;
-    IM_CU(scale(1.0 / beta, h->gw, h->V, n, st));
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int jend = -1;
     for (int j = 0; j < m; ++j) {
       double* w = h->V + (long)(j + 1) * ld;
       IM_AF(A(h->V + (long)j * ld, w));
-      IM_CU(dmul(invd, w, w, n, st));
-      // classical Gram-Schmidt, twice
-      IM_CU(mdot(h->V, ld, j + 1, w, n, h->part, h->d_h, st));
-      IM_CU(maxpy(h->V, ld, j + 1, h->d_h, w, n, st));
-      IM_CU(mdot(h->V, ld, j + 1, w, n, h->part, h->d_h + (m + 1), st));
-      IM_CU(maxpy(h->V, ld, j + 1, h->d_h + (m + 1), w, n, st));
-      IM_CU(dot(w, nullptr, n, h->part, h->scal, st));
-      IM_CU(cudaMemcpyAsync(hh.data(), h->d_h, sizeof(double) * 2 * (m + 1), cudaMemcpyDeviceToHost, st));
-      double hn2 = 0.0;
-      IM_CU(cudaMemcpyAsync(&hn2, h->scal, sizeof(double), cudaMemcpyDeviceToHost, st));
+      IM_CU(gram_schmidt(h->kw, h->V, ld, j + 1, w, invd, n, st));
+      h->op->launches += kGramSchmidtLaunches;
       IM_AF(sync_checked(h->op, st));
-      h->op->launches += 10;
-      for (int i = 0; i <= j; ++i) Hs(i, j) = hh[i] + hh[(m + 1) + i];
-      const double hn = std::sqrt(hn2);
+      for (int i = 0; i <= j; ++i) Hs(i, j) = h->kw.h(i);
+      const double hn = std::sqrt(h->kw.slot(0));
       Hs(j + 1, j) = hn;
-      if (hn > 0.0) IM_CU(scale(1.0 / hn, w, w, n, st));
       for (int i = 0; i < j; ++i) {  // previous rotations
         const double t = cs[i] * Hs(i, j) + sn[i] * Hs(i + 1, j);
         Hs(i + 1, j) = -sn[i] * Hs(i, j) + cs[i] * Hs(i + 1, j);
@@ -204,14 +194,6 @@ static int gmres_solve(af_imex* h, const Apply& A, const double* invd, double* x
   h->stats.gmres_iterations += total;
   if (!converged) return ierr(AF_NO_CONVERGENCE, "GMRES: no convergence within max_iterations");
   return AF_OK;
-}
-
-static double l2norm(af_imex* h, const double* x, long n) {
-  double v = 0.0;
-  dot(x, nullptr, n, h->part, h->scal, h->op->stream);
-  cudaMemcpyAsync(&v, h->scal, sizeof(double), cudaMemcpyDeviceToHost, h->op->stream);
-  cudaStreamSynchronize(h->op->stream);
-  return std::sqrt(v);
 }
 
 // Mass-type system of the current NS_stage: exact cell-wise inverse or CG + Jacobi to eps
@@ -288,8 +270,7 @@ static int pressure_fixed_point(af_imex* h, int stage, int iter) {
     return r;
   }
   Apply S = [o](const double* in, double* out) { return af_vmult(o, out, in); };
-  const double tol = h->opt.eps * l2norm(h, h->rhs_p, ns);
-  return gmres_solve(h, S, h->invd_D, h->pfix, h->rhs_p, ns, tol, nullptr);
+  return gmres_solve(h, S, h->invd_D, h->pfix, h->rhs_p, ns, h->opt.eps, nullptr);
 }
 
 static int update_velocity(af_imex* h, int stage) {
@@ -347,12 +328,10 @@ static int fixed_point(af_imex* h, int stage, double* p_out, double* u_out) {
     IM_AF(pressure_fixed_point(h, stage, iter));
     IM_AF(update_velocity(h, stage));
     ++iters;
-    IM_CU(maxabs2(h->pfix, h->pfix_old, ns, h->part, h->scal, o->stream));
-    double mm[2];
-    IM_CU(cudaMemcpyAsync(mm, h->scal, sizeof(mm), cudaMemcpyDeviceToHost, o->stream));
-    IM_AF(sync_checked(o, o->stream));
+    IM_CU(maxabs2(h->pfix, h->pfix_old, ns, h->part, h->kw.slot_dev(3), o->stream));
     o->launches += 2;
-    err = mm[1] / (mm[0] + 1e-10);
+    IM_AF(sync_checked(o, o->stream));
+    err = h->kw.slot(4) / (h->kw.slot(3) + 1e-10);
     if (err < h->opt.fixed_point_tol) break;
     IM_CU(cudaMemcpyAsync(h->pfix_old, h->pfix, ns * 8, cudaMemcpyDeviceToDevice, o->stream));
   }
@@ -866,9 +845,10 @@ int af_imex_create(const af_mesh_desc* mesh, int degree, double Ma, double Fr, d
   // scalar vectors: rho0 rho2 rho3 rhoc p0 p2 p3 pfix pfix_old rhs_rho rhs_p tmpp invd_M invd_D gw = 15
   // velocity vectors (2 ns): u0 u2 u3 uc ufix rhs_u tmp1 tmpu cg_r cg_z cg_p cg_Ap invd_u = 13
   r = AF_OK;
-  const long total = 15 * (ns + 1) + 13 * 2 * ns + (long)(m + 1) * krylov_stride(ns) + 2 * (m + 1) + 8 +
+  const long total = 15 * (ns + 1) + 13 * 2 * ns + (long)(m + 1) * krylov_stride(ns) + 8 +
                      4 * kMaxPartials + 16;
-  if (cudaMalloc(&h->mem, total * sizeof(double)) != cudaSuccess) {
+  if (krylov_create(&h->kw) != cudaSuccess || cudaMalloc(&h->mem, total * sizeof(double)) != cudaSuccess) {
+    krylov_destroy(&h->kw);
     af_destroy(h->op);
     delete h;
     return ierr(AF_CUDA, "af_imex_create: device allocation failed");
@@ -888,7 +868,6 @@ int af_imex_create(const af_mesh_desc* mesh, int degree, double Ma, double Fr, d
   h->cg_r = take(2 * ns); h->cg_z = take(2 * ns); h->cg_p = take(2 * ns); h->cg_Ap = take(2 * ns);
   h->invd_u = take(2 * ns);
   h->V = take((long)(m + 1) * krylov_stride(ns));
-  h->d_h = take(2 * (m + 1));
   h->scal = take(8);
   h->part = take(4 * kMaxPartials);
   h->kst = reinterpret_cast<KrylovState*>(take(16));
@@ -919,6 +898,7 @@ int af_imex_destroy(af_imex* h) {
   if (h->op) af_synchronize(h->op);
   af_schur_solver_destroy(h->schur);
   cudaFree(h->mem);
+  krylov_destroy(&h->kw);
   cudaFree(h->adj_mem);
   for (int k = 0; k < 2; ++k) {
     for (double* p : h->rec_p[k]) cudaFree(p);

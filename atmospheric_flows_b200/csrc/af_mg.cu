@@ -184,7 +184,9 @@ struct af_schur_solver {
   double* scal = nullptr;
   double* invd = nullptr;       // Jacobi: inverse diagonal of D
   // FGMRES workspace
-  double *V = nullptr, *Z = nullptr, *gw = nullptr, *dh = nullptr;
+  double *V = nullptr, *Z = nullptr, *gw = nullptr;
+  KrylovWork kw;
+  cudaEvent_t ev[2] = {nullptr, nullptr};  // device time of a solve
   std::vector<void*> owned;
   af_schur_stats stats{};
 };
@@ -590,7 +592,9 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
   // reductions and FGMRES workspace
   if ((r = alloc(s, (void**)&s->part, sizeof(double) * 4 * kMaxPartials)) != AF_OK) return cleanup(r);
   if ((r = alloc(s, (void**)&s->scal, sizeof(double) * 8)) != AF_OK) return cleanup(r);
-  if ((r = alloc(s, (void**)&s->dh, sizeof(double) * 2 * (o.restart + 1))) != AF_OK) return cleanup(r);
+  if (krylov_create(&s->kw) != cudaSuccess || cudaEventCreate(&s->ev[0]) != cudaSuccess ||
+      cudaEventCreate(&s->ev[1]) != cudaSuccess)
+    return cleanup(merr(AF_CUDA, "af_schur_solver_create: Krylov workspace"));
   const long ld0 = krylov_stride(ns0);
   if ((r = alloc(s, (void**)&s->V, sizeof(double) * ld0 * (o.restart + 1))) != AF_OK) return cleanup(r);
   if ((r = alloc(s, (void**)&s->Z, sizeof(double) * ld0 * o.restart)) != AF_OK) return cleanup(r);
@@ -663,6 +667,9 @@ int af_schur_solver_destroy(af_schur_solver* s) {
   cudaSetDevice(s->op->device);
   cudaStreamSynchronize(s->op->stream);
   for (void* p : s->owned) cudaFree(p);
+  krylov_destroy(&s->kw);
+  for (cudaEvent_t e : s->ev)
+    if (e) cudaEventDestroy(e);
   delete s;
   return AF_OK;
 }
@@ -717,38 +724,28 @@ int fgmres(af_schur_solver* s, const Apply& A, double* x, const double* b, doubl
   const long n = o->n_scalar();
   const long ld = krylov_stride(n);  // basis vectors start on 16-byte boundaries
   const int m = s->opt.restart;
-  cudaEvent_t e0, e1;
-  MG_CU(cudaEventCreate(&e0));
-  MG_CU(cudaEventCreate(&e1));
-  MG_CU(cudaEventRecord(e0, st));
-  std::vector<double> H((m + 1) * m), cs(m), sn(m), g(m + 1), hh(2 * (m + 1));
+  MG_CU(cudaEventRecord(s->ev[0], st));
+  std::vector<double> H((m + 1) * m), cs(m), sn(m), g(m + 1);
   auto Hs = [&](int i, int j) -> double& { return H[i * m + j]; };
-  auto read_scalar = [&](double* v) -> int {
-    MG_CU(cudaMemcpyAsync(v, s->scal, sizeof(double), cudaMemcpyDeviceToHost, st));
-    MG_AF(sync_checked(o, st));
-    return AF_OK;
-  };
-  double bb = 0.0;
-  MG_CU(dot(b, nullptr, n, s->part, s->scal, st));
-  MG_AF(read_scalar(&bb));
-  const double tol = rel_tol * std::sqrt(bb);
+  // |b|^2 arrives with the first residual's norm
+  MG_CU(norm2_host(s->kw, b, n, 2, st));
+  o->launches += 1;
+  double tol = -1.0;
   int total = 0;
   double res = 0.0, res0 = -1.0;
   bool converged = false;
   while (true) {
     MG_AF(A(s->gw, x));
-    MG_CU(sub(b, s->gw, s->gw, n, st));
-    MG_CU(dot(s->gw, nullptr, n, s->part, s->scal, st));
-    double beta2 = 0.0;
-    MG_AF(read_scalar(&beta2));
+    MG_CU(residual_start(s->kw, b, s->gw, nullptr, s->V, n, st));  // V_0 = r / |r|
     o->launches += 2;
-    const double beta = std::sqrt(beta2);
+    MG_AF(sync_checked(o, st));
+    if (tol < 0.0) tol = rel_tol * std::sqrt(s->kw.slot(2));
+    const double beta = std::sqrt(s->kw.slot(1));
     res = beta;
     if (res0 < 0.0) res0 = beta;
     if (!std::isfinite(beta)) return merr(AF_NAN, "Schur FGMRES: NaN residual");
     if (beta <= tol) { converged = true; break; }
     if (total >= max_iterations) break;
-    MG_CU(scale(1.0 / beta, s->gw, s->V, n, st));
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int jend = -1;
@@ -757,19 +754,12 @@ int fgmres(af_schur_solver* s, const Apply& A, double* x, const double* b, doubl
       double* w = s->V + (long)(j + 1) * ld;
       MG_AF(precondition(s, zj, s->V + (long)j * ld));
       MG_AF(A(w, zj));
-      MG_CU(mdot(s->V, ld, j + 1, w, n, s->part, s->dh, st));
-      MG_CU(maxpy(s->V, ld, j + 1, s->dh, w, n, st));
-      MG_CU(mdot(s->V, ld, j + 1, w, n, s->part, s->dh + (m + 1), st));
-      MG_CU(maxpy(s->V, ld, j + 1, s->dh + (m + 1), w, n, st));
-      MG_CU(dot(w, nullptr, n, s->part, s->scal, st));
-      MG_CU(cudaMemcpyAsync(hh.data(), s->dh, sizeof(double) * 2 * (m + 1), cudaMemcpyDeviceToHost, st));
-      double hn2 = 0.0;
-      MG_AF(read_scalar(&hn2));
-      o->launches += 5;
-      for (int i = 0; i <= j; ++i) Hs(i, j) = hh[i] + hh[(m + 1) + i];
-      const double hn = std::sqrt(hn2);
+      MG_CU(gram_schmidt(s->kw, s->V, ld, j + 1, w, nullptr, n, st));
+      o->launches += kGramSchmidtLaunches;
+      MG_AF(sync_checked(o, st));
+      for (int i = 0; i <= j; ++i) Hs(i, j) = s->kw.h(i);
+      const double hn = std::sqrt(s->kw.slot(0));
       Hs(j + 1, j) = hn;
-      if (hn > 0.0) MG_CU(scale(1.0 / hn, w, w, n, st));
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * Hs(i, j) + sn[i] * Hs(i + 1, j);
         Hs(i + 1, j) = -sn[i] * Hs(i, j) + cs[i] * Hs(i + 1, j);
@@ -799,12 +789,10 @@ int fgmres(af_schur_solver* s, const Apply& A, double* x, const double* b, doubl
     MG_CU(mcombine(s->Z, ld, kk, y.data(), x, n, st));
     o->launches += 1;
   }
-  MG_CU(cudaEventRecord(e1, st));
-  MG_CU(cudaEventSynchronize(e1));
+  MG_CU(cudaEventRecord(s->ev[1], st));
+  MG_CU(cudaEventSynchronize(s->ev[1]));
   float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  cudaEventElapsedTime(&ms, s->ev[0], s->ev[1]);
   s->stats.iterations = total;
   s->stats.initial_residual = res0;
   s->stats.final_residual = res;

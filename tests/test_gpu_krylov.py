@@ -1,0 +1,56 @@
+"""The Krylov basis kernels at the edges of their chunks (1024 elements), basis counts (batches of
+four vectors, up to 64) and vectors of odd length: FGMRES with Jacobi solves to a true relative
+residual of 1e-10, which the operator's own apply confirms to 2e-10 (the Arnoldi estimate stops the
+last cycle and the true residual is checked before returning), for every restart length the same
+solution to 1e-8 (residual 1e-10 times a condition of about 1e2 for these coefficients).  A
+right-hand side that starts off a 16-byte boundary is accepted as before."""
+import numpy as np
+import pytest
+
+from atmospheric_flows_b200 import mesh as M
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("nx,nz,P", [(3, 3, 4), (16, 4, 3), (41, 1, 4), (64, 16, 1), (63, 13, 2), (40, 26, 4)])
+def test_solves_for_every_restart(nx, nz, P):
+    from atmospheric_flows_b200.operator import EULEROperator
+    from atmospheric_flows_b200.schur import SchurSolver
+    sc = M.Scaling()
+    m = M.hill_mesh(nx, nz, periodic_x=True)
+    st = M.hill_state(m, P, modes=4)
+    op = EULEROperator(m, P, sc.Ma, sc.Fr, 0.25)
+    op.set_stream(torch.cuda.current_stream())
+    op.set_schur_mode(1)
+    op.set_HYPERBOLIC_stage(1)
+    op.set_rho_for_fixed(torch.from_numpy(st.rho).cuda())
+    op.set_pres_fixed(torch.from_numpy(st.p).cuda())
+    n = op.n_dofs(1)
+    buf = torch.empty(n + 1, dtype=torch.float64, device="cuda")
+    b = torch.from_numpy(np.random.default_rng(7).standard_normal(n)).cuda()
+    buf[1:] = b
+    xs = []
+    for restart in (1, 2, 3, 5, 8, 30, 63, 64):
+        s = SchurSolver(op, "jacobi", restart=restart)
+        s.setup()
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        if restart == 1:  # restarted after every direction: progress, no convergence asked
+            s.solve(x, b, rel_tol=1e-10, max_iterations=3, raise_on_failure=False)
+            assert torch.isfinite(x).all()
+            continue
+        q = s.solve(x, buf[1:] if restart == 30 else b, rel_tol=1e-10, max_iterations=20000, raise_on_failure=restart > 5)
+        if restart <= 5 and q["status"] != 0:
+            continue
+        r = torch.empty_like(x)
+        op.set_NS_stage(2)
+        op.vmult(r, x)
+        assert rel(r, b) < 2e-10
+        xs.append(x)
+    assert len(xs) >= 4
+    for x in xs:
+        assert rel(x, xs[-1]) < 1e-8
