@@ -1503,24 +1503,31 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
   }
 }
 
-template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>(), int MINB = Layout<P, Phys, CB_>::CTAS>
-cudaError_t launch_cellop(const MeshDev& mesh,
-                          const ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>>& ptr,
-                          const typename Phys::Params& prm, int ncell, cudaStream_t stream) {
-  using L = Layout<P, Phys, CB_>;
-  // The shared-memory attribute belongs to the function on the current device: one bit per
-  // device (devices 0..63; beyond that it is set on every launch), set by whichever thread gets
-  // there first (setting it twice is harmless).
-  static std::atomic<unsigned long long> configured{0};
+// Allows a kernel `bytes` of dynamic shared memory on the current device.  The attribute belongs to the
+// function on that device: one bit per device (devices 0..63; beyond that it is set on every launch),
+// set by whichever thread gets there first (setting it twice is harmless).
+template <class K>
+cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<unsigned long long>& configured) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
   if (bit == 0 || (configured.load(std::memory_order_acquire) & bit) == 0) {
-    e = cudaFuncSetAttribute(k_cellop<P, Phys, CB_, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit, std::memory_order_release);
   }
+  return cudaSuccess;
+}
+
+template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>(), int MINB = Layout<P, Phys, CB_>::CTAS>
+cudaError_t launch_cellop(const MeshDev& mesh,
+                          const ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>>& ptr,
+                          const typename Phys::Params& prm, int ncell, cudaStream_t stream) {
+  using L = Layout<P, Phys, CB_>;
+  static std::atomic<unsigned long long> configured{0};
+  const cudaError_t e = allow_smem(k_cellop<P, Phys, CB_, MINB>, L::BYTES, configured);
+  if (e != cudaSuccess) return e;
   if (mesh.cell0 < 0) return cudaErrorInvalidValue;
   if (ncell <= mesh.cell0) return cudaSuccess;
   const int nblk = (ncell - mesh.cell0 + L::CB - 1) / L::CB;

@@ -55,6 +55,19 @@ constexpr int P = AF_P;
 // threads per cell, about half of the full-quadrature kernel's
 constexpr int kReducedCB = P == 1 ? 64 : (P == 2 ? 42 : (P <= 4 ? 32 : (P == 5 ? 20 : 18)));
 
+constexpr int kND = (P + 1) * (P + 1);
+constexpr int kNPK = kND * (kND + 1) / 2;
+constexpr int kNQ = 2 * P + 1, kNPair = (P + 1) * (P + 2) / 2;
+constexpr int kInvRows = (kND + 1) / 2;         // threads per cell, two rows each
+constexpr int kInvCells = 128 / kInvRows;
+constexpr int kInvThreads = 128;
+// products of basis values: [pair i <= j, pair = j (j+1)/2 + i][point]
+struct PairTab {
+  double ss[kNPair][kNQ];
+};
+static __constant__ PairTab c_pair;
+__host__ __device__ constexpr int pair_of(int i, int j) { return i <= j ? j * (j + 1) / 2 + i : i * (i + 1) / 2 + j; }
+
 cudaError_t upload_tables() {
   static const Tab<P> t = host::make_tab<P>();
   static const TabT<P, float> tf = host::make_tab<P, float>();
@@ -64,7 +77,18 @@ cudaError_t upload_tables() {
   static const TransT<P, float> trf = host::make_trans<P, float>();
   static const CobT<P, double> cob = host::make_cob<P, double>();
   static const CobT<P, float> cobf = host::make_cob<P, float>();
+  static const PairTab pt = [] {
+    PairTab p{};
+    std::vector<host::LD> nd = host::gll(P), x, w;
+    host::gauss(kNQ, x, w);
+    for (int j = 0; j <= P; ++j)
+      for (int i = 0; i <= j; ++i)
+        for (int q = 0; q < kNQ; ++q)
+          p.ss[pair_of(i, j)][q] = (double)(host::lag(nd, i, x[q]) * host::lag(nd, j, x[q]));
+    return p;
+  }();
   cudaError_t e = cudaMemcpyToSymbol(c_tab, &t, sizeof(t));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_pair, &pt, sizeof(pt));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_cob, &cob, sizeof(cob));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_cobf, &cobf, sizeof(cobf));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_tabf, &tf, sizeof(tf));
@@ -240,126 +264,205 @@ cudaError_t inv_diag(const MeshDev& mesh, int ncomp, const double* weight, doubl
 }
 
 // ---------------------------------------------------------------- exact cell inverse
-// Cell mass matrix  M_K[I][J] = sum_q w(q) JxW(q) phi_I(q) phi_J(q)  (w = 1 or a density),
-// its Cholesky factor and its inverse, one warp per cell:
-//   F(q) = w(q) JxW(q) at the Gauss points (lanes over points);
-//   T(qz)[ix][jx] = sum_qx S[qx][ix] S[qx][jx] F(qz, qx),
-//   M[I][J] = sum_qz S[qz][iz] S[qz][jz] T(qz)[ix][jx]   (lanes over entries, packed lower);
-//   Cholesky M = L L^T in place (lanes over rows, one column at a time);
-//   X = L^{-1}: lane j solves L x = e_j for its column in registers;  M^{-1} = X^T X.
-// The packed lower triangle of the inverse (row-major) is stored cell-major,
-// Minv[c * NPK + k], so that one warp of the apply kernel reads a cell's inverse as one
-// contiguous block.
-constexpr int kND = (P + 1) * (P + 1);
-constexpr int kNPK = kND * (kND + 1) / 2;
-constexpr int kFactorWarps = P <= 4 ? 4 : (P == 5 ? 2 : 1);  // static shared memory <= 48 KB
+// Cell mass matrix  M_K[I][J] = sum_q w(q) JxW(q) phi_I(q) phi_J(q)  (w = 1 or a density) and its
+// inverse, stored as the packed lower triangle (row-major) cell-major, Minv[c * NPK + k], so that the
+// apply kernel reads a cell's inverse as one contiguous block.
+//
+// One CTA forms kInvCells cells, one thread per two rows of a cell (117 of 128 threads at degree 4, 125
+// at degree 6):
+//   F(q) = w(q) JxW(q) at the Gauss points, w by sum factorisation;
+//   T(qz)[ix <= jx] = sum_qx S[qx][ix] S[qx][jx] F(qz, qx),  thread = (cell, qz);
+//   Q[iz <= jz][ix <= jx] = sum_qz S[qz][iz] S[qz][jz] T(qz)[ix][jx],  thread = (cell, ix <= jx)
+// (the products S S from constant memory: each value is loaded once per thread and multiplied by
+// compile-time constants), which holds every entry of the matrix once: M[(iz, ix)][(jz, jx)] =
+// Q[iz, jz][ix, jx].  The inverse by the symmetric sweep operator (M is symmetric positive definite,
+// no pivoting): sweeping pivot k maps a_kk -> -1/a_kk, a_rk = a_kr -> a_rk/a_kk and, for r, j != k,
+// a_rj -> a_rj - (a_rk/a_kk) a_kj; sweeping every pivot leaves -M^{-1}.  A thread keeps two rows
+// in registers, rotated so that the pivot column comes first: every pivot runs the same code (a loop,
+// not ND unrolled copies) and writes a[j] from a[j+1].  The pivot row is the column of the threads'
+// first elements, published in shared memory (twice in a row, so that the rotated row is contiguous),
+// one barrier per pivot.
+//
+// Bound by the broadcast loads of the pivot row and FP64 issue (ND^3 multiply-adds a cell); two rows
+// per thread share a load (one row per thread: degree 4 720 us with the shared-memory data path at
+// 96 %, degree 6 980 us), and the loads are of 8 bytes: a 16-byte load of a warp takes four wavefronts
+// even when its lanes read two addresses (degree 6 845 us with them).  Measured: degree 4, 131072 cells 610 us (one warp per cell with lane = row, two exchanges per
+// pivot and all pivots unrolled: 889 us); degree 6, 32385 cells 823 us (Cholesky of the packed matrix in
+// shared memory, one warp per cell: 5085 us).
+struct InvShape {  // shared memory of one cell, in doubles
+  static constexpr int F = 0, T = F + kNQ * kNQ, Q = T + kNQ * kNPair, W = Q + kNPair * kNPair, X = W + kND,
+                       END = X + (P + 1) * kNQ;
+  static constexpr int BASE = END > kNPK ? END : kNPK;  // the packed inverse takes their place
+  static constexpr int RL = 2 * kND;                    // the pivot row, twice
+  static constexpr int R = BASE, ID = R + 2 * RL, GEO = ID + 2;
+  static constexpr int CELL = (GEO + 6) | 1;  // odd: the loads of two cells in a warp meet different banks
+  static constexpr size_t BYTES = sizeof(double) * CELL * kInvCells;
+};
 
-__global__ void __launch_bounds__(32 * kFactorWarps)
-    k_mass_factor(const MeshDev mesh, const double* __restrict__ weight, double* __restrict__ Lg, const int ncell) {
-  using T = Tab<P>;
-  constexpr int P1 = T::P1, NQ = T::NQ, ND = kND, NPK = kNPK;
-  constexpr int NT = NQ * P1 * (P1 + 1) / 2;  // T(qz)[ix >= jx]
-  __shared__ double sA[kFactorWarps][NPK];
-  __shared__ double sX[kFactorWarps][NPK];
-  __shared__ double sF[kFactorWarps][NQ * NQ];
-  __shared__ double sT[kFactorWarps][NT];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * kFactorWarps + warp;
-  if (c >= ncell) return;  // whole warps; no block-wide barrier below
+__global__ void __launch_bounds__(kInvThreads, P <= 4 ? 4 : 2)
+    k_mass_inverse(const MeshDev mesh, const double* __restrict__ weight, double* __restrict__ Lg, const int ncell) {
+  using S = InvShape;
+  constexpr int P1 = P + 1, NQ = kNQ, ND = kND, NT = kInvThreads, NC = kInvCells;
+  extern __shared__ __align__(16) double sm[];
   const Tab<P>& tb = c_tab;
-  double* A = sA[warp];
-  double* X = sX[warp];
-  double* F = sF[warp];
-  double* Tm = sT[warp];
-  const int i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
-  const double2 v0 = mesh.vtx[j * W + i], v1 = mesh.vtx[j * W + i + 1];
-  const double2 v2 = mesh.vtx[(j + 1) * W + i], v3 = mesh.vtx[(j + 1) * W + i + 1];
-  const double Ax = v1.x - v0.x, Az = v1.y - v0.y, Cx = v2.x - v0.x, Cz = v2.y - v0.y;
-  const double Bx = v3.x - v2.x - v1.x + v0.x, Bz = v3.y - v2.y - v1.y + v0.y;
-  // F(q) = w(q) JxW(q)
-  for (int q = lane; q < NQ * NQ; q += 32) {
-    const int qx = q % NQ, qz = q / NQ;
-    const double xi = tb.x[qx], eta = tb.x[qz];
-    const double J00 = fma(Bx, eta, Ax), J10 = fma(Bz, eta, Az), J01 = fma(Bx, xi, Cx), J11 = fma(Bz, xi, Cz);
-    double f = (J00 * J11 - J01 * J10) * tb.w[qx] * tb.w[qz];
-    if (weight) {
-      const double* wc = weight + (size_t)c * ND;
-      double wv = 0.0;
+  const int t = threadIdx.x, c0 = blockIdx.x * NC, nc = min(NC, ncell - c0);
+  // nodal weights and the bilinear maps
+  if (weight)
+    for (int e = t; e < nc * ND; e += NT) sm[(e / ND) * S::CELL + S::W + e % ND] = weight[(size_t)c0 * ND + e];
+  if (t < nc) {
+    const int c = c0 + t, i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
+    const double2* v = mesh.vtx + (size_t)j * W + i;
+    const double2 v0 = v[0], v1 = v[1], v2 = v[W], v3 = v[W + 1];
+    double* g = sm + t * S::CELL + S::GEO;
+    g[0] = v1.x - v0.x; g[1] = v1.y - v0.y;
+    g[2] = v2.x - v0.x; g[3] = v2.y - v0.y;
+    g[4] = v3.x - v2.x - v1.x + v0.x; g[5] = v3.y - v2.y - v1.y + v0.y;
+  }
+  __syncthreads();
+  if (weight) {  // rows of the weight at the x points: thread = (cell, row)
+    for (int e = t; e < nc * P1; e += NT) {
+      double* s = sm + (e / P1) * S::CELL;
+      const int iz = e % P1;
+      double r[P1];
 #pragma unroll
-      for (int iz = 0; iz < P1; ++iz) {
-        double t = 0.0;
+      for (int i = 0; i < P1; ++i) r[i] = s[S::W + iz * P1 + i];
 #pragma unroll
-        for (int ix = 0; ix < P1; ++ix) t = fma(tb.S[qx][ix], wc[iz * P1 + ix], t);
-        wv = fma(tb.S[qz][iz], t, wv);
+      for (int q = 0; q < NQ; ++q) {
+        double a = 0.0;
+#pragma unroll
+        for (int i = 0; i < P1; ++i) a = fma(tb.S[q][i], r[i], a);
+        s[S::X + iz * NQ + q] = a;
       }
-      f *= wv;
     }
-    F[q] = f;
+    __syncthreads();
   }
-  __syncwarp();
-  // T(qz)[ix][jx], ix >= jx
-  for (int e = lane; e < NT; e += 32) {
-    const int qz = e / (P1 * (P1 + 1) / 2);
-    int r = e % (P1 * (P1 + 1) / 2), ix = 0;
-    while (r > ix) { r -= ix + 1; ++ix; }
-    const int jx = r;
-    double s = 0.0;
+  for (int e = t; e < nc * NQ; e += NT) {  // F: thread = (cell, column qx)
+    double* s = sm + (e / NQ) * S::CELL;
+    const double* g = s + S::GEO;
+    const int qx = e % NQ;
+    const double xi = tb.x[qx], wx = tb.w[qx], J01 = fma(g[4], xi, g[2]), J11 = fma(g[5], xi, g[3]);
+    double r[P1];
+    if (weight)
 #pragma unroll
-    for (int qx = 0; qx < NQ; ++qx) s = fma(tb.S[qx][ix] * tb.S[qx][jx], F[qz * NQ + qx], s);
-    Tm[e] = s;
-  }
-  __syncwarp();
-  // M[I][J], I >= J (packed row-major)
-  for (int e = lane; e < NPK; e += 32) {
-    int I = 0, r = e;
-    while (r > I) { r -= I + 1; ++I; }
-    const int J = r;
-    const int iz = I / P1, ix = I % P1, jz = J / P1, jx = J % P1;
-    const int a = ix >= jx ? ix : jx, b = ix >= jx ? jx : ix;
-    const int tix = a * (a + 1) / 2 + b;
-    double s = 0.0;
+      for (int i = 0; i < P1; ++i) r[i] = s[S::X + i * NQ + qx];
 #pragma unroll
-    for (int qz = 0; qz < NQ; ++qz)
-      s = fma(tb.S[qz][iz] * tb.S[qz][jz], Tm[qz * (P1 * (P1 + 1) / 2) + tix], s);
-    A[e] = s;
+    for (int q = 0; q < NQ; ++q) {
+      const double J00 = fma(g[4], tb.x[q], g[0]), J10 = fma(g[5], tb.x[q], g[1]);
+      double f = (J00 * J11 - J01 * J10) * wx * tb.w[q];
+      if (weight) {
+        double a = 0.0;
+#pragma unroll
+        for (int i = 0; i < P1; ++i) a = fma(tb.S[q][i], r[i], a);
+        f *= a;
+      }
+      s[S::F + q * NQ + qx] = f;
+    }
   }
-  __syncwarp();
-  // Cholesky, one column at a time: L_kk = sqrt(A_kk); L_ik = A_ik / L_kk; A_ij -= L_ik L_jk
+  __syncthreads();
+  for (int e = t; e < nc * NQ; e += NT) {  // T: thread = (cell, qz)
+    double* s = sm + (e / NQ) * S::CELL;
+    const int qz = e % NQ;
+    double f[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) f[q] = s[S::F + qz * NQ + q];
+#pragma unroll
+    for (int p = 0; p < kNPair; ++p) {
+      double a = 0.0;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) a = fma(c_pair.ss[p][q], f[q], a);
+      s[S::T + qz * kNPair + p] = a;
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < nc * kNPair; e += NT) {  // Q: thread = (cell, ix <= jx)
+    double* s = sm + (e / kNPair) * S::CELL;
+    const int px = e % kNPair;
+    double f[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) f[q] = s[S::T + q * kNPair + px];
+#pragma unroll
+    for (int p = 0; p < kNPair; ++p) {
+      double a = 0.0;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) a = fma(c_pair.ss[p][q], f[q], a);
+      s[S::Q + p * kNPair + px] = a;
+    }
+  }
+  __syncthreads();
+  // rows 2i, 2i + 1 of cell cc (a row past the last repeats it and publishes nothing; so do threads
+  // past the last cell)
+  const int cc = min(t / kInvRows, nc - 1), i2 = 2 * (t % kInvRows);
+  const bool own = t / kInvRows < nc;
+  double* s = sm + cc * S::CELL;
+  double a[2][ND];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = min(i2 + h, ND - 1), rz = r / P1, rx = r % P1;
+#pragma unroll
+    for (int j = 0; j < ND; ++j) {
+      const int jz = j / P1, jx = j % P1;
+      const int pz = rz <= jz ? jz * (jz + 1) / 2 + rz : rz * (rz + 1) / 2 + jz;
+      const int px = rx <= jx ? jx * (jx + 1) / 2 + rx : rx * (rx + 1) / 2 + jx;
+      a[h][j] = s[S::Q + pz * kNPair + px];
+    }
+  }
+  const bool own1 = own && i2 + 1 < ND;
+#pragma unroll 1
   for (int k = 0; k < ND; ++k) {
-    const double lkk = sqrt(A[k * (k + 1) / 2 + k]);
-    const double inv = 1.0 / lkk;
-    for (int r = k + 1 + lane; r < ND; r += 32) A[r * (r + 1) / 2 + k] *= inv;
-    __syncwarp();
-    if (lane == 0) A[k * (k + 1) / 2 + k] = lkk;
-    for (int r = k + 1 + lane; r < ND; r += 32) {
-      const double lrk = A[r * (r + 1) / 2 + k];
-      for (int q = k + 1; q <= r; ++q) A[r * (r + 1) / 2 + q] -= lrk * A[q * (q + 1) / 2 + k];
+    // buffers alternate: the reads of pivot k-1 need no barrier before these writes, and those of
+    // pivot k-2 lie behind the last one
+    double* W = s + S::R + (k & 1) * S::RL;
+    if (own) {
+      W[i2] = a[0][0];
+      W[i2 + ND] = a[0][0];
     }
-    __syncwarp();
-  }
-  // X = L^{-1}: lane jc solves L x = e_jc (x_i = 0 for i < jc) in registers and stores the
-  // column into the packed lower X; then M^{-1}[I][J] = sum_{k >= I} X[k][I] X[k][J]
-  for (int jc = lane; jc < ND; jc += 32) {
-    double x[ND];
-#pragma unroll
-    for (int ii = 0; ii < ND; ++ii) {
-      double s = (ii == jc) ? 1.0 : 0.0;
-#pragma unroll
-      for (int kk = 0; kk < ii; ++kk) s = fma(-A[ii * (ii + 1) / 2 + kk], x[kk], s);
-      x[ii] = ii >= jc ? s / A[ii * (ii + 1) / 2 + ii] : 0.0;
-      if (ii >= jc) X[ii * (ii + 1) / 2 + jc] = x[ii];
+    if (own1) {
+      W[i2 + 1] = a[1][0];
+      W[i2 + 1 + ND] = a[1][0];
     }
+    if (own && (k & ~1) == i2) s[S::ID + (k & 1)] = 1.0 / ((k & 1) ? a[1][0] : a[0][0]);
+    __syncthreads();
+    const double id = s[S::ID + (k & 1)];
+    double g0 = a[0][0] * id, g1 = a[1][0] * id, m0 = -g0, m1 = -g1;
+    if (i2 == k) {
+      m0 = id;
+      g0 = -id;
+#pragma unroll
+      for (int j = 1; j < ND; ++j) a[0][j] = 0.0;
+    } else if (i2 + 1 == k) {
+      m1 = id;
+      g1 = -id;
+#pragma unroll
+      for (int j = 1; j < ND; ++j) a[1][j] = 0.0;
+    }
+    const double* v = W + k + 1;
+#pragma unroll
+    for (int j = 0; j + 1 < ND; ++j) {
+      a[0][j] = fma(m0, v[j], a[0][j + 1]);
+      a[1][j] = fma(m1, v[j], a[1][j + 1]);
+    }
+    a[0][ND - 1] = g0;
+    a[1][ND - 1] = g1;
   }
-  __syncwarp();
-  double* out = Lg + (size_t)c * NPK;
-  for (int e = lane; e < NPK; e += 32) {
-    int I = 0, r = e;
-    while (r > I) { r -= I + 1; ++I; }
-    const int J = r;
-    double s = 0.0;
-    for (int k = I; k < ND; ++k) s = fma(X[k * (k + 1) / 2 + I], X[k * (k + 1) / 2 + J], s);
-    out[e] = s;
+  __syncthreads();  // the forming arrays are long consumed; the packed inverse takes their place
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = i2 + h;
+    if (h == 0 ? own : own1)
+#pragma unroll
+      for (int j = 0; j < ND; ++j)
+        if (j <= r) s[r * (r + 1) / 2 + j] = -a[h][j];
   }
+  __syncthreads();
+  for (int e = t; e < nc * kNPK; e += NT) Lg[(size_t)c0 * kNPK + e] = sm[(e / kNPK) * S::CELL + e % kNPK];
+}
+
+cudaError_t mass_factor(const MeshDev& mesh, const double* weight, double* L, int ncell, cudaStream_t st) {
+  static std::atomic<unsigned long long> configured{0};
+  const cudaError_t e = allow_smem(k_mass_inverse, InvShape::BYTES, configured);
+  if (e != cudaSuccess) return e;
+  k_mass_inverse<<<(ncell + kInvCells - 1) / kInvCells, kInvThreads, InvShape::BYTES, st>>>(mesh, weight, L, ncell);
+  return cudaGetLastError();
 }
 
 // x = scale * M_K^{-1} b per cell and component: one warp per cell stages the cell's packed
@@ -448,150 +551,6 @@ cudaError_t launch_mass_solve(const R* L, int ncomp, const R* b, R scale, R* x, 
   if (ncomp < 1 || ncomp > 2) return cudaErrorInvalidValue;
   k_mass_solve<R, MODE><<<(ncell + kSolveWarps - 1) / kSolveWarps, 32 * kSolveWarps, 0, st>>>(L, b, x, d, scale, alpha,
                                                                                              first, ncomp, ncell, status);
-  return cudaGetLastError();
-}
-
-// Degrees <= 4 ((P+1)^2 <= 32 rows): the same cell matrix and its inverse with lane i owning
-// row i in registers, which removes the shared-memory traffic and index decoding of the
-// kernel above (instruction-bound: about 11.5 k warp instructions per cell at p = 4):
-//   rows: M[i][j] = sum_qz S[qz][iz] S[qz][jz] T(qz)[ix][jx], T as above (full, not packed),
-//   as sum_qz S[qz][jz] U[qz][jx] with U[qz][jx] = S[qz][iz] T(qz)[ix][jx] formed first;
-//   the inverse by the symmetric sweep operator (M is symmetric positive definite, no
-//   pivoting): sweeping pivot k maps a_kk -> -1/a_kk, a_rk = a_kr -> a_rk/a_kk and, for
-//   r, j != k, a_rj -> a_rj - (a_rk/a_kk) a_kj; it keeps the matrix symmetric, and sweeping
-//   every pivot leaves -M^{-1}.  By symmetry the pivot row is the column k of the lanes'
-//   registers: each lane stores its a_rk (one shared-memory store for the warp) and reads
-//   the row back as broadcasts, every row but k updates itself, and row k takes the new
-//   column k (the a_rk/a_kk of the other lanes) through shared memory.  (Gauss-Jordan with
-//   the pivot lane scaling its row alone, 24 multiplies with one lane active per pivot, and
-//   the row broadcast by warp shuffles took 1.19 ms per launch at 131072 cells; with the row
-//   broadcast through shared memory 1.0 ms.)  The lower triangle is staged in shared memory
-//   and stored coalesced.
-constexpr int kGJWarps = 4;
-template <int ND_ = kND>
-__global__ void __launch_bounds__(32 * kGJWarps)
-    k_mass_inverse_rows(const MeshDev mesh, const double* __restrict__ weight, double* __restrict__ Lg,
-                        const int ncell) {
-  static_assert(ND_ <= 32, "one row per lane");
-  using T = Tab<P>;
-  constexpr int P1 = T::P1, NQ = T::NQ, ND = ND_, NPK = ND * (ND + 1) / 2;
-  __shared__ double sS[NQ * P1];
-  __shared__ double sF[kGJWarps][NQ * NQ];
-  __shared__ double sT[kGJWarps][NQ * P1 * P1];
-  __shared__ double sO[kGJWarps][NPK];
-  constexpr int NDE = (ND + 1) / 2 * 2;  // a row padded to whole double2
-  // per warp: the pivot row (column k) and the new column k, one slot per lane
-  __shared__ __align__(16) double sR[kGJWarps][32];
-  __shared__ __align__(16) double sG[kGJWarps][32];
-  const Tab<P>& tb = c_tab;
-  for (int k = threadIdx.x; k < NQ * P1; k += blockDim.x) sS[k] = tb.S[k / P1][k % P1];
-  __syncthreads();  // the only block-wide barrier; warps past the last cell leave after it
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * kGJWarps + warp;
-  if (c >= ncell) return;
-  double* F = sF[warp];
-  double* Tm = sT[warp];
-  double* O = sO[warp];
-  const int i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
-  const double2 v0 = mesh.vtx[j * W + i], v1 = mesh.vtx[j * W + i + 1];
-  const double2 v2 = mesh.vtx[(j + 1) * W + i], v3 = mesh.vtx[(j + 1) * W + i + 1];
-  const double Ax = v1.x - v0.x, Az = v1.y - v0.y, Cx = v2.x - v0.x, Cz = v2.y - v0.y;
-  const double Bx = v3.x - v2.x - v1.x + v0.x, Bz = v3.y - v2.y - v1.y + v0.y;
-  // F(q) = w(q) JxW(q)
-  for (int q = lane; q < NQ * NQ; q += 32) {
-    const int qx = q % NQ, qz = q / NQ;
-    const double xi = tb.x[qx], eta = tb.x[qz];
-    const double J00 = fma(Bx, eta, Ax), J10 = fma(Bz, eta, Az), J01 = fma(Bx, xi, Cx), J11 = fma(Bz, xi, Cz);
-    double f = (J00 * J11 - J01 * J10) * tb.w[qx] * tb.w[qz];
-    if (weight) {
-      const double* wc = weight + (size_t)c * ND;
-      double wv = 0.0;
-#pragma unroll
-      for (int iz = 0; iz < P1; ++iz) {
-        double t = 0.0;
-#pragma unroll
-        for (int ix = 0; ix < P1; ++ix) t = fma(sS[qx * P1 + ix], wc[iz * P1 + ix], t);
-        wv = fma(sS[qz * P1 + iz], t, wv);
-      }
-      f *= wv;
-    }
-    F[q] = f;
-  }
-  __syncwarp();
-  // T(qz)[ix][jx]
-  for (int e = lane; e < NQ * P1 * P1; e += 32) {
-    const int qz = e / (P1 * P1), ix = (e / P1) % P1, jx = e % P1;
-    double s = 0.0;
-#pragma unroll
-    for (int qx = 0; qx < NQ; ++qx) s = fma(sS[qx * P1 + ix] * sS[qx * P1 + jx], F[qz * NQ + qx], s);
-    Tm[e] = s;
-  }
-  __syncwarp();
-  // row r = lane of the cell matrix (lanes >= ND duplicate the last row and store nothing)
-  const int r = lane < ND ? lane : ND - 1, rz = r / P1, rx = r % P1;
-  // U[qz][jx] = S[qz][rz] T(qz)[rx][jx], then a[jz P1 + jx] = sum_qz S[qz][jz] U[qz][jx]
-  // (qz outermost: one U row live at a time)
-  double a[NDE];
-#pragma unroll
-  for (int jj = 0; jj < NDE; ++jj) a[jj] = 0.0;
-#pragma unroll
-  for (int qz = 0; qz < NQ; ++qz) {
-    const double sz = sS[qz * P1 + rz];
-    double u[P1];
-#pragma unroll
-    for (int jx = 0; jx < P1; ++jx) u[jx] = sz * Tm[qz * P1 * P1 + rx * P1 + jx];
-#pragma unroll
-    for (int jj = 0; jj < ND; ++jj) a[jj] = fma(tb.S[qz][jj / P1], u[jj % P1], a[jj]);
-  }
-  // sweep every pivot; rows r = lane (lanes >= ND repeat the last row and are not stored)
-#pragma unroll
-  for (int k = 0; k < ND; ++k) {
-    // (the previous pivot's barriers order its reads of R and G before these writes)
-    double* R = sR[warp];
-    double* G = sG[warp];
-    R[lane] = a[k];  // a_rk = a_kr: the pivot row, one element per lane
-    __syncwarp();
-    const double id = 1.0 / R[k];
-    const double g = a[k] * id;  // the new a_rk
-    if (lane != k) {
-#pragma unroll
-      for (int jj = 0; jj < NDE / 2; ++jj) {
-        const double2 v = reinterpret_cast<const double2*>(R)[jj];
-        if (2 * jj != k) a[2 * jj] = fma(-g, v.x, a[2 * jj]);
-        if (2 * jj + 1 != k && 2 * jj + 1 < ND) a[2 * jj + 1] = fma(-g, v.y, a[2 * jj + 1]);
-      }
-      a[k] = g;
-    }
-    G[lane] = g;
-    __syncwarp();
-    if (lane == k) {  // row k = the new column k
-#pragma unroll
-      for (int jj = 0; jj < NDE / 2; ++jj) {
-        const double2 v = reinterpret_cast<const double2*>(G)[jj];
-        a[2 * jj] = v.x;
-        a[2 * jj + 1] = v.y;
-      }
-      a[k] = -id;
-      if (NDE > ND) a[NDE - 1] = 0.0;
-    }
-  }
-#pragma unroll
-  for (int jj = 0; jj < ND; ++jj) a[jj] = -a[jj];  // the sweeps leave -M^{-1}
-  // lower triangle of row r, packed row-major, then coalesced
-#pragma unroll
-  for (int jj = 0; jj < ND; ++jj)
-    if (lane < ND && jj <= lane) O[lane * (lane + 1) / 2 + jj] = a[jj];
-  __syncwarp();
-  double* out = Lg + (size_t)c * NPK;
-  for (int e = lane; e < NPK; e += 32) out[e] = O[e];
-}
-
-cudaError_t mass_factor(const MeshDev& mesh, const double* weight, double* L, int ncell, cudaStream_t st) {
-  if constexpr (kND <= 32) {
-    k_mass_inverse_rows<<<(ncell + kGJWarps - 1) / kGJWarps, 32 * kGJWarps, 0, st>>>(mesh, weight, L, ncell);
-  } else {
-    k_mass_factor<<<(ncell + kFactorWarps - 1) / kFactorWarps, 32 * kFactorWarps, 0, st>>>(mesh, weight, L, ncell);
-  }
   return cudaGetLastError();
 }
 
