@@ -281,10 +281,9 @@ namespace af {
 // launches, four reads of the basis with 8-byte loads, and two pageable copies per iteration; the FP64
 // IMEX step at 256x128 (456 iterations) 95.0 -> 74.2 ms, the small 40x16 step 1.17 -> 0.84 ms.
 constexpr int KT = 256, KC = 4 * KT;  // threads per block, elements per chunk
-constexpr int KB = 3 * 148;           // blocks at most
 constexpr int KJ = 4;                 // basis vectors loaded together (6, 8: 5 % faster at k = 28, 10-20 % slower at k = 4)
 
-int krylov_blocks(long n) { return (int)std::min<long>((n + KC - 1) / KC, KB); }
+int krylov_blocks(long n) { return (int)std::min<long>((n + KC - 1) / KC, kKrylovBlocks); }
 
 struct KrylovDev {
   double* part;
@@ -293,15 +292,8 @@ struct KrylovDev {
   double* host;
 };
 KrylovDev krylov_dev(const KrylovWork& k) {
-  double* h1 = k.dev + (size_t)KB * kKrylovMax;
-  return {k.dev, h1, h1 + kKrylovMax, h1 + 2 * kKrylovMax, k.count, k.host_dev};
-}
-
-void krylov_destroy(KrylovWork* k) {
-  cudaFree(k->dev);
-  cudaFree(k->count);
-  if (k->host) cudaFreeHost(k->host);
-  *k = KrylovWork{};
+  double* h1 = k.dev + (size_t)kKrylovBlocks * kKrylovMax;
+  return {k.dev, h1, h1 + kKrylovMax, h1 + 2 * kKrylovMax, reinterpret_cast<unsigned*>(h1 + 2 * kKrylovMax + 2), k.host_dev};
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -546,21 +538,6 @@ cudaError_t normalise(const double* x, double* y, long n, const double* n2, cuda
 }
 }  // namespace
 
-cudaError_t krylov_create(KrylovWork* k) {
-  const size_t nd = (size_t)KB * kKrylovMax + 2 * kKrylovMax + 2;
-  cudaError_t e = cudaMalloc(&k->dev, nd * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&k->count, sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMemset(k->count, 0, sizeof(unsigned));
-  if (e == cudaSuccess)
-    e = cudaHostAlloc((void**)&k->host, (kKrylovMax + KrylovWork::kHostSlots) * sizeof(double),
-                      cudaHostAllocMapped | cudaHostAllocPortable);
-  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&k->host_dev, k->host, 0);
-  const int smem = (int)(sizeof(double) * kKrylovMax * KT);  // of the current device
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gram_schmidt<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gram_schmidt<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) krylov_destroy(k);
-  return e;
-}
 cudaError_t gram_schmidt(const KrylovWork& kw, const double* V, long ldv, int k, double* w, const double* pre, long n,
                          cudaStream_t st) {
   if (k < 1 || k > kKrylovMax || (ldv & 1) || ((reinterpret_cast<size_t>(V) | reinterpret_cast<size_t>(w) |
@@ -569,7 +546,11 @@ cudaError_t gram_schmidt(const KrylovWork& kw, const double* V, long ldv, int k,
   const KrylovDev kd = krylov_dev(kw);
   const int nb = krylov_blocks(n);
   const size_t smem = sizeof(double) * (size_t)k * KT;
-  cudaError_t e = launch_k(k_gram_schmidt<0>, nb, smem, st, V, ldv, k, w, pre, n, kd);
+  static std::atomic<unsigned long long> configured[2]{};
+  constexpr size_t most = sizeof(double) * kKrylovMax * KT;
+  cudaError_t e = allow_smem(k_gram_schmidt<0>, most, configured[0]);
+  if (e == cudaSuccess) e = allow_smem(k_gram_schmidt<1>, most, configured[1]);
+  if (e == cudaSuccess) e = launch_k(k_gram_schmidt<0>, nb, smem, st, V, ldv, k, w, pre, n, kd);
   if (e == cudaSuccess) e = launch_k(k_gram_schmidt<1>, nb, smem, st, V, ldv, k, w, (const double*)nullptr, n, kd);
   if (e == cudaSuccess) e = launch_k(k_gram_schmidt<2>, nb, 0, st, V, ldv, k, w, (const double*)nullptr, n, kd);
   if (e == cudaSuccess) e = normalise(w, w, n, kd.n2, st);

@@ -34,22 +34,22 @@ cudaError_t cg_start(KrylovState* s, const double* b, const double* Ax, const do
 cudaError_t cg_after_apply(KrylovState* s, double* x, double* r, double* z, double* p, const double* Ap,
                            const double* invd, long n, double* part, int maxit, cudaStream_t st);
 
-// ---- Krylov basis kernels.  One KrylovWork per solver: reduction partials, the block counter of
-// the finishing block, the results on the device and, in mapped pinned memory, on the host (read
-// after a stream synchronisation, no copy).
-constexpr int kKrylovMax = 64;  // basis vectors
+// ---- Krylov basis kernels.  One KrylovWork per operator handle, shared by its solvers (a handle is not
+// re-entrant): reduction partials, the block counter of the finishing block, the results on the
+// device and, in mapped pinned memory, on the host (read after a stream synchronisation, no copy).
+constexpr int kKrylovMax = 64;      // basis vectors
+constexpr int kKrylovBlocks = 444;  // 3 x 148 SMs
 struct KrylovWork {
-  double* dev = nullptr;     // partials, then h1[kKrylovMax], h2[kKrylovMax], norm^2 (slot 0, 1)
-  unsigned* count = nullptr;
-  double* host = nullptr;    // h[kKrylovMax], then kHostSlots scalars
-  double* host_dev = nullptr;  // the same memory as the device sees it
   static constexpr int kHostSlots = 8;
+  static constexpr size_t kDevDoubles = (size_t)kKrylovBlocks * kKrylovMax + 2 * kKrylovMax + 2 + 1;
+  static constexpr size_t kHostDoubles = kKrylovMax + kHostSlots;
+  double* dev = nullptr;       // partials, h1[kKrylovMax], h2[kKrylovMax], norm^2 (slot 0, 1), the counter (0)
+  double* host = nullptr;      // h[kKrylovMax], then kHostSlots scalars
+  double* host_dev = nullptr;  // the same memory as the device sees it
   double h(int j) const { return static_cast<const volatile double*>(host)[j]; }
   double slot(int s) const { return static_cast<const volatile double*>(host)[kKrylovMax + s]; }
   double* slot_dev(int s) const { return host_dev + kKrylovMax + s; }
 };
-cudaError_t krylov_create(KrylovWork* k);
-void krylov_destroy(KrylovWork* k);
 // w orthogonalised against V_0 .. V_{k-1} (V_j = V + j*ldv; k <= kKrylovMax) by classical Gram-Schmidt
 // applied twice, w = pre .* w first when pre is given; then w scaled by 1/|w| (when |w| > 0).  Host:
 // h(j) = the sum of both passes' coefficients, slot(0) = |w|^2 before the scaling.

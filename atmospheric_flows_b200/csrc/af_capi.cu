@@ -178,17 +178,26 @@ int af_create(const af_mesh_desc* m, int degree, int nq, double Ma, double Fr, d
       cudaMalloc(&o->d_u_fixed, 2 * ns * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&o->d_invdA, 2 * ns * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&o->d_ws, 6 * 2 * ns * sizeof(double)) != cudaSuccess ||  // t1, t2, r, z, p, Ap
-      cudaMalloc(&o->d_part, 4 * kMaxPartials * sizeof(double)) != cudaSuccess ||
+      cudaMalloc(&o->d_part, (4 * kMaxPartials + KrylovWork::kDevDoubles) * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&o->d_kst, sizeof(KrylovState)) != cudaSuccess)
     return cleanup(fail(AF_CUDA, "device allocation failed"));
+  // the Krylov kernels' block counter starts at zero: queued before the upload below, which is
+  // synchronous, so it is done before anything a stream of the handle queues
+  o->kw.dev = o->d_part + 4 * kMaxPartials;
+  if (cudaMemset(o->kw.dev + KrylovWork::kDevDoubles - 1, 0, sizeof(double)) != cudaSuccess)
+    return cleanup(fail(AF_CUDA, "Krylov workspace initialisation failed"));
   if (cudaMemcpy(o->d_vtx, m->vertices, nv * sizeof(double2), cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(fail(AF_CUDA, "vertex upload failed"));
   int* d_status = nullptr;
-  if (cudaHostAlloc((void**)&o->h_status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
+  constexpr size_t kHostOff = 16;  // ints before the Krylov kernels' host results
+  if (cudaHostAlloc((void**)&o->h_status, kHostOff * sizeof(int) + KrylovWork::kHostDoubles * sizeof(double),
+                    cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess)
     return cleanup(fail(AF_CUDA, "status word allocation failed"));
   *o->h_status = 0;
   if (cudaHostGetDevicePointer((void**)&d_status, o->h_status, 0) != cudaSuccess)
     return cleanup(fail(AF_CUDA, "status word mapping failed"));
+  o->kw.host = reinterpret_cast<double*>(o->h_status + kHostOff);
+  o->kw.host_dev = reinterpret_cast<double*>(d_status + kHostOff);
   o->mesh.status = d_status;
   o->mesh.vtx = o->d_vtx;
   o->mesh.nx = m->nx;

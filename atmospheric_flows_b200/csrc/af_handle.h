@@ -54,6 +54,9 @@ struct af_operator {
   // status word of the handle's kernels (mapped pinned host memory; mesh.status is its device
   // address): a kernel that gives up a bounded wait leaves a code there
   int* h_status = nullptr;
+  // workspace of the Krylov basis kernels (after the reduction partials; host results in the status
+  // word's page)
+  af::KrylovWork kw;
 
   long n_scalar() const { return (long)ncell * nd; }
 };

@@ -45,7 +45,6 @@ struct af_imex {
   double *cg_r, *cg_z, *cg_p, *cg_Ap, *invd_u, *invd_M, *invd_D;
   // GMRES workspace
   double *V, *gw, *scal;
-  KrylovWork kw;
   double* part;
   KrylovState* kst;
   af_schur_solver* schur = nullptr;  // FGMRES + Jacobi/multigrid (schur_preconditioner >= 0)
@@ -133,15 +132,15 @@ static int gmres_solve(af_imex* h, const Apply& A, const double* invd, double* x
   double res = 0.0, tol = -1.0;
   bool converged = false;
   // |b|^2 arrives with the first residual's norm
-  IM_CU(norm2_host(h->kw, b, n, 2, st));
+  IM_CU(norm2_host(h->op->kw, b, n, 2, st));
   h->op->launches += 1;
   while (true) {
     IM_AF(A(x, h->gw));
-    IM_CU(residual_start(h->kw, b, h->gw, invd, h->V, n, st));  // V_0 = P^{-1} r / |P^{-1} r|
+    IM_CU(residual_start(h->op->kw, b, h->gw, invd, h->V, n, st));  // V_0 = P^{-1} r / |P^{-1} r|
     h->op->launches += 2;
     IM_AF(sync_checked(h->op, st));
-    if (tol < 0.0) tol = eps * std::sqrt(h->kw.slot(2));
-    const double beta = std::sqrt(h->kw.slot(1));
+    if (tol < 0.0) tol = eps * std::sqrt(h->op->kw.slot(2));
+    const double beta = std::sqrt(h->op->kw.slot(1));
     res = beta;
     if (!std::isfinite(beta)) return ierr(AF_NAN, "GMRES: NaN residual");
     if (beta <= tol) { converged = true; break; }
@@ -152,11 +151,11 @@ static int gmres_solve(af_imex* h, const Apply& A, const double* invd, double* x
     for (int j = 0; j < m; ++j) {
       double* w = h->V + (long)(j + 1) * ld;
       IM_AF(A(h->V + (long)j * ld, w));
-      IM_CU(gram_schmidt(h->kw, h->V, ld, j + 1, w, invd, n, st));
+      IM_CU(gram_schmidt(h->op->kw, h->V, ld, j + 1, w, invd, n, st));
       h->op->launches += kGramSchmidtLaunches;
       IM_AF(sync_checked(h->op, st));
-      for (int i = 0; i <= j; ++i) Hs(i, j) = h->kw.h(i);
-      const double hn = std::sqrt(h->kw.slot(0));
+      for (int i = 0; i <= j; ++i) Hs(i, j) = h->op->kw.h(i);
+      const double hn = std::sqrt(h->op->kw.slot(0));
       Hs(j + 1, j) = hn;
       for (int i = 0; i < j; ++i) {  // previous rotations
         const double t = cs[i] * Hs(i, j) + sn[i] * Hs(i + 1, j);
@@ -310,7 +309,8 @@ static int set_rho_for_fixed(af_imex* h, const double* rho) {
   af_operator* o = h->op;
   IM_AF(af_set_rho_for_fixed(o, rho));
   IM_AF(af_set_NS_stage(o, 3));
-  return af_compute_diagonal(o, h->invd_u);
+  // the inverse diagonal of A serves the CG solves alone
+  return h->opt.mass_solver == 0 ? af_compute_diagonal(o, h->invd_u) : AF_OK;
 }
 
 static int fixed_point(af_imex* h, int stage, double* p_out, double* u_out) {
@@ -328,10 +328,10 @@ static int fixed_point(af_imex* h, int stage, double* p_out, double* u_out) {
     IM_AF(pressure_fixed_point(h, stage, iter));
     IM_AF(update_velocity(h, stage));
     ++iters;
-    IM_CU(maxabs2(h->pfix, h->pfix_old, ns, h->part, h->kw.slot_dev(3), o->stream));
+    IM_CU(maxabs2(h->pfix, h->pfix_old, ns, h->part, h->op->kw.slot_dev(3), o->stream));
     o->launches += 2;
     IM_AF(sync_checked(o, o->stream));
-    err = h->kw.slot(4) / (h->kw.slot(3) + 1e-10);
+    err = h->op->kw.slot(4) / (h->op->kw.slot(3) + 1e-10);
     if (err < h->opt.fixed_point_tol) break;
     IM_CU(cudaMemcpyAsync(h->pfix_old, h->pfix, ns * 8, cudaMemcpyDeviceToDevice, o->stream));
   }
@@ -847,8 +847,7 @@ int af_imex_create(const af_mesh_desc* mesh, int degree, double Ma, double Fr, d
   r = AF_OK;
   const long total = 15 * (ns + 1) + 13 * 2 * ns + (long)(m + 1) * krylov_stride(ns) + 8 +
                      4 * kMaxPartials + 16;
-  if (krylov_create(&h->kw) != cudaSuccess || cudaMalloc(&h->mem, total * sizeof(double)) != cudaSuccess) {
-    krylov_destroy(&h->kw);
+  if (cudaMalloc(&h->mem, total * sizeof(double)) != cudaSuccess) {
     af_destroy(h->op);
     delete h;
     return ierr(AF_CUDA, "af_imex_create: device allocation failed");
@@ -898,7 +897,6 @@ int af_imex_destroy(af_imex* h) {
   if (h->op) af_synchronize(h->op);
   af_schur_solver_destroy(h->schur);
   cudaFree(h->mem);
-  krylov_destroy(&h->kw);
   cudaFree(h->adj_mem);
   for (int k = 0; k < 2; ++k) {
     for (double* p : h->rec_p[k]) cudaFree(p);

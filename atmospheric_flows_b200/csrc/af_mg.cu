@@ -185,7 +185,6 @@ struct af_schur_solver {
   double* invd = nullptr;       // Jacobi: inverse diagonal of D
   // FGMRES workspace
   double *V = nullptr, *Z = nullptr, *gw = nullptr;
-  KrylovWork kw;
   cudaEvent_t ev[2] = {nullptr, nullptr};  // device time of a solve
   std::vector<void*> owned;
   af_schur_stats stats{};
@@ -592,9 +591,8 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
   // reductions and FGMRES workspace
   if ((r = alloc(s, (void**)&s->part, sizeof(double) * 4 * kMaxPartials)) != AF_OK) return cleanup(r);
   if ((r = alloc(s, (void**)&s->scal, sizeof(double) * 8)) != AF_OK) return cleanup(r);
-  if (krylov_create(&s->kw) != cudaSuccess || cudaEventCreate(&s->ev[0]) != cudaSuccess ||
-      cudaEventCreate(&s->ev[1]) != cudaSuccess)
-    return cleanup(merr(AF_CUDA, "af_schur_solver_create: Krylov workspace"));
+  if (cudaEventCreate(&s->ev[0]) != cudaSuccess || cudaEventCreate(&s->ev[1]) != cudaSuccess)
+    return cleanup(merr(AF_CUDA, "af_schur_solver_create: event creation failed"));
   const long ld0 = krylov_stride(ns0);
   if ((r = alloc(s, (void**)&s->V, sizeof(double) * ld0 * (o.restart + 1))) != AF_OK) return cleanup(r);
   if ((r = alloc(s, (void**)&s->Z, sizeof(double) * ld0 * o.restart)) != AF_OK) return cleanup(r);
@@ -667,7 +665,6 @@ int af_schur_solver_destroy(af_schur_solver* s) {
   cudaSetDevice(s->op->device);
   cudaStreamSynchronize(s->op->stream);
   for (void* p : s->owned) cudaFree(p);
-  krylov_destroy(&s->kw);
   for (cudaEvent_t e : s->ev)
     if (e) cudaEventDestroy(e);
   delete s;
@@ -728,7 +725,7 @@ int fgmres(af_schur_solver* s, const Apply& A, double* x, const double* b, doubl
   std::vector<double> H((m + 1) * m), cs(m), sn(m), g(m + 1);
   auto Hs = [&](int i, int j) -> double& { return H[i * m + j]; };
   // |b|^2 arrives with the first residual's norm
-  MG_CU(norm2_host(s->kw, b, n, 2, st));
+  MG_CU(norm2_host(o->kw, b, n, 2, st));
   o->launches += 1;
   double tol = -1.0;
   int total = 0;
@@ -736,11 +733,11 @@ int fgmres(af_schur_solver* s, const Apply& A, double* x, const double* b, doubl
   bool converged = false;
   while (true) {
     MG_AF(A(s->gw, x));
-    MG_CU(residual_start(s->kw, b, s->gw, nullptr, s->V, n, st));  // V_0 = r / |r|
+    MG_CU(residual_start(o->kw, b, s->gw, nullptr, s->V, n, st));  // V_0 = r / |r|
     o->launches += 2;
     MG_AF(sync_checked(o, st));
-    if (tol < 0.0) tol = rel_tol * std::sqrt(s->kw.slot(2));
-    const double beta = std::sqrt(s->kw.slot(1));
+    if (tol < 0.0) tol = rel_tol * std::sqrt(o->kw.slot(2));
+    const double beta = std::sqrt(o->kw.slot(1));
     res = beta;
     if (res0 < 0.0) res0 = beta;
     if (!std::isfinite(beta)) return merr(AF_NAN, "Schur FGMRES: NaN residual");
@@ -754,11 +751,11 @@ int fgmres(af_schur_solver* s, const Apply& A, double* x, const double* b, doubl
       double* w = s->V + (long)(j + 1) * ld;
       MG_AF(precondition(s, zj, s->V + (long)j * ld));
       MG_AF(A(w, zj));
-      MG_CU(gram_schmidt(s->kw, s->V, ld, j + 1, w, nullptr, n, st));
+      MG_CU(gram_schmidt(o->kw, s->V, ld, j + 1, w, nullptr, n, st));
       o->launches += kGramSchmidtLaunches;
       MG_AF(sync_checked(o, st));
-      for (int i = 0; i <= j; ++i) Hs(i, j) = s->kw.h(i);
-      const double hn = std::sqrt(s->kw.slot(0));
+      for (int i = 0; i <= j; ++i) Hs(i, j) = o->kw.h(i);
+      const double hn = std::sqrt(o->kw.slot(0));
       Hs(j + 1, j) = hn;
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * Hs(i, j) + sn[i] * Hs(i + 1, j);
