@@ -237,11 +237,21 @@ __device__ __forceinline__ void report_status(int* status, int code) {
   }
 }
 
-// Cells per CTA, per degree (see the kernel).
+// Cells per CTA, per degree: whole warps at 2P+1 threads a cell.  Small CTAs wait less for one another
+// at the barriers, but more of their cells have neighbours outside.  Measured (us, 131072 cells; fused
+// stage 1, stage 3, the three split calls of stage 3, C):
+//   p=1 (262144 cells)  42 x 3 CTAs per SM 106, 242, 440, 36;  32 x 4: 100, 231, 436, 35;  21 x 6: 107, 253, 459, 37
+//   p=2  24 x 3: 84, 195, 369, 32;  18 x 4: 86, 203, 391, 33;  12 x 6: 85, 208, 402, 35
+//   p=3  18 x 3: 200, 456, 955, 70;  16 x 3: 211, 482, 985, 70;  13 x 4: 196, 452, 918, 73;
+//        9 x 6: 170, 406, 838, 64;  8 x 6: 180, 437, 904, 68
+//   p=4  14 x 3: 207, 481, 911, 82;  12 x 3: 229, 545, 1007, 91;  10 x 4: 221, 548, 1000, 87;  6 x 6: 232, 557, 1088, 101
+//   p=5 (65536 cells)  11 x 2: 227, 515, 928, 66;  8 x 3: 217, 483, 825, 68 (stage 2 430, not 412);  5 x 4: 224, 545, 978, 67
+//   p=6 (32768 cells)  8 x 2: 152, 327, 561, 44;  4 x 4: 151, 332, 587, 47
+// An odd number of cells needs an even number of nodes a cell: the bulk copies start on 16 bytes.
 template <int P, class R = double>
 constexpr int cells_per_block() {
   if (sizeof(R) == 4) return P <= 1 ? 64 : (P == 2 ? 32 : (P <= 4 ? 16 : 8));
-  return P <= 1 ? 42 : (P == 2 ? 24 : (P == 3 ? 18 : (P == 4 ? 14 : (P == 5 ? 11 : 8))));
+  return P <= 1 ? 32 : (P == 2 ? 24 : (P == 3 ? 9 : (P == 4 ? 14 : (P == 5 ? 11 : 8))));
 }
 
 template <int MAXARR, int MAXOUT, class R = double>
@@ -519,11 +529,29 @@ struct Layout {
   // static shared memory: tables, neighbours, barriers (bound)
   static constexpr int STATIC = 2 * NB * (NTL + 2 * NTT) + 12 * NB * NTF + 16 * CB + 4 * NOUT + 64;
   static constexpr size_t MAX_BYTES = 225 * 1024;  // 227 KB per CTA, up to 2 KB of it static
-  // CTAs per SM, the hint of __launch_bounds__: as many as the shared memory holds, at most three
+  // CTAs per SM, the hint of __launch_bounds__: as many as the shared memory holds, at most 12 warps
+  // (168 registers a thread; degrees 5 and 6 need more: 8 warps) or, with larger CTAs, three (two)
   static constexpr int FIT = (int)(228 * 1024 / (BYTES + 1024 + STATIC));
-  static constexpr int MOST = P >= 5 ? 2 : 3;  // degrees 5 and 6 need more than 168 registers
+  static constexpr int WARPS = (NT + 31) / 32;
+  static constexpr int MOST = P >= 5 ? imax(2, 8 / WARPS) : imax(3, 12 / WARPS);
   static constexpr int CTAS = FIT < 1 ? 1 : (FIT > MOST ? MOST : FIT);
 };
+
+// Cells per CTA of a policy launched without a choice of its own: cells_per_block, or the next smaller
+// count with which the bulk copies stay aligned where the shared memory then holds one more CTA per SM.
+// That is so for the fused stage-2 right-hand sides of degree 4 (12 cells: three CTAs, not two; 455 ->
+// 411 us at 512x256) and degree 3 (8 cells: six, not five; 361 -> 340 us).
+template <int P, class Phys>
+constexpr int default_cells() {
+  using R = RealOf<Phys>;
+  constexpr int CB = cells_per_block<P, R>(), LESS = CB - ((P + 1) * (P + 1) % 2 ? 2 : 1);
+  using L = Layout<P, Phys, CB>;
+  if constexpr (sizeof(R) == 8 && L::FIT < L::MOST) {
+    return Layout<P, Phys, LESS>::FIT > L::FIT ? LESS : CB;
+  } else {
+    return CB;
+  }
+}
 
 // The most cells per CTA, from CB down in steps of two, with which two CTAs share an SM (one, when
 // two do not fit even with two cells).
@@ -625,7 +653,7 @@ __device__ __forceinline__ void contract_eo_T(const R* f, R* y) {
 // ----------------------------------------------------------------------------------
 // the kernel
 // ----------------------------------------------------------------------------------
-template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>(), int MINB = Layout<P, Phys, CB_>::CTAS>
+template <int P, class Phys, int CB_ = default_cells<P, Phys>(), int MINB = Layout<P, Phys, CB_>::CTAS>
 __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
     k_cellop(const __grid_constant__ MeshDev mesh,
              const __grid_constant__ ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>> ptr,
@@ -1520,7 +1548,7 @@ cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<unsigned long long>& 
   return cudaSuccess;
 }
 
-template <int P, class Phys, int CB_ = cells_per_block<P, RealOf<Phys>>(), int MINB = Layout<P, Phys, CB_>::CTAS>
+template <int P, class Phys, int CB_ = default_cells<P, Phys>(), int MINB = Layout<P, Phys, CB_>::CTAS>
 cudaError_t launch_cellop(const MeshDev& mesh,
                           const ArgPtrs<PhysInfo<Phys>::NARR_TOTAL, Phys::NOUT_ARR, RealOf<Phys>>& ptr,
                           const typename Phys::Params& prm, int ncell, cudaStream_t stream) {

@@ -76,3 +76,30 @@ def test_range_launches_at_any_cell(P):
         g.vmult_rhs_fused_host(*host, src)
         for a, b in zip(out, host):
             assert np.array_equal(a.cpu().numpy(), b)
+
+
+# cells per CTA of the fused right-hand sides where they differ from the sizes above: the degree's own
+# count, and the smaller one of stage 2 that lets one more CTA share an SM
+@pytest.mark.parametrize("P,cb", [(1, 32), (3, 9), (3, 8), (4, 12)])
+def test_rhs_at_small_tile_edges(P, cb):
+    from atmospheric_flows_b200.operator import EULEROperator
+    from oracle.oracle import OracleOperator
+    sc = M.Scaling()
+    for k, (nx, nz, per) in enumerate([(cb, 2, True), (cb + 1, 3, False), (3, cb, True), (2 * cb - 1, 1, True)]):
+        m = M.jitter_mesh(M.hill_mesh(nx, nz, periodic_x=per), 0.1, 17 + k)
+        g, o = EULEROperator(m, P, sc.Ma, sc.Fr, 0.5), OracleOperator(m, P, sc.Ma, sc.Fr, 0.5)
+        st = [M.random_state(m, P, 13 * k + j) for j in range(4)]
+        full = [a for s in st for a in (s.rho, s.u, s.p)]
+        for stage in (1, 2, 3):
+            src = full[:3 * stage] + [st[3].rho, st[3].u]
+            d = [torch.from_numpy(a).cuda() for a in src]
+            out = [torch.empty_like(d[0]), torch.empty_like(d[1]), torch.empty_like(d[0])]
+            g.set_HYPERBOLIC_stage(stage)
+            o.set_HYPERBOLIC_stage(stage)
+            g.vmult_rhs_fused(*out, d)
+            g.synchronize()
+            want = [o.vmult_rhs_rho_update([x for j in range(stage) for x in src[3 * j:3 * j + 2]]),
+                    o.vmult_rhs_velocity_fixed(src[:3 * stage] + (src[3 * stage:3 * stage + 1] if stage < 3 else [])),
+                    o.vmult_rhs_pressure(src)]
+            for got, w in zip(out, want):
+                assert rel(got.cpu().numpy(), w) < TOL, (nx, nz, per, stage)
