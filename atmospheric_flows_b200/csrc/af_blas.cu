@@ -279,7 +279,9 @@ namespace af {
 // pass and, with the norm, to the host through mapped memory.  Measured, all four launches: 15
 // vectors of 3.3 M elements 247 us (5.4 TB/s), of 0.8 M 67 us, of 0.2 M 35 us.  Before: eight
 // launches, four reads of the basis with 8-byte loads, and two pageable copies per iteration; the FP64
-// IMEX step at 256x128 (456 iterations) 95.0 -> 74.2 ms, the small 40x16 step 1.17 -> 0.84 ms.
+// IMEX step at 256x128 (456 iterations) 95.0 -> 74.2 ms, the small 40x16 step 1.17 -> 0.84 ms.  The
+// second pass takes the chunks from the last to the first, so that the end of the basis is read from L2
+// by it and the beginning by the third (FP64 step 73.9 -> 71.7 ms).
 constexpr int KT = 256, KC = 4 * KT;  // threads per block, elements per chunk
 constexpr int KJ = 4;                 // basis vectors loaded together (6, 8: 5 % faster at k = 28, 10-20 % slower at k = 4)
 
@@ -410,7 +412,9 @@ __global__ void __launch_bounds__(KT)
       nn += fma(a.x, a.x, a.y * a.y) + fma(b.x, b.x, b.y * b.y);
     }
   };
-  for (long c = blockIdx.x; c * KC < n; c += gridDim.x) {
+  const long nc = (n + KC - 1) / KC;
+  for (long b = blockIdx.x; b < nc; b += gridDim.x) {
+    const long c = MODE == 1 ? nc - 1 - b : b;  // backwards: what the pass before read last is still in L2
     if ((c + 1) * KC <= n) chunk(c, std::true_type{});
     else chunk(c, std::false_type{});
   }
