@@ -72,6 +72,15 @@ struct GsMesh {
   const float* geo;  // [tile][kGsGeo][32]
   FastDiv nx;
   int nz, periodic_x, ncell;
+  int* status;          // as in MeshDev
+  int test_wait_polls;  // as in MeshDev: k_gs_chain waits for a step that nobody reaches
+};
+
+// the coefficients of consecutive Chebyshev steps
+constexpr int kGsSteps = 64;  // even: x takes two directions every second step
+struct GsSteps {
+  int n;
+  float alpha[kGsSteps], s[kGsSteps];
 };
 
 template <int P>
@@ -80,6 +89,10 @@ struct GsShape {
   // CTAs per SM asked of the compiler.  Degree 4, (k_gs_binv, k_gs_zstep), the mixed IMEX step at
   // 512x256: (4, 6) 46.3 ms, (5, 6) 45.4, (5, 7) 45.2, (6, 6) 46.8 (k_gs_binv spills at 64 registers).
   static constexpr int CTAS_B = 800 / NT, CTAS_Z = (P <= 4 ? 1120 : 900) / NT;
+  // k_gs_chain: more CTAs per SM take larger meshes.  Degree 4, 3 / 4 / 5 per SM (128, 102, 80 registers; 0,
+  // 160 and more bytes spilled): 256 tiles 64, 64, 75 us, 576 tiles (the pairs) 166, 82, 120; degree 2, 5 / 8 per SM: 256
+  // tiles 45, 48 us, 1024 tiles (the pairs) 128, 64
+  static constexpr int CTAS_C = (P <= 2 ? 800 : 640) / NT;
   // the thread's element of node or point 0 .. and the strides between its nodes (column m) and faces
   __device__ __forceinline__ static size_t column(int tile, int m, int lane) {
     return (size_t)tile * (ND * kGsTile) + (m * kGsTile + lane);
@@ -388,13 +401,241 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
   for (int f = 0; f < 4; ++f) tB[f * S::SF] = t[f];
 }
 
+// ------------------------------------------------- all steps in one launch, small meshes
+// The pairs (k_gs_binv, k_gs_zstep) of st.n steps by CTAs that stay: one tile each, all resident at the
+// same time (a cooperative launch; gs_chain_tiles), with z, d, x and the coefficients in registers and
+// the fluxes of w in shared memory.  Between half steps only the face values pass through memory, each
+// in one 8-byte word with the count of its half step: a thread reads the words of its four neighbour
+// points until they carry the count that it needs, with no flag, fence or barrier in between, and forms
+// meanwhile what its own tile contributes.  A value is overwritten only after the thread that reads it
+// has published its own next one (the threads of a face point read each other's).  k_gs_entry writes
+// the first words and clears the others; counts go on over the launches of one application.  Waits
+// are bounded: a CTA that gives up reports it and leaves, and so do those that wait for it.
+// What bounds it: latency.  Degree-20 polynomial, us, the pairs (one launch per half step) / with
+// flags per tile, fences and barriers / now:
+//   degree 4  256 tiles 123 / 97 / 64, 444 tiles 166 / 106 / 72, 1 tile 99 / 64 / 42;  degree 2, 576 tiles
+//   100 / 96 / 48;  degree 6, 96 tiles 167 / 94 / 66   (a step and its adjoint at 128x64: 49.9 / 46.6 / 39.2 ms)
+constexpr int kGsWaitPolls = 1 << 19;
+using GsWord = unsigned long long;  // a face value and its count
+__device__ __forceinline__ GsWord gs_word(float v, int count) {
+  return (GsWord)(unsigned)count << 32 | (GsWord)__float_as_uint(v);
+}
+__device__ __forceinline__ void gs_put(GsWord* w, float v, int count) {
+  *reinterpret_cast<volatile GsWord*>(w) = gs_word(v, count);
+}
+
+template <int P>
+__global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
+    k_gs_chain(const __grid_constant__ GsMesh mesh, const __grid_constant__ GsSteps st, const float cB, const float cgg,
+               const float gfac, const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x,
+               float* dtr, GsWord* wd, GsWord* wg, const int base, const int more) {
+  using S = GsShape<P>;
+  constexpr int P1 = S::P1, ND = S::ND;
+  __shared__ float s_sw[ND * kGsTile];      // weighted values of -cB d
+  __shared__ float s_xf[4 * P1 * kGsTile];  // x-face fluxes of B [face][component][point][lane]
+  __shared__ float s_w[2 * ND * kGsTile];   // w [component][node][lane]
+  __shared__ float s_fx[ND * kGsTile], s_d[ND * kGsTile], s_xf2[2 * P1 * kGsTile];
+  const CobT<P, float>& cb = cobr<P, float>();
+  GsThread<P> th(mesh);
+  th.geometry(mesh);
+  th.neighbours(mesh);
+  const int lane = th.lane, m = th.m;
+  const size_t oc = S::column(th.tile, m, lane), op = S::point(th.tile, m, lane);
+  float zc[P1], dc[P1], xc[P1], wa[P1], pc[P1], pt[4], tp[4];
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {
+    zc[q] = z[oc + q * S::SN];
+    dc[q] = d[oc + q * S::SN];
+    xc[q] = x[oc + q * S::SN];
+    wa[q] = WA[oc + q * S::SN];
+    pc[q] = pg[oc + q * S::SN];
+  }
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    tp[f] = dtr[op + f * S::SF];
+    pt[f] = ptr[op + f * S::SF];
+  }
+  gs_ends<P>(pc, pt[2], pt[3]);
+  gs_ends<P>(dc, tp[2], tp[3]);
+  // the neighbours' values of that count (a wall takes the own one); false when the bound was reached
+  const bool hook = mesh.test_wait_polls > 0;
+  const int polls = hook ? mesh.test_wait_polls : kGsWaitPolls;
+  unsigned src[4];  // few tiles: 32 bits hold the offsets
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const int nb = th.nb[f] < 0 ? 0 : th.nb[f];
+    src[f] = (unsigned)S::point(nb >> 5, m, nb & 31) + (f ^ 1) * S::SF;
+  }
+  auto others = [&](const GsWord* w, int count, const float* own, float* v) {
+    if (hook) count = -1;
+    bool ok = false;
+    for (int it = 0; it < polls && !ok; ++it) {
+      GsWord a[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f)
+        a[f] = th.nb[f] >= 0 ? *reinterpret_cast<const volatile GsWord*>(w + src[f]) : gs_word(own[f], count);
+      ok = true;
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        ok = ok && (int)(a[f] >> 32) == count;
+        v[f] = __uint_as_float((unsigned)a[f]);
+      }
+      ok = __all_sync(0xffffffffu, ok);
+    }
+    if (!ok && lane == 0) report_status(mesh.status, kStatusStageTimeout);
+    return ok;
+  };
+
+  const float wx = cb.w[m], lo = cb.lo[m], hi = cb.hi[m], gw = 1.f / cb.w[m];
+  const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]);
+#pragma unroll
+  for (int q = 0; q < P1; ++q) s_sw[(q * P1 + m) * kGsTile + lane] = -cB * dc[q] * (wx * cb.w[q]);
+  __syncthreads();
+#pragma unroll 1
+  for (int it = 1; it <= st.n; ++it) {
+    // ---- k_gs_binv: what the own tile gives, while the neighbours arrive
+    float tm[4], ec[P1], g[4], a0[P1], a1[P1];
+    {
+      float e0[P1], e1[P1];
+#pragma unroll
+      for (int q = 0; q < P1; ++q) {
+        const float sw = -cB * dc[q] * (wx * cb.w[q]);
+        e0[q] = -th.J10(cb.g[q]) * sw;
+        e1[q] = th.J00(cb.g[q]) * sw;
+      }
+#pragma unroll
+      for (int i = 0; i < P1; ++i) {
+        a0[i] = cb.Dg[0][i] * e0[0];
+        a1[i] = cb.Dg[0][i] * e1[0];
+#pragma unroll
+        for (int q = 1; q < P1; ++q) {
+          a0[i] = fmaf(cb.Dg[q][i], e0[q], a0[i]);
+          a1[i] = fmaf(cb.Dg[q][i], e1[q], a1[i]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < P1; ++q) {
+        const float dg = cb.Dg[q][m], k0 = dg * th.J11(cb.g[q]), k1 = -dg * th.J01(cb.g[q]);
+#pragma unroll
+        for (int i = 0; i < P1; ++i) {
+          const float sw = s_sw[(i * P1 + q) * kGsTile + lane];
+          a0[i] = fmaf(k0, sw, a0[i]);
+          a1[i] = fmaf(k1, sw, a1[i]);
+        }
+      }
+    }
+    const bool okd = others(wd, base + 2 * it - 2, tp, tm);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      float n0, n1;
+      th.normal(f, n0, n1);
+      const float a = cB * 0.5f * (tp[f] + tm[f]) * wx;
+      const float F0 = a * n0, F1 = a * n1;
+      if (f < 2) {
+        s_xf[((f * 2 + 0) * P1 + m) * kGsTile + lane] = F0;
+        s_xf[((f * 2 + 1) * P1 + m) * kGsTile + lane] = F1;
+      } else {
+#pragma unroll
+        for (int i = 0; i < P1; ++i) {
+          const float e = f == 2 ? cb.lo[i] : cb.hi[i];
+          a0[i] = fmaf(e, F0, a0[i]);
+          a1[i] = fmaf(e, F1, a1[i]);
+        }
+      }
+    }
+    if (__syncthreads_or(!okd)) return;
+#pragma unroll
+    for (int i = 0; i < P1; ++i) {
+      float v0 = a0[i], v1 = a1[i];
+      v0 = fmaf(lo, s_xf[(0 * P1 + i) * kGsTile + lane], v0);
+      v1 = fmaf(lo, s_xf[(1 * P1 + i) * kGsTile + lane], v1);
+      v0 = fmaf(hi, s_xf[(2 * P1 + i) * kGsTile + lane], v0);
+      v1 = fmaf(hi, s_xf[(3 * P1 + i) * kGsTile + lane], v1);
+      const float w0 = wa[i] * v0, w1 = wa[i] * v1;
+      a0[i] = w0;
+      a1[i] = w1;
+      s_w[(i * P1 + m) * kGsTile + lane] = w0;
+      s_w[(ND + i * P1 + m) * kGsTile + lane] = w1;
+      const float sv = -cgg * pc[i] * (wx * cb.w[i]);
+      s_fx[(i * P1 + m) * kGsTile + lane] = sv * (J11 * w0 - J01 * w1);
+      ec[i] = sv * (th.J00(cb.g[i]) * w1 - th.J10(cb.g[i]) * w0);
+    }
+    {
+      float t0[4], t1[4];
+      gs_ends<P>(a0, t0[2], t0[3]);
+      gs_ends<P>(a1, t1[2], t1[3]);
+      __syncthreads();
+      gs_row_ends<P>(s_w, m, lane, t0[0], t0[1]);
+      gs_row_ends<P>(s_w + ND * kGsTile, m, lane, t1[0], t1[1]);
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        float n0, n1;
+        th.normal(f, n0, n1);
+        g[f] = 0.5f * cgg * wx * pt[f] * (t0[f] * n0 + t1[f] * n1);
+        gs_put(wg + op + f * S::SF, g[f], base + 2 * it - 1);
+      }
+    }
+    // ---- k_gs_zstep
+    float F[4], a[P1];
+#pragma unroll
+    for (int i = 0; i < P1; ++i) {
+      a[i] = cb.Dg[0][i] * ec[0];
+#pragma unroll
+      for (int q = 1; q < P1; ++q) a[i] = fmaf(cb.Dg[q][i], ec[q], a[i]);
+#pragma unroll
+      for (int q = 0; q < P1; ++q) a[i] = fmaf(cb.Dg[q][m], s_fx[(i * P1 + q) * kGsTile + lane], a[i]);
+    }
+    const bool okg = others(wg, base + 2 * it - 1, g, F);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) F[f] = g[f] - F[f];
+    s_xf2[m * kGsTile + lane] = F[0];
+    s_xf2[(P1 + m) * kGsTile + lane] = F[1];
+#pragma unroll
+    for (int i = 0; i < P1; ++i) a[i] = fmaf(cb.hi[i], F[3], fmaf(cb.lo[i], F[2], a[i]));
+    if (__syncthreads_or(!okg)) return;
+    const float alpha = st.alpha[it - 1], s = st.s[it - 1];
+#pragma unroll
+    for (int i = 0; i < P1; ++i) {
+      float y = a[i];
+      y = fmaf(lo, s_xf2[i * kGsTile + lane], y);
+      y = fmaf(hi, s_xf2[(P1 + i) * kGsTile + lane], y);
+      const float det = th.J00(cb.g[i]) * J11 - th.J10(cb.g[i]) * J01;
+      const float zn = zc[i] + __fdividef(gfac * gw * y, det * cb.w[i]) - dc[i];
+      const float nd = alpha * dc[i] + s * zn;
+      if (it % 2 == 0) xc[i] = (xc[i] + dc[i]) + nd;
+      else if (it == st.n) xc[i] = xc[i] + nd;
+      s_d[(i * P1 + m) * kGsTile + lane] = nd;
+      s_sw[(i * P1 + m) * kGsTile + lane] = -cB * nd * (wx * cb.w[i]);
+      zc[i] = zn;
+      dc[i] = nd;
+    }
+    if (it == st.n && !more) break;
+    gs_ends<P>(dc, tp[2], tp[3]);
+    __syncthreads();
+    gs_row_ends<P>(s_d, m, lane, tp[0], tp[1]);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) gs_put(wd + op + f * S::SF, tp[f], base + 2 * it);
+  }
+#pragma unroll
+  for (int q = 0; q < P1; ++q) {
+    x[oc + q * S::SN] = xc[q];
+    if (more) {
+      z[oc + q * S::SN] = zc[q];
+      d[oc + q * S::SN] = dc[q];
+    }
+  }
+  if (more)
+#pragma unroll
+    for (int f = 0; f < 2; ++f) dtr[op + f * S::SF] = tp[f];
+}
+
 // ------------------------------------------------------------ basis changes
 // The preconditioner's input: v (FP64, a residual: dual, nodal) -> b_g = (Vi x Vi)^T v,
-// d = x = sc b_g / JxW, z = theta d and the traces of d.
+// d = x = sc b_g / JxW, z = theta d and the traces of d, for k_gs_chain also as words of count 0 (wd; wg cleared).
 template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT)
     k_gs_entry(const GsMesh mesh, const double* v, const float sc, const float theta,
-               float* z, float* d, float* x, float* dtr) {
+               float* z, float* d, float* x, float* dtr, GsWord* wd, GsWord* wg) {
   using S = GsShape<P>;
   constexpr int P1 = S::P1, ND = S::ND, NDS = ND | 1;
   __shared__ float s_v[kGsTile * NDS], s_t[ND * kGsTile];
@@ -440,6 +681,13 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
   gs_row_ends<P>(s_t, m, lane, t[0], t[1]);
 #pragma unroll
   for (int f = 0; f < 4; ++f) tB[f * S::SF] = t[f];
+  if (wd)
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const size_t o = S::point(th.tile, m, lane) + f * S::SF;
+      wd[o] = gs_word(t[f], 0);
+      wg[o] = 0;
+    }
 }
 
 // The preconditioner's output: x = (Vi x Vi) x_g (nodal, FP64).

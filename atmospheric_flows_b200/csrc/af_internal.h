@@ -132,9 +132,10 @@ struct DegreeOps {
   // ---- the same smoother in the Gauss-point basis (af_gauss.cuh): fields and face arrays in its
   // layout, tiled by gs_tile cells; geo: the mesh's geometry block (kGsGeo floats per cell)
   cudaError_t (*gs_geo)(const MeshDev&, float* geo, int ncell, cudaStream_t);
-  //   entry: d = x = sc (Vi x Vi)^T v / JxW (v FP64 nodal), z = theta d, dtr = traces of d
+  //   entry: d = x = sc (Vi x Vi)^T v / JxW (v FP64 nodal), z = theta d, dtr = traces of d; words (may
+  //   be null): the face words of gs_chain, 8 (P + 1) per cell of whole tiles
   cudaError_t (*gs_entry)(const MeshDev&, const float* geo, const double* v, float sc, float theta, float* z, float* d,
-                          float* x, float* dtr, int ncell, cudaStream_t);
+                          float* x, float* dtr, unsigned long long* words, int ncell, cudaStream_t);
   //   w = diag(WA) B_g d, written as the mapped fluxes of C0 w at the points (fx, fe) and on the
   //   faces (gf); pg, ptr: p_fixed at the points and on the x-faces; cgg = cdt gamma/(gamma-1)
   cudaError_t (*gs_binv)(const MeshDev&, const float* geo, const float* d, const float* dtr, float cB, const float* WA,
@@ -150,6 +151,13 @@ struct DegreeOps {
   //   the coefficients: pg = (V x V) p, its x-face traces, WA = 1 / (rho JxW)
   cudaError_t (*gs_values)(const MeshDev&, const double* p, const double* rho, float* pg, float* ptr, float* WA,
                            int ncell, cudaStream_t);
+  //   the most tiles that gs_chain takes (all resident at once; 0: none) on a device
+  int (*gs_chain_tiles)(int device);
+  //   n pairs (gs_binv, gs_zstep) with (alpha, s) = coef[2 i], coef[2 i + 1], after gs_entry with the
+  //   same words; d, z and dtr are left in between
+  cudaError_t (*gs_chain)(const MeshDev&, const float* geo, const float* coef, int n, float cB, float cgg, float g,
+                          const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x, float* dtr,
+                          unsigned long long* words, int ncell, cudaStream_t);
 };
 
 const DegreeOps* degree_ops(int P);  // null if the degree was not compiled

@@ -1042,15 +1042,54 @@ cudaError_t launch_gs(K kernel, int ncell, cudaStream_t st, bool pdl, A... args)
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 GsMesh gs_mesh(const MeshDev& m, const float* geo, int ncell) {
-  return {geo, FastDiv::make(m.nx), m.nz, m.periodic_x, ncell};
+  return {geo, FastDiv::make(m.nx), m.nz, m.periodic_x, ncell, m.status, m.test_wait_polls};
 }
+// words of one of the two face arrays of k_gs_chain
+size_t gs_words(int ncell) { return (size_t)(ncell + kGsTile - 1) / kGsTile * kGsTile * 4 * (P + 1); }
 cudaError_t gs_geo(const MeshDev& mesh, float* geo, int ncell, cudaStream_t st) {
   k_gs_geo<<<(ncell + 255) / 256, 256, 0, st>>>(mesh, geo, ncell);
   return cudaGetLastError();
 }
 cudaError_t gs_entry(const MeshDev& mesh, const float* geo, const double* v, float sc, float theta, float* z, float* d,
-                     float* x, float* dtr, int ncell, cudaStream_t st) {
-  return launch_gs(k_gs_entry<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), v, sc, theta, z, d, x, dtr);
+                     float* x, float* dtr, unsigned long long* words, int ncell, cudaStream_t st) {
+  return launch_gs(k_gs_entry<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), v, sc, theta, z, d, x, dtr, words,
+                   words ? words + gs_words(ncell) : nullptr);
+}
+int gs_chain_tiles(int device) {
+  int sms = 0, per = 0, coop = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gs_chain<P>, GsShape<P>::NT, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return coop ? sms * per : 0;
+}
+cudaError_t gs_chain(const MeshDev& mesh, const float* geo, const float* coef, int n, float cB, float cgg, float g,
+                     const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x, float* dtr,
+                     unsigned long long* words, int ncell, cudaStream_t st) {
+  if (ncell <= 0) return cudaSuccess;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((ncell + kGsTile - 1) / kGsTile));
+  cfg.blockDim = dim3((unsigned)GsShape<P>::NT);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  for (int k = 0; k < n; k += kGsSteps) {
+    GsSteps s{};
+    s.n = n - k < kGsSteps ? n - k : kGsSteps;
+    for (int i = 0; i < s.n; ++i) {
+      s.alpha[i] = coef[2 * (k + i)];
+      s.s[i] = coef[2 * (k + i) + 1];
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gs_chain<P>, gs_mesh(mesh, geo, ncell), s, cB, cgg, g, WA, pg, ptr,
+                                             z, d, x, dtr, words, words + gs_words(ncell), 2 * k, k + s.n < n ? 1 : 0);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 cudaError_t gs_binv(const MeshDev& mesh, const float* geo, const float* d, const float* dtr, float cB, const float* WA,
                     const float* pg, const float* ptr, float cgg, float* fx, float* fe, float* gf, int ncell,
@@ -1124,7 +1163,8 @@ const DegreeOps kOps = {upload_tables,     rhs,
                         res_chebz_f,       gs_geo,
                         gs_entry,          gs_binv,
                         gs_zstep,          gs_exit,
-                        gs_values};
+                        gs_values,         gs_chain_tiles,
+                        gs_chain};
 
 }  // namespace
 

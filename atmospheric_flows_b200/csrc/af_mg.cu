@@ -165,6 +165,7 @@ struct Level {
   // d, face fluxes of w, p_fixed at the Gauss points and its x-face traces, inverse weights of A; its
   // fields d, x, z and the fluxes of w use the vectors above (allocated for whole tiles)
   float *ggeo = nullptr, *gdtr = nullptr, *gwf = nullptr, *gpg = nullptr, *gptr = nullptr, *gWA = nullptr;
+  unsigned long long* gwords = nullptr;  // face words of gs_chain, where all tiles fit on the device at once
   double lmax = 0.0;
 };
 
@@ -488,21 +489,37 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
   float* x = (float*)L.x;
   float *fx = (float*)L.w, *fe = fx + gs_padded(L.ncell, o->nd);
   // d = x = D^{-1} v / theta;  z = D^{-1} v = theta d
-  MG_CU(k->gs_entry(L.mesh, L.ggeo, v, (float)(ginv / theta), (float)theta, zg, d, x, L.gdtr, L.ncell, o->stream));
+  MG_CU(k->gs_entry(L.mesh, L.ggeo, v, (float)(ginv / theta), (float)theta, zg, d, x, L.gdtr, L.gwords, L.ncell,
+                    o->stream));
   o->launches += 1;
   double rho_old = 1.0 / sigma;
   const int last = s->opt.coarse_degree - 1;
+  std::vector<float> coef(2 * last);  // (a, sc) of the steps
   for (int it = 1; it <= last; ++it) {
     const double rho = 1.0 / (2.0 * sigma - rho_old);
-    const double a = rho * rho_old, sc = 2.0 * rho / delta;
+    coef[2 * it - 2] = (float)(rho * rho_old);
+    coef[2 * it - 1] = (float)(2.0 * rho / delta);
+    rho_old = rho;
+  }
+  bool chained = false;
+  if (L.gwords && last > 0) {  // all steps in one launch
+    MeshDev mesh = L.mesh;
+    mesh.test_wait_polls = o->mesh.test_wait_polls;
+    const cudaError_t e = k->gs_chain(mesh, L.ggeo, coef.data(), last, (float)s->cB, (float)(s->cdt * kGG), (float)ginv,
+                                      L.gWA, L.gpg, L.gptr, zg, d, x, L.gdtr, L.gwords, L.ncell, o->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();  // part of the device only: step by step
+    else if (e != cudaSuccess) MG_CU(e);
+    chained = e == cudaSuccess;
+    o->launches += 1;
+  }
+  for (int it = 1; it <= last && !chained; ++it) {
     // w = A^{-1} B d;  z += D^{-1} C0 w - d;  d = a d + sc z;  x += d (two launches; x takes the
     // directions of an odd step and the next one together)
     MG_CU(k->gs_binv(L.mesh, L.ggeo, d, L.gdtr, (float)s->cB, L.gWA, L.gpg, L.gptr, (float)(s->cdt * kGG), fx, fe,
                      L.gwf, L.ncell, o->stream));
-    MG_CU(k->gs_zstep(L.mesh, L.ggeo, fx, fe, L.gwf, (float)ginv, (float)a, (float)sc, zg, d, x,
+    MG_CU(k->gs_zstep(L.mesh, L.ggeo, fx, fe, L.gwf, (float)ginv, coef[2 * it - 2], coef[2 * it - 1], zg, d, x,
                       it % 2 == 0 ? 1 : (it == last ? 2 : 0), L.gdtr, L.ncell, o->stream));
     o->launches += 2;
-    rho_old = rho;
   }
   MG_CU(k->gs_exit(x, z, L.ncell, o->stream));
   o->launches += 1;
@@ -648,6 +665,11 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
         if ((r = alloc(s, (void**)p, sizeof(float) * nt)) != AF_OK) return cleanup(r);
       for (float** p : {&L.gpg, &L.gWA})
         if ((r = alloc(s, (void**)p, sizeof(float) * nv)) != AF_OK) return cleanup(r);
+      // every step in one launch where the tiles are resident together (k_gs_chain)
+      const int tiles = (int)(cells / 32);
+      if (tiles <= op->ops->gs_chain_tiles(op->device) &&
+          (r = alloc(s, (void**)&L.gwords, sizeof(*L.gwords) * 2 * nt)) != AF_OK)
+        return cleanup(r);
       if (op->ops->gs_geo(L.mesh, L.ggeo, L.ncell, op->stream) != cudaSuccess)
         return cleanup(merr(AF_CUDA, "af_schur_solver_create: geometry block"));
       op->launches += 1;

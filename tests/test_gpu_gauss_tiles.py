@@ -58,3 +58,48 @@ def test_overlapping_applications_repeat(P):
     torch.cuda.synchronize()
     for o in out[1:]:
         assert torch.equal(o, out[0])
+
+
+def both(nx, nz, P, per, degree, dt):
+    z = {}
+    for rq in (1, 2):
+        s, n = setup(nx, nz, P, per, degree, rq, dt)
+        b = torch.from_numpy(np.random.default_rng(5).standard_normal(n)).cuda()
+        z[rq] = torch.zeros_like(b)
+        s.precondition(z[rq], b)
+        torch.cuda.synchronize()
+    return z[2].cpu().numpy(), z[1].cpu().numpy()
+
+
+# more tiles than the device holds at once (148 SMs, 5 to 12 CTAs each): a launch per half step; the same
+# Courant number, hence condition, as the 16x8 mesh above, and the tolerance of up to five steps
+@pytest.mark.parametrize("P,nx,nz", [(1, 301, 200), (2, 199, 201), (3, 161, 150), (4, 141, 137), (5, 121, 119), (6, 99, 97)])
+def test_smoother_of_large_meshes(P, nx, nz):
+    got, want = both(nx, nz, P, True, 5, 0.5 * min(16 / nx, 8 / nz))
+    assert rel(got, want) < 2e-5
+
+
+# one launch takes 64 steps: 64, 65 and 129 steps; rounding grows with their number (2e-5 for five)
+@pytest.mark.parametrize("P", [1, 4, 6])
+@pytest.mark.parametrize("degree", [65, 66, 130])
+def test_many_steps(P, degree):
+    got, want = both(21, 5, P, True, degree, 0.5)
+    assert rel(got, want) < 2e-5 * degree / 5
+
+
+def test_waits_between_tiles_are_bounded():
+    from atmospheric_flows_b200.operator import AF_TIMEOUT, AFError
+    s, n = setup(20, 11, 4, True, 8, 2)
+    b = torch.from_numpy(np.random.default_rng(5).standard_normal(n)).cuda()
+    want, got = torch.zeros_like(b), torch.zeros_like(b)
+    s.precondition(want, b)
+    s.op.synchronize()
+    s.op.set_stage_wait_test(64)
+    s.precondition(got, b)
+    with pytest.raises(AFError) as e:
+        s.op.synchronize()
+    assert e.value.status == AF_TIMEOUT
+    s.op.set_stage_wait_test(0)
+    s.precondition(got, b)
+    s.op.synchronize()
+    assert torch.equal(got, want)
