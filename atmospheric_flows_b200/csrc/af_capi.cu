@@ -210,7 +210,7 @@ int af_create(const af_mesh_desc* m, int degree, int nq, double Ma, double Fr, d
 }
 
 int af_destroy(af_operator* o) {
-  if (!o) return AF_OK;
+  if (!o || --o->refs > 0) return AF_OK;
   cudaSetDevice(o->device);
   if (o->stream) cudaStreamSynchronize(o->stream);
   cudaFree(o->d_vtx);

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "af_blas.h"
 #include "af_internal.h"
 
@@ -12,6 +14,9 @@ using af::DegreeOps;
 
 struct af_operator {
   int device = 0;
+  // the handle and the solvers on it; the last one to be destroyed frees it (a garbage collector
+  // finalises them in any order)
+  std::atomic<int> refs{1};
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int P = 0, NQ = 0, ncell = 0, nd = 0;
   MeshDev mesh{};

@@ -594,6 +594,7 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
   MG_CU(cudaSetDevice(op->device));
   auto* s = new af_schur_solver();
   s->op = op;
+  ++op->refs;
   s->opt = o;
   s->fp32 = o.preconditioner == AF_SCHUR_MG_FP32 || o.preconditioner == AF_SCHUR_CHEB_FP32;
   s->rq = s->fp32 && o.reduced_quadrature != 0;
@@ -689,8 +690,9 @@ int af_schur_solver_destroy(af_schur_solver* s) {
   for (void* p : s->owned) cudaFree(p);
   for (cudaEvent_t e : s->ev)
     if (e) cudaEventDestroy(e);
+  af_operator* op = s->op;
   delete s;
-  return AF_OK;
+  return af_destroy(op);
 }
 
 int af_schur_solver_setup(af_schur_solver* s, int estimate_eigenvalues) {

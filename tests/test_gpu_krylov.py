@@ -54,3 +54,27 @@ def test_solves_for_every_restart(nx, nz, P):
     assert len(xs) >= 4
     for x in xs:
         assert rel(x, xs[-1]) < 1e-8
+
+
+def test_operator_destroyed_before_its_solver():
+    """A garbage collector finalises an operator and its solver in any order."""
+    from atmospheric_flows_b200.operator import EULEROperator
+    from atmospheric_flows_b200.schur import SchurSolver
+    sc = M.Scaling()
+    m = M.hill_mesh(8, 4)
+    st = M.hill_state(m, 2, modes=4)
+    op = EULEROperator(m, 2, sc.Ma, sc.Fr, 0.25)
+    op.set_HYPERBOLIC_stage(1)
+    op.set_rho_for_fixed(torch.from_numpy(st.rho).cuda())
+    op.set_pres_fixed(torch.from_numpy(st.p).cuda())
+    s = SchurSolver(op, "cheb_fp32")
+    s.setup()
+    b = torch.ones(op.n_dofs(1), dtype=torch.float64, device="cuda")
+    want, got = torch.zeros_like(b), torch.zeros_like(b)
+    s.precondition(want, b)
+    torch.cuda.synchronize()
+    op.__del__()
+    s.precondition(got, b)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    s.__del__()
