@@ -24,7 +24,7 @@
 //
 // What bounds it and why this split (FP64, degree 4, 512x256 cells, fused stage-1 right-hand sides):
 // FP64 issue (68 M warp instructions, a 110 us floor at the pipe's rate, against 44 us of HBM
-// traffic) and the shared-memory data path (41 M wavefronts).  402 us before this layout, 206 us with
+// traffic) and the shared-memory data path (39 M wavefronts).  402 us before this layout, 206 us with
 // it.  What gave that:
 // - 14 cells x 9 points fill 4 warps and three such CTAs an SM (168 registers, 74 KB); 16 cells left
 //   half a warp idle and two CTAs an SM;
@@ -247,6 +247,8 @@ __device__ __forceinline__ void report_status(int* status, int code) {
 //   p=4  14 x 3: 207, 481, 911, 82;  12 x 3: 229, 545, 1007, 91;  10 x 4: 221, 548, 1000, 87;  6 x 6: 232, 557, 1088, 101
 //   p=5 (65536 cells)  11 x 2: 227, 515, 928, 66;  8 x 3: 217, 483, 825, 68 (stage 2 430, not 412);  5 x 4: 224, 545, 978, 67
 //   p=6 (32768 cells)  8 x 2: 152, 327, 561, 44;  4 x 4: 151, 332, 587, 47
+// Meshes of less than about two CTAs per SM take 10 percent more or less with the remainder of that count
+// (p=3, 91x32 cells, split stage 1: 9 cells 30, 10 cells 28, 18 cells 34; 40x16: 20, 25, 26).
 // An odd number of cells needs an even number of nodes a cell: the bulk copies start on 16 bytes.
 template <int P, class R = double>
 constexpr int cells_per_block() {

@@ -38,7 +38,7 @@ struct DegreeOps {
   cudaError_t (*inv_diag)(const MeshDev&, int ncomp, const double* weight, double scale, double* dst, int ncell,
                           cudaStream_t);
   // packed inverses (lower triangle) of the cell mass matrices (weight null: plain mass),
-  // stored interleaved L[k * ncell + c], factor_len() doubles per cell
+  // one cell after another, factor_len doubles each
   cudaError_t (*mass_factor)(const MeshDev&, const double* weight, double* L, int ncell, cudaStream_t);
   // x = scale * M^{-1} b (block diagonal, exact), ncomp components per cell
   cudaError_t (*mass_solve)(const double* L, int ncomp, const double* b, double scale, double* x, int ncell,
