@@ -29,7 +29,12 @@
 // is no index arithmetic per element, the column's work stays in registers, the tables are indexed
 // by warp-uniform values, and only the contraction along x passes through shared memory (cell
 // fastest: no bank conflicts).  The edge vectors of a face serve as its normal (the fluxes are
-// linear in it), so a cell's geometry is six floats, formed once per mesh.
+// linear in it).  Geometry is formed once per mesh, in FP64 from the vertices: the four edges of a cell,
+// each rounded once, so that both sides of a face take the same bits for its normal (between opposite
+// edges the map's derivatives are interpolated), and the determinant as three doubles.  On a bilinear
+// cell it is affine, d0 + d1 xi + d2 eta (the product of the map's bilinear term with itself vanishes),
+// so JxW at a point takes two FP64 operations and one rounding; products formed in FP32 cancel on sheared
+// cells.
 //
 // The kernels pass between them what the next one needs and no more: k_gs_binv does not write w but
 // the two mapped fluxes of C0 at the points (p_f w contracted with adj(J)) and one value per face
@@ -49,11 +54,10 @@
 #pragma once
 
 #include "af_cellop.cuh"
+#include "af_internal.h"
 
 namespace af {
 
-constexpr int kGsTile = 32;  // cells per tile (one warp of lanes)
-constexpr int kGsGeo = 6;    // floats per cell: A, C, B of the bilinear map x = v0 + A xi + C eta + B xi eta
 
 // n / d for 0 <= n < 2^31 by one multiplication (Granlund and Montgomery, "Division by invariant
 // integers using multiplication", 1994): m = floor(2^(31+l) / d) + 1, l = ceil(log2 d)
@@ -69,7 +73,8 @@ struct FastDiv {
 };
 
 struct GsMesh {
-  const float* geo;  // [tile][kGsGeo][32]
+  const float* geo;   // [tile][kGsGeo][32]
+  const double* det;  // [tile][kGsDet][32]
   FastDiv nx;
   int nz, periodic_x, ncell;
   int* status;          // as in MeshDev
@@ -108,7 +113,8 @@ template <int P>
 struct GsThread {
   int lane, m, tile, c;
   bool live;
-  float Ax, Az, Cx, Cz, Bx, Bz;
+  float Ax, Az, Cx, Cz, Rx, Rz, Tx, Tz;  // edges of the faces eta = 0, xi = 0, xi = 1, eta = 1
+  float Bx, Bz, Dx, Dz;                  // R - C, T - A
   int nb[4];
   __device__ __forceinline__ explicit GsThread(const GsMesh& g) {
     lane = threadIdx.x & 31;
@@ -119,7 +125,8 @@ struct GsThread {
   }
   __device__ __forceinline__ void geometry(const GsMesh& g) {
     const float* s = g.geo + (size_t)tile * kGsGeo * kGsTile + lane;
-    Ax = s[0]; Az = s[kGsTile]; Cx = s[2 * kGsTile]; Cz = s[3 * kGsTile]; Bx = s[4 * kGsTile]; Bz = s[5 * kGsTile];
+    Ax = s[0]; Az = s[kGsTile]; Cx = s[2 * kGsTile]; Cz = s[3 * kGsTile]; Rx = s[4 * kGsTile]; Rz = s[5 * kGsTile]; Tx = s[6 * kGsTile]; Tz = s[7 * kGsTile];
+    Bx = Rx - Cx; Bz = Rz - Cz; Dx = Tx - Ax; Dz = Tz - Az;
   }
   __device__ __forceinline__ void neighbours(const GsMesh& g) {  // -1: wall (and past the last cell)
     const int nx = g.nx.d, j = g.nx.div(c), i = c - j * nx;
@@ -132,12 +139,12 @@ struct GsThread {
   }
   __device__ __forceinline__ float J01(float xi) const { return fmaf(Bx, xi, Cx); }
   __device__ __forceinline__ float J11(float xi) const { return fmaf(Bz, xi, Cz); }
-  __device__ __forceinline__ float J00(float eta) const { return fmaf(Bx, eta, Ax); }
-  __device__ __forceinline__ float J10(float eta) const { return fmaf(Bz, eta, Az); }
+  __device__ __forceinline__ float J00(float eta) const { return fmaf(Dx, eta, Ax); }
+  __device__ __forceinline__ float J10(float eta) const { return fmaf(Dz, eta, Az); }
   // outward normal times length of face f: (-tz, tx) of the edge on faces 0 and 3, (tz, -tx) on 1, 2
   __device__ __forceinline__ void normal(int f, float& n0, float& n1) const {
-    const float tx = f == 0 ? Cx : (f == 1 ? Cx + Bx : (f == 2 ? Ax : Ax + Bx));
-    const float tz = f == 0 ? Cz : (f == 1 ? Cz + Bz : (f == 2 ? Az : Az + Bz));
+    const float tx = f == 0 ? Cx : (f == 1 ? Rx : (f == 2 ? Ax : Tx));
+    const float tz = f == 0 ? Cz : (f == 1 ? Rz : (f == 2 ? Az : Tz));
     const float s = (f == 0 || f == 3) ? 1.f : -1.f;
     n0 = -s * tz;
     n1 = s * tx;
@@ -172,21 +179,46 @@ __device__ __forceinline__ void gs_row_ends(const float* s, int m, int lane, flo
   gs_ends<P>(row, lo, hi);
 }
 
-// the geometry block of a mesh
-static __global__ void k_gs_geo(const MeshDev mesh, float* __restrict__ geo, const int ncell) {
+// the geometry block of a mesh (thread = cell)
+static __global__ void k_gs_geo(const MeshDev mesh, float* __restrict__ geo, double* __restrict__ det, const int ncell) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (ncell + kGsTile - 1) / kGsTile * kGsTile) return;
   const int c = min(e, ncell - 1), i = c % mesh.nx, j = c / mesh.nx, W = mesh.nx + 1;
   const double2* v = mesh.vtx + (size_t)j * W + i;
   const double2 v0 = v[0], v1 = v[1], v2 = v[W], v3 = v[W + 1];
+  const double G[kGsGeo] = {v1.x - v0.x, v1.y - v0.y, v2.x - v0.x, v2.y - v0.y,
+                            v3.x - v1.x, v3.y - v1.y, v3.x - v2.x, v3.y - v2.y};
+  const double Bx = v3.x - v2.x - v1.x + v0.x, Bz = v3.y - v2.y - v1.y + v0.y;
   float* g = geo + (size_t)(e / kGsTile) * kGsGeo * kGsTile + e % kGsTile;
-  g[0] = (float)(v1.x - v0.x);
-  g[kGsTile] = (float)(v1.y - v0.y);
-  g[2 * kGsTile] = (float)(v2.x - v0.x);
-  g[3 * kGsTile] = (float)(v2.y - v0.y);
-  g[4 * kGsTile] = (float)(v3.x - v2.x - v1.x + v0.x);
-  g[5 * kGsTile] = (float)(v3.y - v2.y - v1.y + v0.y);
+#pragma unroll
+  for (int k = 0; k < kGsGeo; ++k) g[k * kGsTile] = (float)G[k];
+  double* d = det + (size_t)(e / kGsTile) * kGsDet * kGsTile + e % kGsTile;
+  d[0] = G[0] * G[3] - G[2] * G[1];
+  d[kGsTile] = G[0] * Bz - Bx * G[1];      // A x B
+  d[2 * kGsTile] = Bx * G[3] - G[2] * Bz;  // B x C
 }
+
+// JxW at the points of column m of the thread's cell, and its inverse (one Newton step from the
+// approximate quotient: FP32 rounding)
+template <int P>
+struct GsJxW {
+  double dx, dz;
+  __device__ __forceinline__ GsJxW(const GsMesh& g, const GsThread<P>& th) {
+    const CobT<P, double>& cb = cobr<P, double>();
+    const double* d = g.det + (size_t)th.tile * kGsDet * kGsTile + th.lane;
+    const double wx = cb.w[th.m];
+    dx = wx * fma(d[kGsTile], cb.g[th.m], d[0]);
+    dz = wx * d[2 * kGsTile];
+  }
+  __device__ __forceinline__ float inv(int q) const {
+    const float a = (*this)(q), r = __fdividef(1.f, a);
+    return fmaf(r, fmaf(-a, r, 1.f), r);
+  }
+  __device__ __forceinline__ float operator()(int q) const {
+    const CobT<P, double>& cb = cobr<P, double>();
+    return (float)(fma(dz, cb.g[q], dx) * cb.w[q]);
+  }
+};
 
 // ------------------------------------------- w = A^{-1} B d, handed on as the fluxes of C0 w
 // d_g and its traces dtr -> w_g = diag(WA) B_g d_g, then at the points the mapped fluxes of C0,
@@ -340,11 +372,11 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
   pdl_allow_next();
   const CobT<P, float>& cb = cobr<P, float>();
   GsThread<P> th(mesh);
-  th.geometry(mesh);
   th.neighbours(mesh);
   const int lane = th.lane, m = th.m;
-  pdl_wait_previous();
   const size_t oc = S::column(th.tile, m, lane), op = S::point(th.tile, m, lane);
+  const GsJxW<P> jxw(mesh, th);
+  pdl_wait_previous();
   const float *fxB = fx + oc, *feB = fe + oc, *gB = gf + op;
   float *zB = z + oc, *dB = d + oc, *xB = x + oc, *tB = dtr + op;
   float ec[P1], zc[P1], dc[P1], xc[P1], F[4];
@@ -375,7 +407,6 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
   }
   __syncthreads();
   const float lo = cb.lo[m], hi = cb.hi[m];
-  const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]), gw = 1.f / cb.w[m];
 #pragma unroll
   for (int i = 0; i < P1; ++i) {
     float y = a[i];
@@ -383,8 +414,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
     for (int q = 0; q < P1; ++q) y = fmaf(cb.Dg[q][m], s_fx[(i * P1 + q) * kGsTile + lane], y);
     y = fmaf(lo, s_xf[i * kGsTile + lane], y);
     y = fmaf(hi, s_xf[(P1 + i) * kGsTile + lane], y);
-    const float det = th.J00(cb.g[i]) * J11 - th.J10(cb.g[i]) * J01;
-    const float zn = zc[i] + __fdividef(gfac * gw * y, det * cb.w[i]) - dc[i];
+    const float zn = zc[i] + gfac * y * jxw.inv(i) - dc[i];
     const float nd = alpha * dc[i] + s * zn;
     zB[i * S::SN] = zn;
     dB[i * S::SN] = nd;
@@ -435,6 +465,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   __shared__ float s_xf[4 * P1 * kGsTile];  // x-face fluxes of B [face][component][point][lane]
   __shared__ float s_w[2 * ND * kGsTile];   // w [component][node][lane]
   __shared__ float s_fx[ND * kGsTile], s_d[ND * kGsTile], s_xf2[2 * P1 * kGsTile];
+  __shared__ float s_wm[ND * kGsTile];      // g / JxW; each thread reads its own column
   const CobT<P, float>& cb = cobr<P, float>();
   GsThread<P> th(mesh);
   th.geometry(mesh);
@@ -486,8 +517,11 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
     return ok;
   };
 
-  const float wx = cb.w[m], lo = cb.lo[m], hi = cb.hi[m], gw = 1.f / cb.w[m];
+  const float wx = cb.w[m], lo = cb.lo[m], hi = cb.hi[m];
   const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]);
+  const GsJxW<P> jxw(mesh, th);
+#pragma unroll
+  for (int q = 0; q < P1; ++q) s_wm[(q * P1 + m) * kGsTile + lane] = gfac * jxw.inv(q);
 #pragma unroll
   for (int q = 0; q < P1; ++q) s_sw[(q * P1 + m) * kGsTile + lane] = -cB * dc[q] * (wx * cb.w[q]);
   __syncthreads();
@@ -599,8 +633,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
       float y = a[i];
       y = fmaf(lo, s_xf2[i * kGsTile + lane], y);
       y = fmaf(hi, s_xf2[(P1 + i) * kGsTile + lane], y);
-      const float det = th.J00(cb.g[i]) * J11 - th.J10(cb.g[i]) * J01;
-      const float zn = zc[i] + __fdividef(gfac * gw * y, det * cb.w[i]) - dc[i];
+      const float zn = zc[i] + s_wm[(i * P1 + m) * kGsTile + lane] * y - dc[i];
       const float nd = alpha * dc[i] + s * zn;
       if (it % 2 == 0) xc[i] = (xc[i] + dc[i]) + nd;
       else if (it == st.n) xc[i] = xc[i] + nd;
@@ -642,11 +675,11 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
   pdl_allow_next();
   const CobT<P, float>& cb = cobr<P, float>();
   GsThread<P> th(mesh);
-  th.geometry(mesh);
   const int lane = th.lane, m = th.m;
   const int n = min(kGsTile, mesh.ncell - th.tile * kGsTile) * ND;
   const size_t oc = S::column(th.tile, m, lane);
   float *zB = z + oc, *dB = d + oc, *xB = x + oc, *tB = dtr + S::point(th.tile, m, lane);
+  const GsJxW<P> jxw(mesh, th);
   pdl_wait_previous();
   for (int e = threadIdx.x; e < n; e += S::NT) s_v[(e / ND) * NDS + e % ND] = (float)v[(size_t)th.tile * kGsTile * ND + e];
   __syncthreads();
@@ -662,14 +695,12 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
 #pragma unroll
   for (int i = 0; i < P1; ++i) u[i] = s_t[(i * P1 + m) * kGsTile + lane];
   __syncthreads();
-  const float J01 = th.J01(cb.g[m]), J11 = th.J11(cb.g[m]);
 #pragma unroll
   for (int q = 0; q < P1; ++q) {  // along z on column m, then the weights
     float b = 0.f;
 #pragma unroll
     for (int i = 0; i < P1; ++i) b = fmaf(cb.Vi[i][q], u[i], b);
-    const float det = th.J00(cb.g[q]) * J11 - th.J10(cb.g[q]) * J01;
-    dc[q] = __fdividef(sc * b, det * (cb.w[m] * cb.w[q]));
+    dc[q] = sc * b * jxw.inv(q);
     dB[q * S::SN] = dc[q];
     xB[q * S::SN] = dc[q];
     zB[q * S::SN] = theta * dc[q];

@@ -23,6 +23,15 @@ struct RhsSources {
   const double* u_fix;  // u_fixed / u_curr
 };
 
+// the tiles and the geometry blocks of the Gauss-point smoother (af_gauss.cuh)
+constexpr int kGsTile = 32;  // cells per tile (one warp of lanes)
+constexpr int kGsGeo = 8;    // floats per cell: the edges of the faces eta = 0 (A), xi = 0 (C), xi = 1, eta = 1
+constexpr int kGsDet = 3;    // doubles per cell: the determinant d0 + d1 xi + d2 eta
+struct GsGeo {
+  float* map = nullptr;
+  double* det = nullptr;
+};
+
 struct DegreeOps {
   cudaError_t (*upload_tables)();
   cudaError_t (*rhs)(const MeshDev&, int stage, int mask, const RhsSources&, const RhsParams&, double* out_rho,
@@ -130,20 +139,20 @@ struct DegreeOps {
                              const CParamsT<float>&, const float* WM, float g, float alpha, float s, float* z,
                              float* dout, float* x, int first, int reduced, int ncell, cudaStream_t);
   // ---- the same smoother in the Gauss-point basis (af_gauss.cuh): fields and face arrays in its
-  // layout, tiled by gs_tile cells; geo: the mesh's geometry block (kGsGeo floats per cell)
-  cudaError_t (*gs_geo)(const MeshDev&, float* geo, int ncell, cudaStream_t);
+  // layout, tiled by gs_tile cells; geo: the mesh's geometry blocks
+  cudaError_t (*gs_geo)(const MeshDev&, GsGeo geo, int ncell, cudaStream_t);
   //   entry: d = x = sc (Vi x Vi)^T v / JxW (v FP64 nodal), z = theta d, dtr = traces of d; words (may
   //   be null): the face words of gs_chain, 8 (P + 1) per cell of whole tiles
-  cudaError_t (*gs_entry)(const MeshDev&, const float* geo, const double* v, float sc, float theta, float* z, float* d,
+  cudaError_t (*gs_entry)(const MeshDev&, const GsGeo& geo, const double* v, float sc, float theta, float* z, float* d,
                           float* x, float* dtr, unsigned long long* words, int ncell, cudaStream_t);
   //   w = diag(WA) B_g d, written as the mapped fluxes of C0 w at the points (fx, fe) and on the
   //   faces (gf); pg, ptr: p_fixed at the points and on the x-faces; cgg = cdt gamma/(gamma-1)
-  cudaError_t (*gs_binv)(const MeshDev&, const float* geo, const float* d, const float* dtr, float cB, const float* WA,
+  cudaError_t (*gs_binv)(const MeshDev&, const GsGeo& geo, const float* d, const float* dtr, float cB, const float* WA,
                          const float* pg, const float* ptr, float cgg, float* fx, float* fe, float* gf, int ncell,
                          cudaStream_t);
   //   z += g C0_g w / JxW - d;  d = alpha d + s z (in place);  x += 0, d_old + d, d (xmode 0, 1, 2);
   //   dtr = traces of d
-  cudaError_t (*gs_zstep)(const MeshDev&, const float* geo, const float* fx, const float* fe, const float* gf, float g,
+  cudaError_t (*gs_zstep)(const MeshDev&, const GsGeo& geo, const float* fx, const float* fe, const float* gf, float g,
                           float alpha, float s, float* z, float* d, float* x, int xmode, float* dtr, int ncell,
                           cudaStream_t);
   //   out = (Vi x Vi) x (FP64 nodal)
@@ -155,7 +164,7 @@ struct DegreeOps {
   int (*gs_chain_tiles)(int device);
   //   n pairs (gs_binv, gs_zstep) with (alpha, s) = coef[2 i], coef[2 i + 1], after gs_entry with the
   //   same words; d, z and dtr are left in between
-  cudaError_t (*gs_chain)(const MeshDev&, const float* geo, const float* coef, int n, float cB, float cgg, float g,
+  cudaError_t (*gs_chain)(const MeshDev&, const GsGeo& geo, const float* coef, int n, float cB, float cgg, float g,
                           const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x, float* dtr,
                           unsigned long long* words, int ncell, cudaStream_t);
 };

@@ -1041,16 +1041,16 @@ cudaError_t launch_gs(K kernel, int ncell, cudaStream_t st, bool pdl, A... args)
   cfg.numAttrs = (kPDL && pdl) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
-GsMesh gs_mesh(const MeshDev& m, const float* geo, int ncell) {
-  return {geo, FastDiv::make(m.nx), m.nz, m.periodic_x, ncell, m.status, m.test_wait_polls};
+GsMesh gs_mesh(const MeshDev& m, const GsGeo& geo, int ncell) {
+  return {geo.map, geo.det, FastDiv::make(m.nx), m.nz, m.periodic_x, ncell, m.status, m.test_wait_polls};
 }
 // words of one of the two face arrays of k_gs_chain
 size_t gs_words(int ncell) { return (size_t)(ncell + kGsTile - 1) / kGsTile * kGsTile * 4 * (P + 1); }
-cudaError_t gs_geo(const MeshDev& mesh, float* geo, int ncell, cudaStream_t st) {
-  k_gs_geo<<<(ncell + 255) / 256, 256, 0, st>>>(mesh, geo, ncell);
+cudaError_t gs_geo(const MeshDev& mesh, GsGeo geo, int ncell, cudaStream_t st) {
+  k_gs_geo<<<(ncell + 255) / 256, 256, 0, st>>>(mesh, geo.map, geo.det, ncell);
   return cudaGetLastError();
 }
-cudaError_t gs_entry(const MeshDev& mesh, const float* geo, const double* v, float sc, float theta, float* z, float* d,
+cudaError_t gs_entry(const MeshDev& mesh, const GsGeo& geo, const double* v, float sc, float theta, float* z, float* d,
                      float* x, float* dtr, unsigned long long* words, int ncell, cudaStream_t st) {
   return launch_gs(k_gs_entry<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), v, sc, theta, z, d, x, dtr, words,
                    words ? words + gs_words(ncell) : nullptr);
@@ -1065,7 +1065,7 @@ int gs_chain_tiles(int device) {
   }
   return coop ? sms * per : 0;
 }
-cudaError_t gs_chain(const MeshDev& mesh, const float* geo, const float* coef, int n, float cB, float cgg, float g,
+cudaError_t gs_chain(const MeshDev& mesh, const GsGeo& geo, const float* coef, int n, float cB, float cgg, float g,
                      const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x, float* dtr,
                      unsigned long long* words, int ncell, cudaStream_t st) {
   if (ncell <= 0) return cudaSuccess;
@@ -1091,12 +1091,12 @@ cudaError_t gs_chain(const MeshDev& mesh, const float* geo, const float* coef, i
   }
   return cudaSuccess;
 }
-cudaError_t gs_binv(const MeshDev& mesh, const float* geo, const float* d, const float* dtr, float cB, const float* WA,
+cudaError_t gs_binv(const MeshDev& mesh, const GsGeo& geo, const float* d, const float* dtr, float cB, const float* WA,
                     const float* pg, const float* ptr, float cgg, float* fx, float* fe, float* gf, int ncell,
                     cudaStream_t st) {
   return launch_gs(k_gs_binv<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), d, dtr, cB, WA, pg, ptr, cgg, fx, fe, gf);
 }
-cudaError_t gs_zstep(const MeshDev& mesh, const float* geo, const float* fx, const float* fe, const float* gf, float g,
+cudaError_t gs_zstep(const MeshDev& mesh, const GsGeo& geo, const float* fx, const float* fe, const float* gf, float g,
                      float alpha, float s, float* z, float* d, float* x, int xmode, float* dtr, int ncell,
                      cudaStream_t st) {
   return launch_gs(k_gs_zstep<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), fx, fe, gf, g, alpha, s, z, d, x, xmode,

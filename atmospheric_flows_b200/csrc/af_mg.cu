@@ -161,10 +161,11 @@ struct Level {
   void* LA = nullptr;
   void* LM = nullptr;
   void *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *u = nullptr, *w = nullptr;
-  // the Gauss-point smoother (af_gauss.cuh), in its tiled layout: the geometry block, face traces of
-  // d, face fluxes of w, p_fixed at the Gauss points and its x-face traces, inverse weights of A; its
+  // the Gauss-point smoother (af_gauss.cuh), in its tiled layout: the geometry blocks, face traces
+  // of d, face fluxes of w, p_fixed at the Gauss points and its x-face traces, inverse weights of A; its
   // fields d, x, z and the fluxes of w use the vectors above (allocated for whole tiles)
-  float *ggeo = nullptr, *gdtr = nullptr, *gwf = nullptr, *gpg = nullptr, *gptr = nullptr, *gWA = nullptr;
+  GsGeo ggeo;
+  float *gdtr = nullptr, *gwf = nullptr, *gpg = nullptr, *gptr = nullptr, *gWA = nullptr;
   unsigned long long* gwords = nullptr;  // face words of gs_chain, where all tiles fit on the device at once
   double lmax = 0.0;
 };
@@ -471,8 +472,8 @@ int build_mass_inverses(af_schur_solver* s) {
   return AF_OK;
 }
 
-// elements of a field of the Gauss-point smoother: whole tiles of 32 cells
-size_t gs_padded(int ncell, int nd) { return (size_t)(ncell + 31) / 32 * 32 * nd; }
+// elements of a field of the Gauss-point smoother: whole tiles
+size_t gs_padded(int ncell, int nd) { return (size_t)(ncell + kGsTile - 1) / kGsTile * kGsTile * nd; }
 
 // z = the single-level FP32 Chebyshev polynomial in the Gauss-point basis applied to v (FP64 in
 // and out): the iteration of chebyshev() on z = D^{-1} r (zero start, no final residual), with
@@ -661,13 +662,14 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
       if ((r = alloc(s, p, rs * 2 * nv)) != AF_OK) return cleanup(r);
     if (s->gauss) {
       const size_t cells = gs_padded(L.ncell, 1), nt = 4 * cells * (op->P + 1);
-      if ((r = alloc(s, (void**)&L.ggeo, sizeof(float) * 6 * cells)) != AF_OK) return cleanup(r);
+      if ((r = alloc(s, (void**)&L.ggeo.map, sizeof(float) * kGsGeo * cells)) != AF_OK) return cleanup(r);
+      if ((r = alloc(s, (void**)&L.ggeo.det, sizeof(double) * kGsDet * cells)) != AF_OK) return cleanup(r);
       for (float** p : {&L.gdtr, &L.gwf, &L.gptr})
         if ((r = alloc(s, (void**)p, sizeof(float) * nt)) != AF_OK) return cleanup(r);
       for (float** p : {&L.gpg, &L.gWA})
         if ((r = alloc(s, (void**)p, sizeof(float) * nv)) != AF_OK) return cleanup(r);
       // every step in one launch where the tiles are resident together (k_gs_chain)
-      const int tiles = (int)(cells / 32);
+      const int tiles = (int)(cells / kGsTile);
       if (tiles <= op->ops->gs_chain_tiles(op->device) &&
           (r = alloc(s, (void**)&L.gwords, sizeof(*L.gwords) * 2 * nt)) != AF_OK)
         return cleanup(r);
