@@ -440,7 +440,8 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
 // meanwhile what its own tile contributes.  A value is overwritten only after the thread that reads it
 // has published its own next one (the threads of a face point read each other's).  k_gs_entry writes
 // the first words and clears the others; counts go on over the launches of one application.  Waits
-// are bounded: a CTA that gives up reports it and leaves, and so do those that wait for it.
+// are bounded: a CTA that gives up reports it, marks the application in *gave_up (cleared by k_gs_entry)
+// and leaves, and so do those that wait for it; k_gs_exit then writes nothing.
 // What bounds it: latency.  Degree-20 polynomial, us, the pairs (one launch per half step) / with
 // flags per tile, fences and barriers / now:
 //   degree 4  256 tiles 123 / 97 / 64, 444 tiles 166 / 106 / 72, 1 tile 99 / 64 / 42;  degree 2, 576 tiles
@@ -458,7 +459,7 @@ template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
     k_gs_chain(const __grid_constant__ GsMesh mesh, const __grid_constant__ GsSteps st, const float cB, const float cgg,
                const float gfac, const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x,
-               float* dtr, GsWord* wd, GsWord* wg, const int base, const int more) {
+               float* dtr, GsWord* wd, GsWord* wg, GsWord* gave_up, const int base, const int more) {
   using S = GsShape<P>;
   constexpr int P1 = S::P1, ND = S::ND;
   __shared__ float s_sw[ND * kGsTile];      // weighted values of -cB d
@@ -466,6 +467,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   __shared__ float s_w[2 * ND * kGsTile];   // w [component][node][lane]
   __shared__ float s_fx[ND * kGsTile], s_d[ND * kGsTile], s_xf2[2 * P1 * kGsTile];
   __shared__ float s_wm[ND * kGsTile];      // g / JxW; each thread reads its own column
+  if (base > 0 && *gave_up) return;  // an earlier launch of this application
   const CobT<P, float>& cb = cobr<P, float>();
   GsThread<P> th(mesh);
   th.geometry(mesh);
@@ -513,7 +515,10 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
       }
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (!ok && lane == 0) report_status(mesh.status, kStatusStageTimeout);
+    if (!ok && lane == 0) {
+      *reinterpret_cast<volatile GsWord*>(gave_up) = 1;
+      report_status(mesh.status, kStatusStageTimeout);
+    }
     return ok;
   };
 
@@ -664,11 +669,12 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
 
 // ------------------------------------------------------------ basis changes
 // The preconditioner's input: v (FP64, a residual: dual, nodal) -> b_g = (Vi x Vi)^T v,
-// d = x = sc b_g / JxW, z = theta d and the traces of d, for k_gs_chain also as words of count 0 (wd; wg cleared).
+// d = x = sc b_g / JxW, z = theta d and the traces of d, for k_gs_chain also as words of count 0 (wd; wg and the
+// mark *gave_up cleared).
 template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT)
     k_gs_entry(const GsMesh mesh, const double* v, const float sc, const float theta,
-               float* z, float* d, float* x, float* dtr, GsWord* wd, GsWord* wg) {
+               float* z, float* d, float* x, float* dtr, GsWord* wd, GsWord* wg, GsWord* gave_up) {
   using S = GsShape<P>;
   constexpr int P1 = S::P1, ND = S::ND, NDS = ND | 1;
   __shared__ float s_v[kGsTile * NDS], s_t[ND * kGsTile];
@@ -719,12 +725,14 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
       wd[o] = gs_word(t[f], 0);
       wg[o] = 0;
     }
+  if (wd && blockIdx.x == 0 && threadIdx.x == 0) *gave_up = 0;
 }
 
-// The preconditioner's output: x = (Vi x Vi) x_g (nodal, FP64).
+// The preconditioner's output: x = (Vi x Vi) x_g (nodal, FP64); nothing when k_gs_chain gave up (gave_up:
+// null where it did not run).
 template <int P>
 __global__ void __launch_bounds__(GsShape<P>::NT)
-    k_gs_exit(const float* xg, double* out, const int ncell) {
+    k_gs_exit(const float* xg, double* out, const GsWord* gave_up, const int ncell) {
   using S = GsShape<P>;
   constexpr int P1 = S::P1, ND = S::ND, NDS = ND | 1;
   __shared__ float s_v[kGsTile * NDS], s_t[ND * kGsTile];
@@ -733,6 +741,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
   const int lane = threadIdx.x & 31, m = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), tile = blockIdx.x;
   const int n = min(kGsTile, ncell - tile * kGsTile) * ND;
   pdl_wait_previous();
+  if (gave_up && *gave_up) return;
   float u[P1];
 #pragma unroll
   for (int q = 0; q < P1; ++q) u[q] = xg[S::column(tile, m, lane) + q * S::SN];

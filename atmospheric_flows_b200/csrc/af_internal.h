@@ -142,7 +142,8 @@ struct DegreeOps {
   // layout, tiled by gs_tile cells; geo: the mesh's geometry blocks
   cudaError_t (*gs_geo)(const MeshDev&, GsGeo geo, int ncell, cudaStream_t);
   //   entry: d = x = sc (Vi x Vi)^T v / JxW (v FP64 nodal), z = theta d, dtr = traces of d; words (may
-  //   be null): the face words of gs_chain, 8 (P + 1) per cell of whole tiles
+  //   be null): the face words of gs_chain, 8 (P + 1) per cell of whole tiles, and one that marks a
+  //   given-up wait
   cudaError_t (*gs_entry)(const MeshDev&, const GsGeo& geo, const double* v, float sc, float theta, float* z, float* d,
                           float* x, float* dtr, unsigned long long* words, int ncell, cudaStream_t);
   //   w = diag(WA) B_g d, written as the mapped fluxes of C0 w at the points (fx, fe) and on the
@@ -155,8 +156,8 @@ struct DegreeOps {
   cudaError_t (*gs_zstep)(const MeshDev&, const GsGeo& geo, const float* fx, const float* fe, const float* gf, float g,
                           float alpha, float s, float* z, float* d, float* x, int xmode, float* dtr, int ncell,
                           cudaStream_t);
-  //   out = (Vi x Vi) x (FP64 nodal)
-  cudaError_t (*gs_exit)(const float* x, double* out, int ncell, cudaStream_t);
+  //   out = (Vi x Vi) x (FP64 nodal); after gs_chain with its words: nothing when a wait was given up
+  cudaError_t (*gs_exit)(const float* x, double* out, const unsigned long long* words, int ncell, cudaStream_t);
   //   the coefficients: pg = (V x V) p, its x-face traces, WA = 1 / (rho JxW)
   cudaError_t (*gs_values)(const MeshDev&, const double* p, const double* rho, float* pg, float* ptr, float* WA,
                            int ncell, cudaStream_t);

@@ -1044,7 +1044,7 @@ cudaError_t launch_gs(K kernel, int ncell, cudaStream_t st, bool pdl, A... args)
 GsMesh gs_mesh(const MeshDev& m, const GsGeo& geo, int ncell) {
   return {geo.map, geo.det, FastDiv::make(m.nx), m.nz, m.periodic_x, ncell, m.status, m.test_wait_polls};
 }
-// words of one of the two face arrays of k_gs_chain
+// words of one of the two face arrays of k_gs_chain (the mark of a given-up wait follows the second)
 size_t gs_words(int ncell) { return (size_t)(ncell + kGsTile - 1) / kGsTile * kGsTile * 4 * (P + 1); }
 cudaError_t gs_geo(const MeshDev& mesh, GsGeo geo, int ncell, cudaStream_t st) {
   k_gs_geo<<<(ncell + 255) / 256, 256, 0, st>>>(mesh, geo.map, geo.det, ncell);
@@ -1053,7 +1053,7 @@ cudaError_t gs_geo(const MeshDev& mesh, GsGeo geo, int ncell, cudaStream_t st) {
 cudaError_t gs_entry(const MeshDev& mesh, const GsGeo& geo, const double* v, float sc, float theta, float* z, float* d,
                      float* x, float* dtr, unsigned long long* words, int ncell, cudaStream_t st) {
   return launch_gs(k_gs_entry<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), v, sc, theta, z, d, x, dtr, words,
-                   words ? words + gs_words(ncell) : nullptr);
+                   words ? words + gs_words(ncell) : nullptr, words ? words + 2 * gs_words(ncell) : nullptr);
 }
 int gs_chain_tiles(int device) {
   int sms = 0, per = 0, coop = 0;
@@ -1086,7 +1086,8 @@ cudaError_t gs_chain(const MeshDev& mesh, const GsGeo& geo, const float* coef, i
       s.s[i] = coef[2 * (k + i) + 1];
     }
     const cudaError_t e = cudaLaunchKernelEx(&cfg, k_gs_chain<P>, gs_mesh(mesh, geo, ncell), s, cB, cgg, g, WA, pg, ptr,
-                                             z, d, x, dtr, words, words + gs_words(ncell), 2 * k, k + s.n < n ? 1 : 0);
+                                             z, d, x, dtr, words, words + gs_words(ncell), words + 2 * gs_words(ncell), 2 * k,
+                                             k + s.n < n ? 1 : 0);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -1102,8 +1103,8 @@ cudaError_t gs_zstep(const MeshDev& mesh, const GsGeo& geo, const float* fx, con
   return launch_gs(k_gs_zstep<P>, ncell, st, true, gs_mesh(mesh, geo, ncell), fx, fe, gf, g, alpha, s, z, d, x, xmode,
                    dtr);
 }
-cudaError_t gs_exit(const float* x, double* out, int ncell, cudaStream_t st) {
-  return launch_gs(k_gs_exit<P>, ncell, st, true, x, out, ncell);
+cudaError_t gs_exit(const float* x, double* out, const unsigned long long* words, int ncell, cudaStream_t st) {
+  return launch_gs(k_gs_exit<P>, ncell, st, true, x, out, words ? words + 2 * gs_words(ncell) : nullptr, ncell);
 }
 cudaError_t gs_values(const MeshDev& mesh, const double* p, const double* rho, float* pg, float* ptr, float* WA,
                       int ncell, cudaStream_t st) {

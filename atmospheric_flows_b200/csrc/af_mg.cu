@@ -522,7 +522,7 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
                       it % 2 == 0 ? 1 : (it == last ? 2 : 0), L.gdtr, L.ncell, o->stream));
     o->launches += 2;
   }
-  MG_CU(k->gs_exit(x, z, L.ncell, o->stream));
+  MG_CU(k->gs_exit(x, z, chained ? L.gwords : nullptr, L.ncell, o->stream));
   o->launches += 1;
   return AF_OK;
 }
@@ -671,7 +671,7 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
       // every step in one launch where the tiles are resident together (k_gs_chain)
       const int tiles = (int)(cells / kGsTile);
       if (tiles <= op->ops->gs_chain_tiles(op->device) &&
-          (r = alloc(s, (void**)&L.gwords, sizeof(*L.gwords) * 2 * nt)) != AF_OK)
+          (r = alloc(s, (void**)&L.gwords, sizeof(*L.gwords) * (2 * nt + 1))) != AF_OK)
         return cleanup(r);
       if (op->ops->gs_geo(L.mesh, L.ggeo, L.ncell, op->stream) != cudaSuccess)
         return cleanup(merr(AF_CUDA, "af_schur_solver_create: geometry block"));

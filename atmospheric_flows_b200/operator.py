@@ -284,7 +284,8 @@ class EULEROperator:
 
     def set_stage_wait_test(self, polls):
         """Test hook: polls > 0 makes the handle's cell kernels give up a bounded wait (before any
-        copy is issued) after that many polls; 0 restores normal operation."""
+        copy is issued), and the one-launch preconditioner a wait for its neighbours, after that many
+        polls; 0 restores normal operation."""
         check(lib().af_set_stage_wait_test(self._h, polls))
 
     def set_schur_mode(self, mode=0, rel_tol=1e-12, max_iter=10000):

@@ -28,10 +28,11 @@ enum {
   AF_NAN = 4,              /* NaN/Inf met in a Krylov recurrence                  */
   AF_UNSUPPORTED = 5,      /* degree not compiled into this library               */
   AF_NO_DEVICE = 6,        /* no CUDA device available                            */
-  AF_TIMEOUT = 7           /* a kernel gave up a bounded wait for its staged
-                              inputs and left its outputs unwritten (reported by
-                              the next call on the handle, or by the call that
-                              synchronizes; see af_synchronize)                    */
+  AF_TIMEOUT = 7           /* a kernel gave up a bounded wait (for its staged
+                              inputs, or for the values of another block) and left
+                              its outputs unwritten (reported by the next call on
+                              the handle, or by the call that synchronizes; see
+                              af_set_stage_wait_test)                              */
 };
 
 typedef struct af_operator af_operator;
@@ -157,14 +158,17 @@ int af_set_sponge(af_operator* op, double z_start, double z_top, double rate_top
                   double width_lateral, double rate_lateral, double u_ref);
 
 /* Failure detection (no counterpart in the reference, whose deal.II loops have no waits):
- * the cell kernels wait for their bulk copies with a bounded number of polls.  A kernel that
- * gives up leaves a code in the handle's status word and returns without writing its
- * outputs; the next call on the handle (any call that queues work, af_synchronize, and every
+ * the cell kernels wait for their bulk copies with a bounded number of polls, and the
+ * one-launch form of the FP32 Chebyshev preconditioner (meshes whose tiles are resident on the
+ * device together) waits for the face values of neighbouring tiles, 2^19 polls at most.  A kernel
+ * that gives up leaves a code in the handle's status word and returns without writing its
+ * outputs (of the one-launch form: the preconditioner's dst); the next call on the handle (any call that queues work, af_synchronize, and every
  * call that synchronizes internally: solves, IMEX steps, host-buffer applies, diagnostics)
  * then returns AF_TIMEOUT once and clears the word.
  * Test hook: polls > 0 makes every cell kernel of this handle first wait on a barrier phase
  * that nothing completes and give up after that many polls, before it issues any copy (the
- * timeout path without copies in flight); 0 restores normal operation. */
+ * timeout path without copies in flight), and the one-launch preconditioner wait that long for a
+ * step that no tile reaches; 0 restores normal operation. */
 int af_set_stage_wait_test(af_operator* op, int polls);
 
 /* ---------------------------------------------------------------- Schur pressure solver

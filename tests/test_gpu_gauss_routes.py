@@ -1,0 +1,50 @@
+"""The two routes of the Gauss-point polynomial: all steps in one cooperative launch (meshes whose tiles
+are resident together) and one launch per half step (the others)."""
+import numpy as np
+import pytest
+
+from atmospheric_flows_b200 import mesh as M
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a - b).norm() / b.norm())
+
+
+def setup(nx, nz, P, per, degree, rq=2, dt=0.5):
+    from atmospheric_flows_b200.operator import EULEROperator
+    from atmospheric_flows_b200.schur import SchurSolver
+    sc = M.Scaling()
+    m = M.hill_mesh(nx, nz, periodic_x=per)
+    op = EULEROperator(m, P, sc.Ma, sc.Fr, dt)
+    op.set_stream(torch.cuda.current_stream())
+    op.set_HYPERBOLIC_stage(1)
+    st = M.hill_state(m, P, modes=4)
+    op.set_rho_for_fixed(torch.from_numpy(st.rho).cuda())
+    op.set_pres_fixed(torch.from_numpy(st.p).cuda())
+    s = SchurSolver(op, "cheb_fp32", poly_degree=degree, reduced_quadrature=rq)
+    s.setup()
+    b = torch.from_numpy(np.random.default_rng(5).standard_normal(m.n_cells * (P + 1) ** 2)).cuda()
+    return s, b
+
+
+@pytest.mark.parametrize("degree", [8, 130])  # one launch; three, of which the first gives up
+def test_given_up_wait_leaves_the_output_unwritten(degree):
+    from atmospheric_flows_b200.operator import AF_TIMEOUT, AFError
+    s, b = setup(20, 11, 4, True, degree)
+    want = torch.zeros_like(b)
+    s.precondition(want, b)
+    s.op.synchronize()
+    got = torch.full_like(b, 12345.0)
+    s.op.set_stage_wait_test(64)
+    s.precondition(got, b)
+    with pytest.raises(AFError) as e:
+        s.op.synchronize()
+    assert e.value.status == AF_TIMEOUT
+    assert bool((got == 12345.0).all())
+    s.op.set_stage_wait_test(0)
+    s.precondition(got, b)
+    s.op.synchronize()
+    assert torch.equal(got, want)
