@@ -164,10 +164,10 @@ struct DegreeOps {
   //   the most tiles that gs_chain takes (all resident at once; 0: none) on a device
   int (*gs_chain_tiles)(int device);
   //   n pairs (gs_binv, gs_zstep) with (alpha, s) = coef[2 i], coef[2 i + 1], after gs_entry with the
-  //   same words; d, z and dtr are left in between
+  //   same words; d, z and dtr are left in between; launched: its launches
   cudaError_t (*gs_chain)(const MeshDev&, const GsGeo& geo, const float* coef, int n, float cB, float cgg, float g,
                           const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x, float* dtr,
-                          unsigned long long* words, int ncell, cudaStream_t);
+                          unsigned long long* words, int ncell, cudaStream_t, int* launched);
 };
 
 const DegreeOps* degree_ops(int P);  // null if the degree was not compiled

@@ -1067,7 +1067,8 @@ int gs_chain_tiles(int device) {
 }
 cudaError_t gs_chain(const MeshDev& mesh, const GsGeo& geo, const float* coef, int n, float cB, float cgg, float g,
                      const float* WA, const float* pg, const float* ptr, float* z, float* d, float* x, float* dtr,
-                     unsigned long long* words, int ncell, cudaStream_t st) {
+                     unsigned long long* words, int ncell, cudaStream_t st, int* launched) {
+  *launched = 0;
   if (ncell <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)((ncell + kGsTile - 1) / kGsTile));
@@ -1089,6 +1090,7 @@ cudaError_t gs_chain(const MeshDev& mesh, const GsGeo& geo, const float* coef, i
                                              z, d, x, dtr, words, words + gs_words(ncell), words + 2 * gs_words(ncell), 2 * k,
                                              k + s.n < n ? 1 : 0);
     if (e != cudaSuccess) return e;
+    ++*launched;
   }
   return cudaSuccess;
 }

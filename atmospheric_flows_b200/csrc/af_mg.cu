@@ -506,12 +506,17 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
   if (L.gwords && last > 0) {  // all steps in one launch
     MeshDev mesh = L.mesh;
     mesh.test_wait_polls = o->mesh.test_wait_polls;
+    int launched = 0;
     const cudaError_t e = k->gs_chain(mesh, L.ggeo, coef.data(), last, (float)s->cB, (float)(s->cdt * kGG), (float)ginv,
-                                      L.gWA, L.gpg, L.gptr, zg, d, x, L.gdtr, L.gwords, L.ncell, o->stream);
-    if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();  // part of the device only: step by step
-    else if (e != cudaSuccess) MG_CU(e);
-    chained = e == cudaSuccess;
-    o->launches += 1;
+                                      L.gWA, L.gpg, L.gptr, zg, d, x, L.gdtr, L.gwords, L.ncell, o->stream, &launched);
+    o->launches += launched;
+    chained = launched > 0;
+    if (e == cudaErrorCooperativeLaunchTooLarge && !chained) {
+      cudaGetLastError();  // part of the device only: step by step, from now on
+      L.gwords = nullptr;
+    } else {
+      MG_CU(e);
+    }
   }
   for (int it = 1; it <= last && !chained; ++it) {
     // w = A^{-1} B d;  z += D^{-1} C0 w - d;  d = a d + sc z;  x += d (two launches; x takes the

@@ -48,3 +48,12 @@ def test_given_up_wait_leaves_the_output_unwritten(degree):
     s.precondition(got, b)
     s.op.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("degree,launches", [(1, 2), (8, 3), (65, 3), (66, 4), (130, 5)])
+def test_launch_count_of_the_one_launch_route(degree, launches):
+    """Entry and exit, and one launch per 64 of the degree - 1 steps."""
+    s, b = setup(20, 11, 4, True, degree)
+    out, before = torch.empty_like(b), s.op.launch_count()
+    s.precondition(out, b)
+    assert s.op.launch_count() - before == launches
