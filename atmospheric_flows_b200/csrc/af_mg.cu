@@ -180,6 +180,7 @@ struct af_schur_solver {
   bool fp32 = false;
   bool rq = false;              // FP32 levels with the reduced quadrature (P+1 Gauss points)
   bool gauss = false;           // the single-level FP32 Chebyshev in the Gauss-point basis
+  bool one_launch = true;       // its steps in one launch where L.gwords allows (test hook: false)
   bool setup_done = false, eig_done = false;
   double cB = 0, cdt = 0;       // B and C coefficients of the last setup
   double* part = nullptr;       // reductions
@@ -489,8 +490,9 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
   float* d = (float*)L.d;
   float* x = (float*)L.x;
   float *fx = (float*)L.w, *fe = fx + gs_padded(L.ncell, o->nd);
+  unsigned long long* const words = s->one_launch ? L.gwords : nullptr;
   // d = x = D^{-1} v / theta;  z = D^{-1} v = theta d
-  MG_CU(k->gs_entry(L.mesh, L.ggeo, v, (float)(ginv / theta), (float)theta, zg, d, x, L.gdtr, L.gwords, L.ncell,
+  MG_CU(k->gs_entry(L.mesh, L.ggeo, v, (float)(ginv / theta), (float)theta, zg, d, x, L.gdtr, words, L.ncell,
                     o->stream));
   o->launches += 1;
   double rho_old = 1.0 / sigma;
@@ -503,12 +505,12 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
     rho_old = rho;
   }
   bool chained = false;
-  if (L.gwords && last > 0) {  // all steps in one launch
+  if (words && last > 0) {  // all steps in one launch
     MeshDev mesh = L.mesh;
     mesh.test_wait_polls = o->mesh.test_wait_polls;
     int launched = 0;
     const cudaError_t e = k->gs_chain(mesh, L.ggeo, coef.data(), last, (float)s->cB, (float)(s->cdt * kGG), (float)ginv,
-                                      L.gWA, L.gpg, L.gptr, zg, d, x, L.gdtr, L.gwords, L.ncell, o->stream, &launched);
+                                      L.gWA, L.gpg, L.gptr, zg, d, x, L.gdtr, words, L.ncell, o->stream, &launched);
     o->launches += launched;
     chained = launched > 0;
     if (e == cudaErrorCooperativeLaunchTooLarge && !chained) {
@@ -527,7 +529,7 @@ int apply_gauss(af_schur_solver* s, double* z, const double* v) {
                       it % 2 == 0 ? 1 : (it == last ? 2 : 0), L.gdtr, L.ncell, o->stream));
     o->launches += 2;
   }
-  MG_CU(k->gs_exit(x, z, chained ? L.gwords : nullptr, L.ncell, o->stream));
+  MG_CU(k->gs_exit(x, z, chained ? words : nullptr, L.ncell, o->stream));
   o->launches += 1;
   return AF_OK;
 }
@@ -726,6 +728,12 @@ int af_schur_solver_levels(const af_schur_solver* s, int* n_levels, double* lmax
   *n_levels = s->nact;
   if (lmax)
     for (int l = 0; l < s->nact; ++l) lmax[l] = s->lv[l].lmax;
+  return AF_OK;
+}
+
+int af_schur_solver_set_one_launch(af_schur_solver* s, int enable) {
+  if (!s) return merr(AF_BAD_ARG, "null solver");
+  s->one_launch = enable != 0;
   return AF_OK;
 }
 

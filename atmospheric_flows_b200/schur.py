@@ -40,6 +40,7 @@ def _bind():
     L.af_schur_solver_setup.argtypes = [vp, ctypes.c_int]
     L.af_schur_solver_levels.argtypes = [vp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_double)]
     L.af_schur_solver_precondition.argtypes = [vp, vp, vp]
+    L.af_schur_solver_set_one_launch.argtypes = [vp, ctypes.c_int]
     L.af_schur_solve.argtypes = [vp, vp, vp, ctypes.c_double, ctypes.c_int, ctypes.POINTER(Stats)]
     L.af_schur_solve_transpose.argtypes = [vp, vp, vp, vp, ctypes.c_double, ctypes.c_int, ctypes.POINTER(Stats)]
     L._schur_bound = True
@@ -89,6 +90,11 @@ class SchurSolver:
 
     def precondition(self, dst, src):
         check(_bind().af_schur_solver_precondition(self._h, _ptr(dst), _ptr(src)))
+
+    def set_one_launch(self, enable):
+        """Test hook: False makes the Gauss-point polynomial run a launch per half step on small
+        meshes too; True (the default) lets the mesh decide."""
+        check(_bind().af_schur_solver_set_one_launch(self._h, int(enable)))
 
     def solve_transpose(self, p, x, b, rel_tol=1e-10, max_iterations=1000, raise_on_failure=True):
         """Adjoint solve J_S(p)^T x = b (x: initial guess in, solution out)."""

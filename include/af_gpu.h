@@ -223,6 +223,10 @@ int af_schur_solver_setup(af_schur_solver* s, int estimate_eigenvalues);
 int af_schur_solver_levels(const af_schur_solver* s, int* n_levels, double* lmax);
 /* dst = one application of the preconditioner to src (DEVICE pointers, pressure space). */
 int af_schur_solver_precondition(af_schur_solver* s, double* dst, const double* src);
+/* Test hook: 0 makes the AF_SCHUR_CHEB_FP32 polynomial (reduced_quadrature 2) of this solver run a
+ * launch per half step on meshes that one launch could take, as larger meshes do; 1 (the default)
+ * lets the mesh decide. */
+int af_schur_solver_set_one_launch(af_schur_solver* s, int enable);
 /* x (initial guess in, solution out) for S x = b; returns AF_NO_CONVERGENCE at the cap. */
 int af_schur_solve(af_schur_solver* s, double* x, const double* b, double rel_tol, int max_iterations,
                    af_schur_stats* stats);
