@@ -81,3 +81,34 @@ def test_iterates_on_long_vectors(precond):
         x.zero_()
         q = s.solve(x, b, rel_tol=1.0001 * res / float(beta), max_iterations=steps)
         assert q["iterations"] == k
+
+
+@pytest.mark.parametrize("restart", [1, 2, 3, 5])
+def test_short_restarts_never_lose_ground(restart):
+    """Each cycle minimises the residual from where the last one ended: the true residual, by the
+    operator's own apply, is what the solver reports (1e-10 of |b|) and does not grow with the cap."""
+    from atmospheric_flows_b200.operator import EULEROperator
+    from atmospheric_flows_b200.schur import SchurSolver
+    P, sc = 4, M.Scaling()
+    m = M.hill_mesh(40, 26, periodic_x=True)
+    st = M.hill_state(m, P, modes=4)
+    op = EULEROperator(m, P, sc.Ma, sc.Fr, 0.25)
+    op.set_stream(torch.cuda.current_stream())
+    op.set_schur_mode(1)
+    op.set_HYPERBOLIC_stage(1)
+    op.set_rho_for_fixed(torch.from_numpy(st.rho).cuda())
+    op.set_pres_fixed(torch.from_numpy(st.p).cuda())
+    b = torch.from_numpy(np.random.default_rng(7).standard_normal(op.n_dofs(1))).cuda()
+    s = SchurSolver(op, "jacobi", restart=restart)
+    s.setup()
+    last = float(b.norm())
+    for cap in (1, 2, 4, 7, 12, 20):
+        x, r = torch.zeros_like(b), torch.empty_like(b)
+        q = s.solve(x, b, rel_tol=1e-10, max_iterations=cap, raise_on_failure=False)
+        op.set_NS_stage(2)
+        op.vmult(r, x)
+        true = float((b - r).norm())
+        assert abs(true - q["final_residual"]) < 1e-10 * float(b.norm())
+        assert true <= last * (1 + 1e-10)
+        last = true
+    assert last < float(b.norm())
