@@ -436,11 +436,13 @@ struct Layout {
   // Own-cell staging: the nodes of every (cell, component) of a batch's arrays form one list of
   // lines of ND nodes at stride LS, array after array, [cell][component] inside an array (the
   // global order).  With an odd number of nodes per cell the list is the arrays' image and arrives
-  // by one bulk copy (TMA) per array; with an even number in FP64 by one bulk copy per line, 16
-  // bytes apart against bank conflicts (degree 5: unpadded 748 us, padded 707 us for the fused
-  // right-hand sides at 512x256); else by per-element copies.  Consecutive threads take
-  // consecutive lines, an odd number of elements apart.
-  static constexpr bool BULK = (ND % 2 == 1 && (CB * ND * (int)sizeof(R)) % 16 == 0) || (ND % 2 == 0 && sizeof(R) == 8 && P >= 3);
+  // by one bulk copy (TMA) per array; at degree 5 in FP64 by one bulk copy per line of 36 nodes, 16
+  // bytes apart against bank conflicts (unpadded 748 us, padded 707 us for the fused right-hand
+  // sides at 512x256); else by per-element copies of all threads.  At degree 3 a bulk copy of a line
+  // of 16 nodes costs more than the elements (one warp issues 63 to 130 of them): stage 3 at 512x256
+  // 405 -> 352 us with element copies, the split right-hand sides at 91x32 28.6 -> 19.4 us, C at 40x16
+  // 5.2 -> 4.9 us.  Consecutive threads take consecutive lines, an odd number of elements apart.
+  static constexpr bool BULK = (ND % 2 == 1 && (CB * ND * (int)sizeof(R)) % 16 == 0) || (ND % 2 == 0 && sizeof(R) == 8 && P >= 5);
   static constexpr int PADB = (BULK && ND % 2 == 0) ? ALIGN : 0;
   static constexpr int LS = BULK ? ND + PADB : odd(ND);
   static constexpr int ISSUE_LANES = PADB ? 32 : 1;  // threads that issue the copies
@@ -744,6 +746,23 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
       }
     });
   };
+  // the same by per-element copies of all threads (waited for with cp_async_wait_all)
+  auto copy_batch = [&](auto bc) {
+    constexpr int B = decltype(bc)::value;
+    sfor<Phys::NG>([&](auto gc) {
+      constexpr int G = decltype(gc)::value;
+      if constexpr (I::batch_of(G) == B) {
+        using Gi = GroupInfo<Phys, G>;
+        sfor<Gi::NARR>([&](auto ac) {
+          constexpr int A = decltype(ac)::value;
+          constexpr int NC = Gi::Gr::ncomp(A);
+          const R* src = ptr.in[I::arr_base(G) + A] + (size_t)c0 * NC * ND;
+          for (int e = tid; e < ncb * NC * ND; e += NT)
+            cp_async_el(&smem[L::O_IN + (L::template line_base<G>(A) + e / ND) * L::LS + e % ND], src + e);
+        });
+      }
+    });
+  };
   // copies were issued and not yet waited for; their phase
   bool pending = L::BULK && bulk;
   unsigned phase = 0u;
@@ -780,11 +799,12 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
   }
-  // the copies that read what earlier kernels wrote: batch 0 (bulk layout) and the epilogue's chunks
+  // the copies that read what earlier kernels wrote: batch 0 and the epilogue's chunks
   auto issue_inputs = [&]() {
     if constexpr (L::BULK) {
       if (tid < L::ISSUE_LANES && bulk) issue_batch(std::integral_constant<int, 0>{});
     }
+    if (!bulk) copy_batch(std::integral_constant<int, 0>{});
     if constexpr (L::EPI != 0) {
       if (epi_bulk) {
         if (tid == 0) {
@@ -962,19 +982,6 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
         report_status(mesh.status, kStatusStageTimeout);
       }
     } else {
-      sfor<Phys::NG>([&](auto gc) {
-        constexpr int G = decltype(gc)::value;
-        if constexpr (I::batch_of(G) == B) {
-          using Gi = GroupInfo<Phys, G>;
-          sfor<Gi::NARR>([&](auto ac) {
-            constexpr int A = decltype(ac)::value;
-            constexpr int NC = Gi::Gr::ncomp(A);
-            const R* src = ptr.in[I::arr_base(G) + A] + (size_t)c0 * NC * ND;
-            for (int e = tid; e < ncb * NC * ND; e += NT)
-              cp_async_el(&s_in[(L::template line_base<G>(A) + e / ND) * L::LS + e % ND], src + e);
-          });
-        }
-      });
       cp_async_wait_all();
       __syncthreads();
     }
@@ -1052,6 +1059,8 @@ __global__ void __launch_bounds__(Layout<P, Phys, CB_>::NT, MINB)
       if (bulk) {
         if (tid < L::ISSUE_LANES) issue_batch(std::integral_constant<int, B + 1>{});
         pending = true;
+      } else {
+        copy_batch(std::integral_constant<int, B + 1>{});
       }
     }
 
