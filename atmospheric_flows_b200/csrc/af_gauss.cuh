@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
   const int lane = threadIdx.x & 31, m = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), tile = blockIdx.x;
   const int n = min(kGsTile, ncell - tile * kGsTile) * ND;
   pdl_wait_previous();
-  if (gave_up && *gave_up) return;
+  const bool skip = gave_up && *gave_up;  // looked at with the store: its load overlaps the others
   float u[P1];
 #pragma unroll
   for (int q = 0; q < P1; ++q) u[q] = xg[S::column(tile, m, lane) + q * S::SN];
@@ -763,6 +763,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT)
     s_v[lane * NDS + m * P1 + i] = t;
   }
   __syncthreads();
+  if (skip) return;
   for (int e = threadIdx.x; e < n; e += S::NT)
     out[(size_t)tile * kGsTile * ND + e] = (double)s_v[(e / ND) * NDS + e % ND];
 }
