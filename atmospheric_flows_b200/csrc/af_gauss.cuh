@@ -466,6 +466,8 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   __shared__ float s_xf[4 * P1 * kGsTile];  // x-face fluxes of B [face][component][point][lane]
   __shared__ float s_w[2 * ND * kGsTile];   // w [component][node][lane]
   __shared__ float s_fx[ND * kGsTile], s_d[ND * kGsTile], s_xf2[2 * P1 * kGsTile];
+  constexpr bool SHARED_EDGES = P <= 5;
+  __shared__ float s_rt[SHARED_EDGES ? 4 * kGsTile : 1];  // edges of the faces xi = 1 and eta = 1
   __shared__ float s_wm[ND * kGsTile];      // g / JxW; each thread reads its own column
   if (base > 0 && *gave_up) return;  // an earlier launch of this application
   const CobT<P, float>& cb = cobr<P, float>();
@@ -490,6 +492,23 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   }
   gs_ends<P>(pc, pt[2], pt[3]);
   gs_ends<P>(dc, tp[2], tp[3]);
+  // the far edges' normals come from shared memory up to degree 5 (degree 4, 256 tiles: 59.9 us a polynomial
+  // with them in registers, 56.7 us so; degree 6, 96 tiles: 60.5 and 71.9 us, nothing spills there)
+  if (SHARED_EDGES && m == 0) {
+    s_rt[lane] = th.Rx;
+    s_rt[kGsTile + lane] = th.Rz;
+    s_rt[2 * kGsTile + lane] = th.Tx;
+    s_rt[3 * kGsTile + lane] = th.Tz;
+  }
+  auto normal = [&](int f, float& n0, float& n1) {
+    if (SHARED_EDGES && (f & 1)) {
+      const float s = f == 3 ? 1.f : -1.f;
+      n0 = -s * s_rt[f * kGsTile + lane];
+      n1 = s * s_rt[(f - 1) * kGsTile + lane];
+    } else {
+      th.normal(f, n0, n1);
+    }
+  };
   // the neighbours' values of that count (a wall takes the own one); false when the bound was reached
   const bool hook = mesh.test_wait_polls > 0;
   const int polls = hook ? mesh.test_wait_polls : kGsWaitPolls;
@@ -567,7 +586,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
       float n0, n1;
-      th.normal(f, n0, n1);
+      normal(f, n0, n1);
       const float a = cB * 0.5f * (tp[f] + tm[f]) * wx;
       const float F0 = a * n0, F1 = a * n1;
       if (f < 2) {
@@ -609,7 +628,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
         float n0, n1;
-        th.normal(f, n0, n1);
+        normal(f, n0, n1);
         g[f] = 0.5f * cgg * wx * pt[f] * (t0[f] * n0 + t1[f] * n1);
         gs_put(wg + op + f * S::SF, g[f], base + 2 * it - 1);
       }
