@@ -53,7 +53,7 @@ namespace {
 constexpr int P = AF_P;
 // cells per CTA of the reduced-quadrature (P+1 points) B kernel: its CTAs have NQ = P+1
 // threads per cell, about half of the full-quadrature kernel's
-constexpr int kReducedCB = P == 1 ? 64 : (P == 2 ? 42 : (P <= 4 ? 32 : (P == 5 ? 20 : 18)));
+constexpr int kReducedCB = P == 1 ? 64 : (P == 2 ? 42 : (P == 3 ? 8 : (P == 4 ? 32 : (P == 5 ? 20 : 18))));
 
 constexpr int kND = (P + 1) * (P + 1);
 constexpr int kNPK = kND * (kND + 1) / 2;
