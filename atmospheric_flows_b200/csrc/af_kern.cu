@@ -51,9 +51,12 @@ __device__ __forceinline__ const CobT<AF_P, float>& cobr<AF_P, float>() {
 namespace {
 
 constexpr int P = AF_P;
-// cells per CTA of the reduced-quadrature (P+1 points) B kernel: its CTAs have NQ = P+1
-// threads per cell, about half of the full-quadrature kernel's
-constexpr int kReducedCB = P == 1 ? 64 : (P == 2 ? 42 : (P == 3 ? 8 : (P == 4 ? 32 : (P == 5 ? 20 : 18))));
+// Cells per CTA of the reduced-quadrature (P+1 points) B kernel: its CTAs have NQ = P+1 threads per cell,
+// about half of the full-quadrature kernel's.  Measured, us at 128x64 and 512x256 cells:
+//   p=1  64: 3.6, 12.1;  32: 3.5, 12.3      p=2  32: 3.5, 15.3;  42: 3.7, 16.0
+//   p=3  8: 6.9, 37.5;  16: 5.3 to 9, 41.8;  24: 9.1, 39.5;  32: 9.4, 40.8;  64: 9.3, 42.5
+//   p=4  32: 5.5, 34.8;  16: 5.7, 39.8      p=5  8: 7.4, 61.2;  20: 9.0, 64.0     p=6  18: 6.9, 68.6;  8: 6.6, 71.4
+constexpr int kReducedCB = P == 1 ? 64 : (P == 2 ? 32 : (P == 3 ? 8 : (P == 4 ? 32 : (P == 5 ? 8 : 18))));
 
 constexpr int kND = (P + 1) * (P + 1);
 constexpr int kNPK = kND * (kND + 1) / 2;
