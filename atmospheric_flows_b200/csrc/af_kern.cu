@@ -668,7 +668,14 @@ __global__ void k_inject(const double* __restrict__ ff, double* __restrict__ fc,
 }
 
 // ------------------------------------------------------------------ adjoint
-constexpr int kAdjCells = P <= 2 ? 16 : 10;
+// Cells per CTA of the tangents and adjoints (fit_cells takes fewer where two CTAs would not share an
+// SM): whole warps up to degree 3.  Measured, us of the stage-1 backward at 128x64 and 512x256 cells:
+//   p=1  21: 10.9, 104;  16: 14.8, 114;  32: 14.2, 114;  42: 11.2, 106 (at 160x80 cells 18.0, 14.9, 14.4, 18.2:
+//        the remainder of CTAs per SM)
+//   p=2  12: 19.4, 183;  16: 22.9, 230;  19: 20.9, 249      p=3  9: 32.8, 393;  8: 33.6, 436;  13: 34.9, 428;  10: 40.0, 522
+//   p=4  10: 41.9, 575;  7: 39.4, 590 (the tangent 535 and 744)
+//   p=5  10 and 8 (one CTA shape by fit_cells): 84.3, 1188;  5: 90.4, 1348      p=6  10 and 4: 112, 1728
+constexpr int kAdjCells = P == 1 ? 21 : (P == 2 ? 12 : (P == 3 ? 9 : 10));
 cudaError_t rhs_adjoint1(const MeshDev& mesh, const double* const* in, const double* const* ybar,
                          double* const* xbar, const RhsParams& prm, int ncell, cudaStream_t st) {
   ArgPtrs<8, 5> a{{in[0], in[1], in[2], in[3], in[4], ybar[0], ybar[1], ybar[2]},
