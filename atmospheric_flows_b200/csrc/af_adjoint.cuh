@@ -32,10 +32,7 @@ struct RhsAdj1Phys {
   static constexpr int out_ncomp(int a) { return (a == 1 || a == 4) ? 2 : 1; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return 8; }
   static constexpr bool face_field(int, int f) { return f < 4 || f >= 7; }  // rho0, u0, p0 and the cotangents
-  static constexpr int nf_of(int) { return 11; }
-  static constexpr int nfc_of(int) { return 11; }
   static constexpr int nfg_of(int) { return 4; }
   template <int G>
   struct Grp {
@@ -170,10 +167,7 @@ struct RhsTlm1Phys {
   static constexpr int out_ncomp(int a) { return a == 1 ? 2 : 1; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return true; }
-  static constexpr int narr_of(int) { return 10; }
   static constexpr bool face_field(int, int f) { return f % 7 < 4; }  // rho0, u0, p0 and their tangents
-  static constexpr int nf_of(int) { return 14; }
-  static constexpr int nfc_of(int) { return 14; }
   template <int G>
   struct Grp {
     static constexpr int NARR = 10;
@@ -278,9 +272,6 @@ struct BTPhys {
   static constexpr int out_ncomp(int) { return 1; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return 1; }
-  static constexpr int nf_of(int) { return 2; }
-  static constexpr int nfc_of(int) { return 2; }
   static constexpr int nfg_of(int) { return 2; }
   template <int G>
   struct Grp {
@@ -324,9 +315,6 @@ struct CTlmPhys {
   static constexpr int out_ncomp(int) { return 1; }
   static constexpr bool has_val(int) { return false; }
   static constexpr bool has_grad(int) { return true; }
-  static constexpr int narr_of(int) { return 3; }
-  static constexpr int nf_of(int) { return 5; }
-  static constexpr int nfc_of(int) { return 5; }
   template <int G>
   struct Grp {
     static constexpr int NARR = 3;
@@ -369,9 +357,6 @@ struct CTPhys {
   static constexpr int out_ncomp(int) { return 2; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return 3; }
-  static constexpr int nf_of(int) { return 4; }
-  static constexpr int nfc_of(int) { return 4; }
   static constexpr int nfg_of(int) { return 1; }
   template <int G>
   struct Grp {
@@ -419,9 +404,6 @@ struct MassRhoTPhys {
   static constexpr int out_ncomp(int) { return 1; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return 2; }
-  static constexpr int nf_of(int) { return 4; }
-  static constexpr int nfc_of(int) { return 4; }
   template <int G>
   struct Grp {
     static constexpr int NARR = 2;
@@ -456,9 +438,6 @@ struct CPfTPhys {
   static constexpr int out_ncomp(int) { return 1; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return 2; }
-  static constexpr int nf_of(int) { return 3; }
-  static constexpr int nfc_of(int) { return 3; }
   static constexpr int nfg_of(int) { return 1; }
   template <int G>
   struct Grp {
@@ -510,9 +489,6 @@ struct RhsTanPhys {
   static constexpr int out_ncomp(int a) { return Base::out_ncomp(a); }
   static constexpr bool has_val(int o) { return Base::has_val(o); }
   static constexpr bool has_grad(int o) { return Base::has_grad(o); }
-  static constexpr int narr_of(int g) { return 2 * Base::narr_of(g); }
-  static constexpr int nf_of(int g) { return 2 * Base::nf_of(g); }
-  static constexpr int nfc_of(int g) { return 2 * Base::nfc_of(g); }
   template <int G>
   struct Grp {
     using BG = typename Base::template Grp<G>;
@@ -601,9 +577,6 @@ struct RhsAdjGPhys {
   static constexpr int out_ncomp(int a) { return BG::ncomp(a); }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return NB + 3; }
-  static constexpr int nf_of(int) { return NFb + NY; }
-  static constexpr int nfc_of(int) { return NFCb + NY; }
   static constexpr int nfg_of(int) { return NY; }
   template <int G>
   struct Grp {

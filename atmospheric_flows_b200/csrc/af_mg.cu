@@ -663,10 +663,13 @@ int af_schur_solver_create(af_operator* op, const af_schur_options* opt, af_schu
     if ((r = alloc(s, &L.LA, rs * nf)) != AF_OK) return cleanup(r);
     if ((r = alloc(s, &L.LM, rs * nf)) != AF_OK) return cleanup(r);
     const size_t nv = s->gauss ? gs_padded(L.ncell, nd) : (size_t)L.ns;
-    for (void** p : {&L.x, &L.b, &L.r, &L.d})
+    for (void** p : {&L.x, &L.r, &L.d})
       if ((r = alloc(s, p, rs * nv)) != AF_OK) return cleanup(r);
-    for (void** p : {&L.u, &L.w})
-      if ((r = alloc(s, p, rs * 2 * nv)) != AF_OK) return cleanup(r);
+    if ((r = alloc(s, &L.w, rs * 2 * nv)) != AF_OK) return cleanup(r);
+    if (!s->gauss) {  // the Gauss-point polynomial needs neither
+      if ((r = alloc(s, &L.b, rs * nv)) != AF_OK) return cleanup(r);
+      if ((r = alloc(s, &L.u, rs * 2 * nv)) != AF_OK) return cleanup(r);
+    }
     if (s->gauss) {
       const size_t cells = gs_padded(L.ncell, 1), nt = 4 * cells * (op->P + 1);
       if ((r = alloc(s, (void**)&L.ggeo.map, sizeof(float) * kGsGeo * cells)) != AF_OK) return cleanup(r);

@@ -409,9 +409,6 @@ struct BPhysT {
   static constexpr int out_ncomp(int) { return 2; }
   static constexpr bool has_val(int) { return false; }
   static constexpr bool has_grad(int) { return true; }
-  static constexpr int narr_of(int) { return 1; }
-  static constexpr int nf_of(int) { return 1; }
-  static constexpr int nfc_of(int) { return 1; }
   template <int G>
   struct Grp {
     static constexpr int NARR = 1;
@@ -483,9 +480,6 @@ struct CPhys {
   static constexpr int out_ncomp(int) { return 1; }
   static constexpr bool has_val(int) { return WITH_D; }
   static constexpr bool has_grad(int) { return true; }
-  static constexpr int narr_of(int g) { return g == GW ? 2 : 1; }
-  static constexpr int nf_of(int g) { return g == GW ? 3 : 1; }
-  static constexpr int nfc_of(int g) { return nf_of(g); }
   template <int G>
   struct Grp {
     static constexpr int NARR = G == GW ? 2 : 1;
@@ -601,9 +595,6 @@ struct MassPhys {
   static constexpr int out_ncomp(int) { return NC; }
   static constexpr bool has_val(int) { return true; }
   static constexpr bool has_grad(int) { return false; }
-  static constexpr int narr_of(int) { return WEIGHTED ? 2 : 1; }
-  static constexpr int nf_of(int) { return NC + (WEIGHTED ? 1 : 0); }
-  static constexpr int nfc_of(int) { return NC + (WEIGHTED ? 1 : 0); }
   template <int G>
   struct Grp {
     static constexpr int NARR = WEIGHTED ? 2 : 1;
