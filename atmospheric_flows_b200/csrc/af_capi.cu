@@ -467,11 +467,12 @@ int af_vmult_rhs_fused_host(af_operator* o, double* h_rho, double* h_u, double* 
   // Rows of cells go through in chunks so that the copies overlap the kernel: the sources of
   // chunk k+1 travel (copy_in) while chunk k is computed (the operator's stream) and chunk
   // k-1's results return (copy_out).  A chunk's kernel also reads the row of cells above it
-  // (face neighbours), so it starts once the next chunk's sources are in.  Chunk boundaries
-  // are multiples of the kernel's cells per CTA; otherwise the call runs as one chunk.
-  const int nx = o->mesh.nx, nz = o->mesh.nz, cpb = o->ops->cells_per_block;
+  // (face neighbours), so it starts once the next chunk's sources are in.  A chunk starts on
+  // a multiple of range_cells (16 bytes: an even cell with an odd number of nodes per cell);
+  // otherwise the call runs as one chunk.
+  const int nx = o->mesh.nx, nz = o->mesh.nz, align = o->ops->range_cells;
   int rpc = (nz + af_operator::kHostChunks - 1) / af_operator::kHostChunks;  // rows per chunk
-  if (((long)rpc * nx) % cpb != 0) rpc = nz;
+  if (((long)rpc * nx) % align != 0) rpc = nz;
   const int K = (nz + rpc - 1) / rpc;
   if (!o->copy_in) AF_CU(cudaStreamCreateWithFlags(&o->copy_in, cudaStreamNonBlocking));
   if (!o->copy_out) AF_CU(cudaStreamCreateWithFlags(&o->copy_out, cudaStreamNonBlocking));

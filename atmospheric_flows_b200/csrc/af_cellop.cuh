@@ -192,9 +192,9 @@ constexpr int odd(int n) { return n | 1; }
 // anything a kernel can write.  Geometry-first prologue (the geometry before the wait, the
 // own-cell copies after it) or wait-first (the copies issued at once, overlapping the
 // geometry, as without the dependent launch): AF_PDL_GEO_FIRST 1 always, 0 never, 2 for the
-// FP32 kernels only.  Measured at 512x256, p = 4: the fused FP64 rhs 401.0 us without the
-// dependent launch, 401.9 geometry-first, 397.5 wait-first; the mixed IMEX step (FP32
-// smoothers, about 1000 launches of 45-55 us) 77.8, 75.0 and 75.6 ms.
+// FP32 kernels only.  Measured, us without the dependent launch / geometry-first / wait-first, p = 4: the
+// fused FP64 rhs at 512x256 207.6 / 208.4 / 206.5, at 64x32 10.5 / 8.4 / 8.4; the degree-16 nodal FP32
+// polynomial (32 launches) at 512x256 1348 / 1269 / 1279, at 64x32 224 / 162 / 172.
 #ifndef AF_PDL
 #define AF_PDL 1
 #endif
@@ -242,13 +242,12 @@ __device__ __forceinline__ void report_status(int* status, int code) {
 // stage 1, stage 3, the three split calls of stage 3, C):
 //   p=1 (262144 cells)  42 x 3 CTAs per SM 106, 242, 440, 36;  32 x 4: 100, 231, 436, 35;  21 x 6: 107, 253, 459, 37
 //   p=2  24 x 3: 84, 195, 369, 32;  18 x 4: 86, 203, 391, 33;  12 x 6: 85, 208, 402, 35
-//   p=3  18 x 3: 200, 456, 955, 70;  16 x 3: 211, 482, 985, 70;  13 x 4: 196, 452, 918, 73;
-//        9 x 6: 170, 406, 838, 64;  8 x 6: 180, 437, 904, 68
+//   p=3 (element copies)  9 x 6: 163, 352, 725, 63;  13 x 4: 176, 385, 771, 66;  18 x 3: 178, 376, 739, 62
 //   p=4  14 x 3: 207, 481, 911, 82;  12 x 3: 229, 545, 1007, 91;  10 x 4: 221, 548, 1000, 87;  6 x 6: 232, 557, 1088, 101
 //   p=5 (65536 cells)  11 x 2: 227, 515, 928, 66;  8 x 3: 217, 483, 825, 68 (stage 2 430, not 412);  5 x 4: 224, 545, 978, 67
 //   p=6 (32768 cells)  8 x 2: 152, 327, 561, 44;  4 x 4: 151, 332, 587, 47
-// Meshes of less than about two CTAs per SM take 10 percent more or less with the remainder of that count
-// (p=3, 91x32 cells, split stage 1: 9 cells 30, 10 cells 28, 18 cells 34; 40x16: 20, 25, 26).
+// Meshes of a few CTAs per SM take 10 to 15 percent more or less with the remainder of that count (p=3, C at
+// 128x64 cells: 9 cells, 911 CTAs on 888 places, 8.4;  13 cells 8.0;  160x80: 8.3 and 10.1).
 // An odd number of cells needs an even number of nodes a cell: the bulk copies start on 16 bytes.
 template <int P, class R = double>
 constexpr int cells_per_block() {
@@ -316,7 +315,7 @@ constexpr int arr_total(int upto, std::integer_sequence<int, G...>) {
 // with two and three explicit groups) each is its own batch and so is the implicit group after
 // them: the batches' fields follow one another through the same shared memory, which keeps two or
 // three CTAs on an SM (all of them at once left one CTA of 16 cells per SM at degree 4: the
-// stage-3 right-hand sides at 2048x512 10.8 ms, in batches 5.4 ms).
+// stage-3 right-hand sides at 2048x512 10.8 ms in the layout before, 3.8 ms now).
 template <class Phys>
 struct PhysInfo {
   using Seq = std::make_integer_sequence<int, Phys::NG>;
@@ -544,7 +543,7 @@ struct Layout {
 // Cells per CTA of a policy launched without a choice of its own: cells_per_block, or the next smaller
 // count with which the bulk copies stay aligned where the shared memory then holds one more CTA per SM.
 // That is so for the fused stage-2 right-hand sides of degree 4 (12 cells: three CTAs, not two; 455 ->
-// 411 us at 512x256) and degree 3 (8 cells: six, not five; 361 -> 340 us).
+// 411 us at 512x256) and degree 3 (8 cells: six, not five; 361 -> 340 us, 298 with element copies).
 template <int P, class Phys>
 constexpr int default_cells() {
   using R = RealOf<Phys>;

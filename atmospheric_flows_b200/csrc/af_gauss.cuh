@@ -94,9 +94,10 @@ struct GsShape {
   // CTAs per SM asked of the compiler.  Degree 4, (k_gs_binv, k_gs_zstep), the mixed IMEX step at
   // 512x256: (4, 6) 46.3 ms, (5, 6) 45.4, (5, 7) 45.2, (6, 6) 46.8 (k_gs_binv spills at 64 registers).
   static constexpr int CTAS_B = 800 / NT, CTAS_Z = (P <= 4 ? 1120 : 900) / NT;
-  // k_gs_chain: more CTAs per SM take larger meshes.  Degree 4, 3 / 4 / 5 per SM (128, 102, 80 registers; 0,
-  // 160 and more bytes spilled): 256 tiles 64, 64, 75 us, 576 tiles (the pairs) 166, 82, 120; degree 2, 5 / 8 per SM: 256
-  // tiles 45, 48 us, 1024 tiles (the pairs) 128, 64
+  // k_gs_chain: more CTAs per SM take larger meshes.  Degree-20 polynomial, degree 4, 3 / 4 / 5 per SM (128,
+  // 96, 80 registers; 0, 164, 356 bytes of spill loads): 256 tiles 58, 62, 72 us, 440 tiles 64, 70, 92, 550
+  // tiles (165 by the pairs) 165, 79, 107; degree 2, 5 / 8 per SM: 256 tiles 45, 48 us, 1024 tiles (122 by
+  // the pairs) 122, 63
   static constexpr int CTAS_C = (P <= 2 ? 800 : 640) / NT;
   // the thread's element of node or point 0 .. and the strides between its nodes (column m) and faces
   __device__ __forceinline__ static size_t column(int tile, int m, int lane) {
@@ -444,8 +445,8 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_Z)
 // and leaves, and so do those that wait for it; k_gs_exit then writes nothing.
 // What bounds it: latency.  Degree-20 polynomial, us, the pairs (one launch per half step) / with
 // flags per tile, fences and barriers / now:
-//   degree 4  256 tiles 123 / 97 / 64, 444 tiles 166 / 106 / 72, 1 tile 99 / 64 / 42;  degree 2, 576 tiles
-//   100 / 96 / 48;  degree 6, 96 tiles 167 / 94 / 66   (a step and its adjoint at 128x64: 49.9 / 46.6 / 39.2 ms)
+//   degree 4  256 tiles 123 / 97 / 62, 440 tiles 166 / 106 / 70;  degree 6, 96 tiles 167 / 94 / 60
+//   (a step and its adjoint at 128x64: 49.9 / 46.6 / 38.8 ms)
 constexpr int kGsWaitPolls = 1 << 19;
 using GsWord = unsigned long long;  // a face value and its count
 __device__ __forceinline__ GsWord gs_word(float v, int count) {

@@ -52,7 +52,7 @@ struct DegreeOps {
   // x = scale * M^{-1} b (block diagonal, exact), ncomp components per cell
   cudaError_t (*mass_solve)(const double* L, int ncomp, const double* b, double scale, double* x, int ncell,
                             int* status, cudaStream_t);
-  int cells_per_block;
+  int range_cells;  // a range launch (MeshDev::cell0) of aligned bulk copies starts on a multiple of this
   int factor_len;  // (p+1)^2 ((p+1)^2 + 1) / 2
 
   // ---- h-multigrid level kernels, in FP64 (_d) and FP32 (_f) ----

@@ -674,7 +674,7 @@ __global__ void k_inject(const double* __restrict__ ff, double* __restrict__ fc,
 //        the remainder of CTAs per SM)
 //   p=2  12: 19.4, 183;  16: 22.9, 230;  19: 20.9, 249      p=3  9: 32.8, 393;  8: 33.6, 436;  13: 34.9, 428;  10: 40.0, 522
 //   p=4  10: 41.9, 575;  7: 39.4, 590 (the tangent 535 and 744)
-//   p=5  10 and 8 (one CTA shape by fit_cells): 84.3, 1188;  5: 90.4, 1348      p=6  10 and 4: 112, 1728
+//   p=5  10 (6 by fit_cells): 84.3, 1188;  5: 90.4, 1348      p=6  10 (4 by fit_cells): 112, 1728
 constexpr int kAdjCells = P == 1 ? 21 : (P == 2 ? 12 : (P == 3 ? 9 : 10));
 cudaError_t rhs_adjoint1(const MeshDev& mesh, const double* const* in, const double* const* ybar,
                          double* const* xbar, const RhsParams& prm, int ncell, cudaStream_t st) {
@@ -933,9 +933,12 @@ cudaError_t cob_cheb(const R* W, const R* r, R alpha, R s, R* d, R* x, int first
 }
 
 // ------------------------------------------------------------------ fused epilogues
-// Launch shapes of the two FP32 smoother kernels at p = 4 (1024x256, us per launch):
-// cells per CTA / CTAs per SM  16/2: B+A^-1 190.6, residual+Chebyshev 258.2;  32/2: 176.4,
-// 237.7;  32/3: 172.5, 240.5;  8/8: 215.1, 314.7;  64/1: 209.1, 372.2.
+// Launch shapes of the nodal FP32 smoother's kernels (cells per CTA; CTAs per SM asked of the compiler).
+// Measured, us of the degree-16 polynomial with P+1 points per direction at 64x32, 256x128 and 512x256:
+//   p=4  32: 162, 393, 1269;  16: 218, 435, 1424      p=3  16: 144, 334, 944;  32: 140, 334, 954 (with 2P+1
+//   points 215, 434, 1477 and 155, 412, 1393; the multigrid solve at 256x128 18.6 and 19.2 ms)
+// CTAs per SM at p = 4, (B with A^-1, residual): (3, 2) and (2, 3) the same times; p = 3, 16 cells, 3, 6
+// and 8 the same solve.
 constexpr int kFusedCB = P == 4 ? 32 : cells_per_block<P, float>();
 constexpr int kFusedMinB = P == 3 || P == 5 ? 3 : 2;
 constexpr int kBInvMinB = P == 4 ? 3 : kFusedMinB;
@@ -984,7 +987,7 @@ cudaError_t b_inv_fr(const MeshDev& mesh, const float* p, float c, const float* 
   q.c = c;
   q.inv = WA;
   q.scale = scale;
-  return launch_cellop<P, BInvRPhys<float>, kFusedCB, (P == 4 ? 4 : kBInvMinB)>(mesh, a, q, ncell, st);  // 92 vs 95 us
+  return launch_cellop<P, BInvRPhys<float>, kFusedCB, kBInvMinB>(mesh, a, q, ncell, st);
 }
 cudaError_t res_cheb_fr(const MeshDev& mesh, const float* w, const float* pf, const float* din,
                         const CParamsT<float>& prm, const float* WM, float alpha, float s, float* r, float* dout,

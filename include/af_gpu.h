@@ -123,8 +123,8 @@ int af_vmult_pressure(af_operator* op, double* dst, const double* src);
 /* C: velocity -> pressure space (vmult_enthalpy, :2440-2453), uses pres_fixed */
 int af_vmult_enthalpy(af_operator* op, double* dst, const double* src);
 /* Exact inverse of the block-diagonal mass-type operator selected by NS_stage (1/4: M,
- * 6: D = M/(gamma-1), 3/5: A weighted by rho_for_fixed): per-cell inverses (from a Cholesky
- * factorisation, stored as packed symmetric matrices), built
+ * 6: D = M/(gamma-1), 3/5: A weighted by rho_for_fixed): per-cell inverses (symmetric
+ * sweeps without pivoting, stored as packed symmetric matrices), built
  * on first use and after set_rho_for_fixed.  Replaces the CG + multigrid solves of the
  * reference's update_density / update_velocity / update_pressure (Atmospheric_Flow.cc:
  * 527-535, 775-779, 870) by a direct solve; NS_stage 2 returns AF_BAD_ARG. */
