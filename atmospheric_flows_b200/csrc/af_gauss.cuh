@@ -48,7 +48,7 @@
 //
 // Measured at 512x256, p = 4 (131072 cells), us per launch in a chain, before (cell-major arrays,
 // element-wise copies through shared memory: 21.7 M and 26.6 M warp instructions) and now:
-//   k_gs_binv 32.9 -> 23.5, k_gs_zstep 46.9 -> 20.5 (the mixed IMEX step 70.2 -> 45.5 ms)
+//   k_gs_binv 32.9 -> 23.8, k_gs_zstep 46.9 -> 21.0 (the mixed IMEX step 70.2 -> 45.5 ms)
 // The step moves about 250 MB through L2 (164 MB of it DRAM) at 1024x256 in 37 us, 6.8 TB/s: it is
 // bound by memory; k_gs_binv (200 MB, 41 us) by issue (0.66 of the cycles) and latency.
 #pragma once
@@ -493,8 +493,8 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   }
   gs_ends<P>(pc, pt[2], pt[3]);
   gs_ends<P>(dc, tp[2], tp[3]);
-  // the far edges' normals come from shared memory up to degree 5 (degree 4, 256 tiles: 59.9 us a polynomial
-  // with them in registers, 56.7 us so; degree 6, 96 tiles: 60.5 and 71.9 us, nothing spills there)
+  // the far edges' normals come from shared memory up to degree 5 (in a trace, degree 4, 256 tiles: 59.9 us a
+  // polynomial with them in registers, 56.7 us so; degree 6, 96 tiles: 60.5 and 71.9 us, nothing spills there)
   if (SHARED_EDGES && m == 0) {
     s_rt[lane] = th.Rx;
     s_rt[kGsTile + lane] = th.Rz;
