@@ -93,7 +93,9 @@ struct GsShape {
   static constexpr int P1 = P + 1, ND = P1 * P1, NT = kGsTile * P1;
   // CTAs per SM asked of the compiler.  Degree 4, (k_gs_binv, k_gs_zstep), the mixed IMEX step at
   // 512x256: (4, 6) 46.3 ms, (5, 6) 45.4, (5, 7) 45.2, (6, 6) 46.8 (k_gs_binv spills at 64 registers).
-  static constexpr int CTAS_B = 800 / NT, CTAS_Z = (P <= 4 ? 1120 : 900) / NT;
+  // Degree 3, 6 / 7 of k_gs_binv (80, 72 registers), us a degree-20 polynomial: 320x160 cells 191, 193;
+  // 512x256 433, 422;  640x256 588, 569;  1024x256 1045, 1016.
+  static constexpr int CTAS_B = (P == 3 ? 900 : 800) / NT, CTAS_Z = (P <= 4 ? 1120 : 900) / NT;
   // k_gs_chain: more CTAs per SM take larger meshes.  Degree-20 polynomial, degree 4, 3 / 4 / 5 per SM (128,
   // 96, 80 registers; 0, 164, 356 bytes of spill loads): 256 tiles 58, 62, 72 us, 440 tiles 64, 70, 92, 550
   // tiles (165 by the pairs) 165, 79, 107; degree 2, 5 / 8 per SM: 256 tiles 45, 48 us, 1024 tiles (122 by
