@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   __shared__ float s_xf[4 * P1 * kGsTile];  // x-face fluxes of B [face][component][point][lane]
   __shared__ float s_w[2 * ND * kGsTile];   // w [component][node][lane]
   __shared__ float s_fx[ND * kGsTile], s_d[ND * kGsTile], s_xf2[2 * P1 * kGsTile];
-  constexpr bool SHARED_EDGES = P <= 5;
+  constexpr bool SHARED_EDGES = P >= 2 && P <= 5;
   __shared__ float s_rt[SHARED_EDGES ? 4 * kGsTile : 1];  // edges of the faces xi = 1 and eta = 1
   __shared__ float s_wm[ND * kGsTile];      // g / JxW; each thread reads its own column
   if (base > 0 && *gave_up) return;  // an earlier launch of this application
@@ -495,8 +495,9 @@ __global__ void __launch_bounds__(GsShape<P>::NT, GsShape<P>::CTAS_C)
   }
   gs_ends<P>(pc, pt[2], pt[3]);
   gs_ends<P>(dc, tp[2], tp[3]);
-  // the far edges' normals come from shared memory up to degree 5 (in a trace, degree 4, 256 tiles: 59.9 us a
-  // polynomial with them in registers, 56.7 us so; degree 6, 96 tiles: 60.5 and 71.9 us, nothing spills there)
+  // the far edges' normals come from shared memory at degrees 2 to 5 (in a trace, degree 4, 256 tiles: 59.9 us a
+  // polynomial with them in registers, 56.7 us so; degree 6, 96 tiles: 60.5 and 71.9 us, nothing spills there;
+  // degree 1, 256 and 437 tiles: 38.1 and 39.7 us in registers, 38.6 and 40.1 us so)
   if (SHARED_EDGES && m == 0) {
     s_rt[lane] = th.Rx;
     s_rt[kGsTile + lane] = th.Rz;
